@@ -327,3 +327,140 @@ def tolerance(case):
     with it (1.1e-5 in all and 5e-4 in single elements seen on the mid-sized network)."""
     relu = case["path"] in ("gcn", "gin") and case["train"] or case["path"] == "layer" or case.get("conv") == "gcn"
     return {"rel": 5e-5, "max": 2e-2} if relu else {"rel": 5e-6, "max": 2e-4}
+
+
+# ------------------------------------------------------------------------------------------------ 64 bits
+class _Sum64(torch.autograd.Function):
+    """out[r,h,:] = sum over edges of w[e,h] * x[col_e,h,:] in 64 bits, a slice of the edge list at a time."""
+
+    @staticmethod
+    def forward(ctx, x, w, rows, cols, n_rows):
+        ctx.save_for_backward(x, w, rows, cols)
+        out = x.new_zeros(n_rows, *x.shape[1:])
+        for e in _slices(rows, x):
+            part = x[cols[e]]
+            out.index_add_(0, rows[e], part if w is None else part * w[e].unsqueeze(-1))
+        return out
+
+    @staticmethod
+    def backward(ctx, grad):
+        x, w, rows, cols = ctx.saved_tensors
+        grad_x = torch.zeros_like(x)
+        grad_w = torch.empty_like(w) if ctx.needs_input_grad[1] else None
+        for e in _slices(rows, x):
+            part = grad[rows[e]]
+            if grad_w is not None:
+                grad_w[e] = (part * x[cols[e]]).sum(-1)
+            grad_x.index_add_(0, cols[e], part if w is None else part * w[e].unsqueeze(-1))
+        return grad_x, grad_w, None, None, None
+
+
+def _slices(rows, x):
+    step = max(1, (1 << 28) // max(1, x[0].numel()))
+    return [slice(e, e + step) for e in range(0, rows.numel(), step)]
+
+
+def _wide(t):
+    return t.detach().double().requires_grad_(True)
+
+
+def _edge_rows(indptr):
+    return torch.repeat_interleave(torch.arange(indptr.numel() - 1, device=indptr.device), (indptr[1:] - indptr[:-1]).long())
+
+
+def _sum64(x, rows, cols, n_rows, w=None):
+    return _Sum64.apply(x.unsqueeze(1), None if w is None else w.unsqueeze(1), rows, cols, n_rows).squeeze(1)
+
+
+def _attention64(q, k, x, rows, cols):
+    """Softmax over each row's edges of LeakyReLU(q[row] + k[col]), and the sum of x[col] weighted by it: [n_rows, H, F]."""
+    score = F.leaky_relu(q[rows] + k[cols], 0.2)
+    top = torch.full_like(q, -math.inf).index_reduce_(0, rows, score.detach(), "amax")
+    e = torch.exp(score - top.detach()[rows])
+    total = torch.zeros_like(q).index_add(0, rows, e)
+    return _Sum64.apply(x, e / total[rows], rows, cols, q.size(0))
+
+
+def _gat64(v, q, k, heads, x_src, x_dst, rows, cols):
+    """A GATLayer's mean over heads; v, q and k are the (weight, bias) pairs of its three dense products."""
+    h_src, h_dst = F.linear(x_src, *v), F.linear(x_dst, *v)
+    return _attention64(F.linear(h_dst, *q), F.linear(h_src, *k), h_src.view(h_src.size(0), heads, -1), rows, cols).mean(1)
+
+
+def exact(case, seed):
+    """What run() returns, in 64 bits and plain torch, for the inputs that prepare() makes."""
+    s = prepare(case, seed)
+    path = case["path"]
+    if path in ("gcn", "gin"):
+        rows, cols = _edge_rows(s.info.row_pointers), s.info.column_index.long()
+        norm, (w1, w2), n = s.info.degrees.double(), [_wide(p) for p in s.params], case["n"]
+        w = norm[rows] * norm[cols]
+        if path == "gcn":
+            logits = _sum64(torch.relu(_sum64(s.x.double() @ w1, rows, cols, n, w)) @ w2, rows, cols, n, w)
+        else:
+            logits = 0.5 * _sum64(torch.relu(0.5 * _sum64(s.x.double(), rows, cols, n) @ w1), rows, cols, n) @ w2
+        if not case["train"]:
+            return logits
+        loss = F.cross_entropy(logits, s.labels)
+        return [logits, loss, *torch.autograd.grad(loss, [w1, w2])]
+    if path == "rgcn":
+        return _rgcn64(s, case, seed)
+    if path == "rgat":
+        return _rgat64(s, case, seed)
+    if path == "batch":
+        key = torch.unique(s.dst.long() * case["n_src"] + s.src.long())
+        rows = torch.div(key, case["n_src"], rounding_mode="floor")
+        cols = key - rows * case["n_src"]
+        n_dst = case["n_dst"]
+    else:
+        indptr, indices = s.block.adj_sparse
+        rows, cols, n_dst = _edge_rows(indptr), indices.long(), case["n"]
+    if path == "spmm":
+        x = _wide(s.x)
+        out = _sum64(x, rows, cols, n_dst, None if s.weights is None else s.weights.double())
+        return [out, *torch.autograd.grad(out, [x], s.grad.double())] if case["train"] else out
+    if path == "attn":
+        q, k, x = params = [_wide(p) for p in s.params]
+        out = _attention64(q, k, x, rows, cols)
+        out = out.mean(1) if case["head_mean"] else out
+    elif path == "gat" or case.get("conv") == "gat":
+        x, *p = params = [_wide(t) for t in s.params]  # linear_q, linear_k, linear_v
+        out = F.elu(_gat64(p[4:6], p[0:2], p[2:4], case["heads"], x, x[:n_dst], rows, cols))
+    else:
+        x, w, b = params = [_wide(t) for t in s.params]
+        norm = 1.0 / torch.bincount(rows, minlength=n_dst).clamp(min=1).double()
+        out = torch.relu(norm.unsqueeze(1) * _sum64(F.linear(x, w, b), rows, cols, n_dst))
+    if not case.get("train", True):
+        return out
+    return [out, *torch.autograd.grad(out, params, s.grad.double())]
+
+
+def _rgcn64(s, case, seed):
+    sizes = [int(x.size(0)) for x in s.x]
+    rels = graphs.hetero_rgcn(device=DEVICE, type_sizes=sizes, n_relations=case["relations"], e_per_rel=case["edges"], seed=seed)
+    params = [_wide(p) for p in s.params]
+    used = sorted({st for st, _, _, _ in rels})
+    xs, weights = dict(zip(used, params)), iter(params[len(used):])
+    outs = []
+    for dt in sorted({r[1] for r in rels}):
+        out = 0.0
+        for st, _, indptr, indices in (r for r in rels if r[1] == dt):
+            rows = _edge_rows(indptr)
+            mean = 1.0 / (indptr[1:] - indptr[:-1]).double()[rows]
+            out = out + _sum64(F.linear(xs[st], next(weights), next(weights)), rows, indices.long(), sizes[dt], mean)
+        outs.append(out)
+    return [*outs, *torch.autograd.grad(outs, params, [g.double() for _, _, g in s.convs])]
+
+
+def _rgat64(s, case, seed):
+    params = [_wide(p) for p in s.params]
+    n_rel = case["relations"]
+    xs, x_dst, p = params[:n_rel], params[n_rel], params[n_rel + 1:]
+    out = 0.0
+    for r in range(n_rel):
+        src, dst = graphs.rmat_edges(seed * 100 + r, case["n_src"], case["n_dst"], case["edges"], device=DEVICE)
+        indptr, indices = graphs.csr_by_destination(src, dst, case["n_src"], case["n_dst"])
+        own = p[6 * r:6 * r + 6]
+        out = out + _gat64(own[4:6], own[0:2], own[2:4], case["heads"], xs[r], x_dst, _edge_rows(indptr), indices.long())
+    out = out / n_rel
+    return [out, *torch.autograd.grad(out, params, s.grad.double())]
