@@ -155,6 +155,64 @@ def test_stream_kernel_row_patterns(oracle, monkeypatch, pattern, D):
     assert_close(got.cpu().numpy(), ref_edge, what="rows-kernel %s D=%d" % (pattern, D))
 
 
+GROUP_WIDTHS = [1, 2, 4, 5, 8, 9, 12, 16, 17, 20, 24, 32, 33, 36, 40, 41, 48, 49, 60, 64, 65, 72, 97, 100, 120, 128, 129, 132, 136, 260, 264, 520]
+
+
+@pytest.mark.parametrize("D", GROUP_WIDTHS)
+@pytest.mark.parametrize("degrees", ["short", "mixed"])
+def test_group_kernel_dispatch_edges(oracle, monkeypatch, D, degrees):
+    """Every width class of the group kernel (two widths around each border; 256-, 128- and 32-bit loads), with rows that
+    end inside, at and behind a tile of ids, hub rows cut into chunks, and strided and misaligned outputs of the C ABI."""
+    import ctypes as C
+    from yitu_b200 import ops
+    from yitu_b200._lib import SpmmArgs, check, lib
+    monkeypatch.setenv("YITU_SPMM_STREAM", "0")
+    rng = np.random.default_rng(D * 3 + len(degrees))
+    n_cols = 400
+    degs = [0, 1, 2, 3, 4, 5, 7, 8, 9, 0, 6] * 3 if degrees == "short" else \
+        [0, 1, 8, 15, 16, 17, 31, 32, 33, 63, 64, 65, 0, 129, 300, 2, 0, 7]
+    indptr, indices = _csr_from_degrees(rng, degs, n_cols)
+    n_rows = len(degs)
+    x = rng.standard_normal((n_cols, D)).astype(np.float32)
+    vals = rng.standard_normal(indices.shape[0]).astype(np.float32)
+    bias = rng.standard_normal(D).astype(np.float32)
+    base = rng.standard_normal((n_rows, D)).astype(np.float32)
+    ref = oracle.spmm(indptr, indices, x, wmode=oracle.W_EDGE, values=vals)
+    ref_acc = np.maximum(oracle.spmm(indptr, indices, x, alpha=0.5, out=base) + bias, 0)
+    g = ops.PreparedGraph(_dev(indptr, torch.int32), _dev(indices), n_cols)
+    for chunk in (0, 64, None):
+        got = ops.spmm(g, _dev(x), mode=ops.W_EDGE, edge_values=_dev(vals), chunk_edges=chunk)
+        assert_close(got.cpu().numpy(), ref, what="group %s D=%d chunk=%s" % (degrees, D, chunk))
+        out = _dev(base).clone()
+        ops.spmm(g, _dev(x), out=out, accumulate=True, alpha=0.5, bias=_dev(bias), activation="relu", chunk_edges=chunk)
+        assert_close(out.cpu().numpy(), ref_acc, what="group %s D=%d chunk=%s accumulate" % (degrees, D, chunk))
+    # rows that start 4 / 16 bytes behind a 32-byte boundary, and strides wider than the rows
+    for shift, pad in ((1, 3), (4, 4), (0, 8)):
+        xs = torch.zeros(n_cols, D + pad, device="cuda").view(-1)
+        xs = torch.cat([xs, xs.new_zeros(8)])[shift:shift + n_cols * (D + pad)].view(n_cols, D + pad)
+        xs[:, :D] = _dev(x)
+        out = torch.full((n_rows, D + pad), 7.0, device="cuda")
+        a = SpmmArgs()
+        a.graph, a.n_heads, a.n_feats, a.weight_mode, a.alpha = g.csr, 1, D, ops.W_EDGE, 1.0
+        v = _dev(vals)
+        a.edge_values, a.x, a.x_stride = ops._ptr(v), C.c_void_p(xs.data_ptr()), D + pad
+        a.out, a.out_stride = ops._ptr(out), D + pad
+        check(lib().yitu_spmm_csr_f32(C.byref(a), ops._stream(xs.device)))
+        assert_close(out[:, :D].cpu().numpy(), ref, what="group %s D=%d shift=%d pad=%d" % (degrees, D, shift, pad))
+        assert bool((out[:, D:] == 7.0).all())
+
+
+def test_infinite_features_stay_infinite():
+    """Lanes behind a row's last edge gather nothing, so an infinite feature sums to infinity and not to NaN."""
+    from yitu_b200 import ops
+    x = torch.randn(8, 64, device="cuda")
+    x[3] = float("inf")
+    g = ops.PreparedGraph(torch.tensor([0, 3, 4], dtype=torch.int32, device="cuda"),
+                          torch.tensor([3, 1, 2, 5], dtype=torch.int32, device="cuda"), 8)
+    out = ops.spmm(g, x)
+    assert bool(torch.isinf(out[0]).all()) and torch.equal(out[1], x[5])
+
+
 def test_kernel_module_matches_oracle_on_gcn_graph(oracle):
     """2-layer GCN forward of the small benchmark configuration, plus the other YiTu_GNN_kernel entry points."""
     from yitu_b200 import YiTu_GNN_kernel as K, graphs

@@ -82,6 +82,9 @@ __device__ __forceinline__ void load_vec(float (&r)[VEC], const float *p) {
     } else if constexpr (VEC == 4) {
         const float4 v = __ldg(reinterpret_cast<const float4 *>(p));
         r[0] = v.x; r[1] = v.y; r[2] = v.z; r[3] = v.w;
+    } else if constexpr (VEC == 2) {
+        const float2 v = __ldg(reinterpret_cast<const float2 *>(p));
+        r[0] = v.x; r[1] = v.y;
     } else {
         r[0] = __ldg(p);
     }
@@ -95,6 +98,8 @@ __device__ __forceinline__ void store_vec(float *p, const float (&r)[VEC]) {
         __stcs(reinterpret_cast<float4 *>(p) + 1, make_float4(r[4], r[5], r[6], r[7]));
     } else if constexpr (VEC == 4) {
         __stcs(reinterpret_cast<float4 *>(p), make_float4(r[0], r[1], r[2], r[3]));
+    } else if constexpr (VEC == 2) {
+        __stcs(reinterpret_cast<float2 *>(p), make_float2(r[0], r[1]));
     } else {
         __stcs(p, r[0]);
     }

@@ -1,21 +1,22 @@
 // CSR pull SpMM for sm_100a:  out[r,:] = act(alpha*row_scale[r] * sum_{e in row r} w(e) * x[col_e,:] + bias)
 //
 // Work decomposition
-//   * a group of LPR lanes (4..32, one warp for rows of >= 128 floats) owns one destination row, or one
-//     chunk of a hub row; each lane keeps NV independent 128-bit accumulators, so a warp has up to
-//     4 edges x NV x 512 B of feature gathers in flight;
-//   * column ids / edge weights are fetched LPR at a time, one per lane (coalesced, streamed past L1)
-//     and broadcast with warp shuffles, so the gather loop issues nothing but 128-bit loads and FMAs;
+//   * scalar weights: spmm_group_kernel, the narrowest group of lanes that covers a source row owns one destination row or
+//     one chunk of a hub row; spmm_stream_kernel for wide rows of huge graphs (a warp walks 16 rows as one edge stream);
+//     per-head weights: spmm_heads_kernel;
+//   * column ids / edge weights are fetched one per lane (coalesced, streamed past L1) and broadcast with shuffles, so the
+//     gather loop issues nothing but 128- or 256-bit loads and FMAs;
 //   * rows longer than plan->chunk_edges are cut into chunks handled by the first n_chunks groups of the
-//     grid (scheduled first: they are the longest tasks); partial sums land in scratch and a second tiny
-//     kernel adds them in chunk order.  No float atomics anywhere: results are run-to-run identical.
+//     grid (scheduled first: they are the longest tasks); partial sums land in scratch and a second small
+//     kernel adds them in a fixed order.  No float atomics anywhere: results are run-to-run identical.
 //
 // Measured alternatives that lost on B200 and are not kept: staging rows in a shared-memory ring with
 // cp.async.bulk + mbarrier (2.2x slower: 1 KiB per bulk copy is too fine a grain) or per-lane cp.async (equal
-// at best, only at the same occupancy); sub-warp groups narrower than the row (lose coalescing); a persistent
+// at best, only at the same occupancy); a persistent
 // grid with software-pipelined row pointers / index tiles (1.7x slower than letting the CTA scheduler
-// balance short CTAs); batches of 8 consecutive rows per warp with the next row's index tile prefetched
-// (1.1-1.4x slower: fewer, longer warps hide less latency than many short ones); for heads that share one source
+// balance short CTAs); the features in slices of 128 or 64 floats, one pass over the graph per slice, so that a larger
+// share of the gathered table stays in L2 (uniform graph 1 M rows x 32 edges x 256 floats: 4.87 ms in one pass, 4.84 in
+// two, 5.11 in four; R-MAT 2.1 M rows x 30 edges: 5.75-6.1 in one, 6.7 in two); for heads that share one source
 // row (x_shared_heads), a lane-per-feature layout with the H edge weights broadcast by shuffle (5.4 ms against 3.7 ms
 // for the per-head layout below on the 8x32 layer: ten shuffles per edge cost more than the replicated loads).
 //
@@ -65,8 +66,9 @@ __device__ __forceinline__ void finish_vec(float (&r)[VEC], const SpmmParams &p,
     }
 }
 
-template <int LPR, int NV, int VEC, int EU, bool PER_HEAD, bool IDX32>
-__global__ void __launch_bounds__(256) spmm_kernel(const __grid_constant__ SpmmParams p) {
+// Per-head edge values (weight of an edge differs from head to head): LPR lanes per row, NV slices of VEC floats per lane.
+template <int LPR, int NV, int VEC, int EU, bool IDX32>
+__global__ void __launch_bounds__(256) spmm_heads_kernel(const __grid_constant__ SpmmParams p) {
     static_assert(EU <= LPR && (EU & (EU - 1)) == 0, "edge unroll must be a power of two <= lanes per row");
     const int lane = threadIdx.x & 31;
     const int l = lane & (LPR - 1);
@@ -102,8 +104,8 @@ __global__ void __launch_bounds__(256) spmm_kernel(const __grid_constant__ SpmmP
     for (int i = 0; i < NV; ++i) {
         off[i] = d0 + static_cast<int64_t>(i * LPR + l) * VEC;
         valid[i] = off[i] < p.D;
-        hd[i] = PER_HEAD ? static_cast<int>(off[i] / p.F) : 0;
-        xo[i] = (PER_HEAD && p.xshared) ? off[i] - static_cast<int64_t>(hd[i]) * p.F : off[i];
+        hd[i] = static_cast<int>(off[i] / p.F);
+        xo[i] = p.xshared ? off[i] - static_cast<int64_t>(hd[i]) * p.F : off[i];
     }
 
     float acc[NV][VEC];
@@ -112,33 +114,19 @@ __global__ void __launch_bounds__(256) spmm_kernel(const __grid_constant__ SpmmP
 #pragma unroll
         for (int v = 0; v < VEC; ++v) acc[i][v] = 0.0f;
 
-    const float nd = (p.wmode == YITU_W_NODE) ? __ldg(p.norm_dst + row) : 0.0f;
-
     for (int64_t e0 = eb; e0 < ee; e0 += LPR) {
         const int n = static_cast<int>(min(static_cast<int64_t>(LPR), ee - e0));
         int my_col = 0, my_vi = 0;
-        float my_w = 0.0f;
         if (l < n) {
             const int64_t e = e0 + l;
             const int rawidx = ld_stream(p.indices + e);
             my_col = p.mask ? (rawidx & p.mask) : rawidx;
-            if constexpr (PER_HEAD) {
-                my_vi = p.perm ? ld_stream(p.perm + e) : static_cast<int>(e);
-            } else {
-                if (p.wmode == YITU_W_NONE) {
-                    my_w = 1.0f;
-                } else if (p.wmode == YITU_W_NODE) {
-                    my_w = nd * __ldg(p.norm_src + my_col);
-                } else {
-                    const int64_t vi = p.perm ? static_cast<int64_t>(ld_stream(p.perm + e)) : e;
-                    my_w = ld_stream(p.values + vi);
-                }
-            }
+            my_vi = p.perm ? ld_stream(p.perm + e) : static_cast<int>(e);
         }
         // lanes past the end of the row repeat the tile's first edge with weight 0, so the gather loop
         // below runs in steps of EU edges without a remainder path (the repeated row is an L1 hit)
         const int c_first = __shfl_sync(gmask, my_col, 0, LPR);
-        const int v_first = PER_HEAD ? __shfl_sync(gmask, my_vi, 0, LPR) : 0;
+        const int v_first = __shfl_sync(gmask, my_vi, 0, LPR);
         if (l >= n) {
             my_col = c_first;
             my_vi = v_first;
@@ -146,15 +134,10 @@ __global__ void __launch_bounds__(256) spmm_kernel(const __grid_constant__ SpmmP
         const int n_up = (n + EU - 1) & ~(EU - 1);
         for (int j = 0; j < n_up; j += EU) {
             int c[EU], vi[EU];
-            float w[EU];
 #pragma unroll
             for (int u = 0; u < EU; ++u) {
                 c[u] = __shfl_sync(gmask, my_col, j + u, LPR);
-                if constexpr (PER_HEAD) {
-                    vi[u] = __shfl_sync(gmask, my_vi, j + u, LPR);
-                } else {
-                    w[u] = __shfl_sync(gmask, my_w, j + u, LPR);
-                }
+                vi[u] = __shfl_sync(gmask, my_vi, j + u, LPR);
             }
             float v[EU][NV][VEC];
             float wh[EU][NV];
@@ -168,8 +151,7 @@ __global__ void __launch_bounds__(256) spmm_kernel(const __grid_constant__ SpmmP
                     if (valid[i]) {
                         if constexpr (IDX32) load_vec<VEC>(v[u][i], p.x + (xr32 + static_cast<uint32_t>(xo[i])));
                         else load_vec<VEC>(v[u][i], xr + xo[i]);
-                        if constexpr (PER_HEAD)
-                            wh[u][i] = (j + u < n) ? __ldg(p.values + static_cast<int64_t>(vi[u]) * p.H + hd[i]) : 0.0f;
+                        wh[u][i] = (j + u < n) ? __ldg(p.values + static_cast<int64_t>(vi[u]) * p.H + hd[i]) : 0.0f;
                     } else {
 #pragma unroll
                         for (int q = 0; q < VEC; ++q) v[u][i][q] = 0.0f;
@@ -180,11 +162,9 @@ __global__ void __launch_bounds__(256) spmm_kernel(const __grid_constant__ SpmmP
 #pragma unroll
             for (int u = 0; u < EU; ++u)
 #pragma unroll
-                for (int i = 0; i < NV; ++i) {
-                    const float ww = PER_HEAD ? wh[u][i] : w[u];
+                for (int i = 0; i < NV; ++i)
 #pragma unroll
-                    for (int q = 0; q < VEC; ++q) acc[i][q] = fmaf(ww, v[u][i][q], acc[i][q]);
-                }
+                    for (int q = 0; q < VEC; ++q) acc[i][q] = fmaf(wh[u][i], v[u][i][q], acc[i][q]);
         }
     }
 
@@ -212,16 +192,25 @@ __global__ void __launch_bounds__(256) spmm_kernel(const __grid_constant__ SpmmP
     }
 }
 
-// Rows of at most 128 floats with 256-bit loads: the warp still owns one destination row (or hub chunk), but one
-// load instruction now fetches 32 / LPE edges at once — LPE = D/8 lanes (32 bytes each) cover a source row, so the
-// lanes of sub-group s gather edge s of every step.  Each sub-group accumulates its own edges; a butterfly over the
-// sub-groups adds them up at the end of the row.  Scalar weights only (no per-head values).
-template <int LPE, int EU, bool IDX32>
-__global__ void __launch_bounds__(256) spmm_wide_kernel(const __grid_constant__ SpmmParams p) {
-    constexpr int EPI = 32 / LPE;  // edges per load instruction
+// Scalar weights.  A group of RW lanes owns one destination row (or hub chunk); LPE of them cover a source row (NV slices
+// of VEC floats each), so one load instruction of the group fetches RW/LPE edges, and EU such instructions are in flight per
+// step.  With RW > LPE every sub-group sums its own edges and a reduce-scatter over the sub-groups ends the row (half of the
+// values change hands at every level, so 8 values over 8 sub-groups cost 7 shuffles instead of 24) and leaves each lane one
+// contiguous piece of the result to store.
+//   What bounds it: DRAM and L2 bandwidth for wide rows; for narrow ones the chain of three dependent latencies per row
+// (row pointer, ids, gathers).  A row's edges are therefore gathered 8 to 16 at a time, and the next tile of ids is
+// requested before the current one is consumed.
+template <int RW, int LPE, int NV, int VEC, int EU, bool IDX32>
+__global__ void __launch_bounds__(128) spmm_group_kernel(const __grid_constant__ SpmmParams p) {
+    constexpr int EPI = RW / LPE;  // edges per load instruction
+    constexpr int STEP = EPI * EU;
+    static_assert(RW % LPE == 0 && RW % STEP == 0, "a tile of RW ids is consumed in whole steps");
     const int lane = threadIdx.x & 31;
-    const int sub = lane / LPE, l = lane & (LPE - 1);
-    const int64_t gid = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int gl = lane & (RW - 1);
+    const int sub = gl / LPE, l = gl & (LPE - 1);
+    const unsigned gmask = (RW == 32) ? 0xffffffffu : (((1u << (RW & 31)) - 1u) << (lane & ~(RW - 1)));
+    const int64_t gid = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / RW;
+    const int64_t d0 = static_cast<int64_t>(blockIdx.y) * (LPE * NV * VEC);
     int64_t row, eb, ee;
     float *dst;
     bool raw;
@@ -237,87 +226,130 @@ __global__ void __launch_bounds__(256) spmm_wide_kernel(const __grid_constant__ 
         if (row >= p.row_tasks) return;
         eb = load_ptr(p.indptr, p.is64, row);
         ee = load_ptr(p.indptr, p.is64, row + 1);
-        if (p.n_chunks > 0 && ee - eb > p.chunk_edges) return;
+        if (p.n_chunks > 0 && ee - eb > p.chunk_edges) return;  // hub row: done by its chunks
         dst = p.out + row * p.os;
         raw = false;
     }
-    const int off = l * 8;
-    const bool valid = off < p.D;
-    float acc[8];
+    int off[NV];
+    bool valid[NV];
+    float acc[NV][VEC];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) acc[q] = 0.0f;
+    for (int i = 0; i < NV; ++i) {
+        off[i] = static_cast<int>(d0) + (i * LPE + l) * VEC;
+        valid[i] = off[i] < p.D;
+#pragma unroll
+        for (int q = 0; q < VEC; ++q) acc[i][q] = 0.0f;
+    }
     const float nd = (p.wmode == YITU_W_NODE) ? __ldg(p.norm_dst + row) : 0.0f;
 
-    for (int64_t e0 = eb; e0 < ee; e0 += 32) {
-        const int n = static_cast<int>(min(static_cast<int64_t>(32), ee - e0));
-        int my_col = 0;
-        float my_w = 0.0f;
-        if (lane < n) {
-            const int64_t e = e0 + lane;
+    auto load_tile = [&](int64_t e0, int &col, float &w) {
+        col = 0;
+        w = 0.0f;
+        const int64_t e = e0 + gl;
+        if (e < ee) {
             const int rawidx = ld_stream(p.indices + e);
-            my_col = p.mask ? (rawidx & p.mask) : rawidx;
+            col = p.mask ? (rawidx & p.mask) : rawidx;
             if (p.wmode == YITU_W_NONE) {
-                my_w = 1.0f;
+                w = 1.0f;
             } else if (p.wmode == YITU_W_NODE) {
-                my_w = nd * __ldg(p.norm_src + my_col);
+                w = nd * __ldg(p.norm_src + col);
             } else {
                 const int64_t vi = p.perm ? static_cast<int64_t>(ld_stream(p.perm + e)) : e;
-                my_w = ld_stream(p.values + vi);
+                w = ld_stream(p.values + vi);
             }
         }
-        const int c_first = __shfl_sync(0xffffffffu, my_col, 0);
-        if (lane >= n) my_col = c_first;  // weight 0, a row that is in flight anyway
-        constexpr int STEP = EPI * EU;     // edges per unrolled step
-        const int n_up = (n + STEP - 1) / STEP * STEP;
-        for (int j = 0; j < n_up; j += STEP) {
+    };
+    int my_col;
+    float my_w;
+    load_tile(eb, my_col, my_w);
+    for (int64_t e0 = eb; e0 < ee; e0 += RW) {
+        const int n = static_cast<int>(min(static_cast<int64_t>(RW), ee - e0));
+        int nx_col = 0;
+        float nx_w = 0.0f;
+        if (e0 + RW < ee) load_tile(e0 + RW, nx_col, nx_w);
+        for (int j = 0; j < n; j += STEP) {
             int c[EU];
             float w[EU];
 #pragma unroll
             for (int u = 0; u < EU; ++u) {
-                const int idx = (j + u * EPI + sub) & 31;
-                c[u] = __shfl_sync(0xffffffffu, my_col, idx);
-                w[u] = (j + u * EPI + sub < 32) ? __shfl_sync(0xffffffffu, my_w, idx) : (__shfl_sync(0xffffffffu, my_w, idx), 0.0f);
+                c[u] = __shfl_sync(gmask, my_col, j + u * EPI + sub, RW);
+                w[u] = __shfl_sync(gmask, my_w, j + u * EPI + sub, RW);  // 0 behind the last edge
             }
-            float v[EU][8];
+            float v[EU][NV][VEC];
 #pragma unroll
             for (int u = 0; u < EU; ++u) {
-                if (valid) {
-                    if constexpr (IDX32)
-                        load_vec<8>(v[u], p.x + (static_cast<uint32_t>(c[u]) * static_cast<uint32_t>(p.xs) + static_cast<uint32_t>(off)));
-                    else
-                        load_vec<8>(v[u], p.x + static_cast<int64_t>(c[u]) * p.xs + off);
-                } else {
+                const bool live = j + u * EPI + sub < n;
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) v[u][q] = 0.0f;
+                for (int i = 0; i < NV; ++i) {
+                    if (live && valid[i]) {
+                        if constexpr (IDX32)
+                            load_vec<VEC>(v[u][i], p.x + (static_cast<uint32_t>(c[u]) * static_cast<uint32_t>(p.xs) + static_cast<uint32_t>(off[i])));
+                        else
+                            load_vec<VEC>(v[u][i], p.x + static_cast<int64_t>(c[u]) * p.xs + off[i]);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < VEC; ++q) v[u][i][q] = 0.0f;
+                    }
                 }
             }
 #pragma unroll
             for (int u = 0; u < EU; ++u)
 #pragma unroll
-                for (int q = 0; q < 8; ++q) acc[q] = fmaf(w[u], v[u][q], acc[q]);
+                for (int i = 0; i < NV; ++i)
+#pragma unroll
+                    for (int q = 0; q < VEC; ++q) acc[i][q] = fmaf(w[u], v[u][i][q], acc[i][q]);
         }
+        my_col = nx_col;
+        my_w = nx_w;
     }
-    // add the sub-groups' partial sums (fixed order: deterministic)
+    // reduce-scatter over the sub-groups (fixed order: deterministic); piece = floats of a slice that this lane ends up with
+    constexpr int PIECE = (VEC >= EPI) ? VEC / EPI : 1;
+    int piece_at = 0;    // offset of the lane's piece inside its VEC-wide slice
+    bool owner = true;   // with more sub-groups than values several lanes hold the same piece: the first one stores it
 #pragma unroll
-    for (int o = LPE; o < 32; o <<= 1)
+    for (int o = LPE, have = VEC; o < RW; o <<= 1) {
+        const bool upper = (gl & o) != 0;
+        if (have > 1) {
+            const int half = have / 2;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
-    if (sub != 0 || !valid) return;
-    if (raw) {
-        store_vec<8>(dst + off, acc);
-    } else {
-        const float s = p.alpha * (p.row_scale ? __ldg(p.row_scale + row) : 1.0f);
-        float r[8];
-        if (p.accumulate) {
-            load_vec<8>(r, dst + off);
+            for (int i = 0; i < NV; ++i)
 #pragma unroll
-            for (int q = 0; q < 8; ++q) r[q] = fmaf(s, acc[q], r[q]);
+                for (int q = 0; q < VEC / 2; ++q)
+                    if (q < half) {
+                        const float send = upper ? acc[i][q] : acc[i][q + half];
+                        const float keep = upper ? acc[i][q + half] : acc[i][q];
+                        acc[i][q] = keep + __shfl_xor_sync(gmask, send, o, RW);
+                    }
+            if (upper) piece_at += half;
+            have = half;
         } else {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) r[q] = s * acc[q];
+            for (int i = 0; i < NV; ++i) acc[i][0] += __shfl_xor_sync(gmask, acc[i][0], o, RW);
+            owner = owner && !upper;
         }
-        finish_vec<8>(r, p, off);
-        store_vec<8>(dst + off, r);
+    }
+    if (!owner) return;
+    const float s = raw ? 1.0f : p.alpha * (p.row_scale ? __ldg(p.row_scale + row) : 1.0f);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        if (!valid[i]) continue;
+        const int at = off[i] + piece_at;
+        float r[PIECE];
+#pragma unroll
+        for (int q = 0; q < PIECE; ++q) r[q] = acc[i][q];
+        if (!raw) {
+            if (p.accumulate) {
+                float old[PIECE];
+                load_vec<PIECE>(old, dst + at);
+#pragma unroll
+                for (int q = 0; q < PIECE; ++q) r[q] = fmaf(s, r[q], old[q]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < PIECE; ++q) r[q] = s * r[q];
+            }
+            finish_vec<PIECE>(r, p, at);
+        }
+        store_vec<PIECE>(dst + at, r);
     }
 }
 
@@ -344,7 +376,7 @@ __global__ void __launch_bounds__(128, (VEC * EU <= 32) ? 6 : 4) spmm_stream_ker
     const int64_t gid = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
 
     // rp: first edge of row `lane` of the batch, relative to the batch's first edge (positions inside a batch fit 32
-    // bits: the launcher sends graphs of 2^31 or more edges to the warp-per-row kernel)
+    // bits: the launcher sends graphs of 2^31 or more edges to the group kernel)
     int64_t r0, E0;
     int nr, rp;
     bool raw;
@@ -526,31 +558,59 @@ __global__ void __launch_bounds__(128, (VEC * EU <= 32) ? 6 : 4) spmm_stream_ker
     flush(INT32_MAX);
 }
 
-// Adds the chunk partials of each hub row in chunk order and applies the epilogue.
-__global__ void __launch_bounds__(128) hub_reduce_kernel(const __grid_constant__ SpmmParams p) {
+// Adds the chunk partials of each hub row and applies the epilogue.  One CTA per hub row (the CTAs of a row's later
+// chunks leave at once): `cols` threads span the features and the others split the chunks, each group summing every
+// groups-th chunk; thread 0 of a feature then adds the groups in order, so the sum is the same in every run.  A serial
+// loop over the chunks made a row of a few hundred chunks the tail of the whole aggregation.
+__global__ void __launch_bounds__(256) hub_reduce_kernel(const __grid_constant__ SpmmParams p, int cols) {
+    __shared__ float s_part[256];
     const int64_t chunk = blockIdx.x;
     const int64_t row = __ldg(p.chunk_row + chunk);
     const int64_t rb = load_ptr(p.indptr, p.is64, row);
     if (__ldg(p.chunk_begin + chunk) != rb) return;  // only a row's first chunk reduces
     const int64_t re = load_ptr(p.indptr, p.is64, row + 1);
-    const int64_t nch = (re - rb + p.chunk_edges - 1) / p.chunk_edges;
+    const int nch = static_cast<int>((re - rb + p.chunk_edges - 1) / p.chunk_edges);
     const float s = p.alpha * (p.row_scale ? __ldg(p.row_scale + row) : 1.0f);
-    for (int64_t d = threadIdx.x; d < p.D; d += blockDim.x) {
+    const int tx = threadIdx.x & (cols - 1), grp = threadIdx.x / cols, groups = blockDim.x / cols;
+    const float *part = p.scratch + chunk * p.D;
+    for (int64_t d0 = 0; d0 < p.D; d0 += cols) {
+        const int64_t d = d0 + tx;
         float a = 0.0f;
-        for (int64_t k = 0; k < nch; ++k) a += p.scratch[(chunk + k) * p.D + d];
-        float *o = p.out + row * p.os + d;
-        float r = p.accumulate ? fmaf(s, a, *o) : s * a;
-        if (p.bias) r += __ldg(p.bias + d);
-        *o = activate(r, p.act);
+        if (d < p.D) {
+#pragma unroll 4
+            for (int k = grp; k < nch; k += groups) a += part[k * p.D + d];
+        }
+        if (groups > 1) {
+            s_part[threadIdx.x] = a;
+            __syncthreads();
+            if (grp == 0)
+                for (int g = 1; g < groups && g < nch; ++g) a += s_part[g * cols + tx];
+            __syncthreads();
+        }
+        if (grp == 0 && d < p.D) {
+            float *o = p.out + row * p.os + d;
+            float r = p.accumulate ? fmaf(s, a, *o) : s * a;
+            if (p.bias) r += __ldg(p.bias + d);
+            *o = activate(r, p.act);
+        }
     }
+}
+
+static int launch_hub_reduce(const SpmmParams &p, cudaStream_t st) {
+    if (p.n_chunks == 0) return YITU_OK;
+    int cols = 16;
+    while (cols < p.D && cols < 256) cols <<= 1;
+    hub_reduce_kernel<<<static_cast<unsigned>(p.n_chunks), 256, 0, st>>>(p, cols);
+    YITU_LAUNCH_CHECK();
+    return YITU_OK;
 }
 
 // 128-thread CTAs: with 256 a CTA waits for its longest row and occupancy drops (measured 7.57 -> 6.98 ms on the
 // D=256 R-MAT workload; 32/64/128/256 gave 6.86/7.21/6.98/7.57 ms and 128 was best over all workloads).
 static int block_threads() { return 128; }
 
-template <int LPR, int NV, int VEC, int EU, int EU_HEAD = 4>
-static int launch(const SpmmParams &p, bool per_head, cudaStream_t st, bool reduce = true) {
+template <int LPR, int NV, int VEC>
+static int launch_heads(const SpmmParams &p, cudaStream_t st) {
     const int64_t groups = p.chunk_tasks + p.row_tasks;
     if (groups == 0) return YITU_OK;
     const int threads = block_threads();
@@ -560,21 +620,11 @@ static int launch(const SpmmParams &p, bool per_head, cudaStream_t st, bool redu
     YITU_REQUIRE(gx < (1ll << 31) && gy <= 65535, YITU_ERR_LIMIT, "spmm grid too large (%lld x %lld)",
                  (long long)gx, (long long)gy);
     dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
-    // element offsets into x fit 32 bits?
-    const bool idx32 = VEC >= 4 && p.n_cols * p.xs < (1ll << 32);
-    if (per_head) {  // per-head weights cost registers per gathered slice: those variants unroll 4 edges only
-        if (idx32) spmm_kernel<LPR, NV, VEC, EU_HEAD, true, true><<<grid, threads, 0, st>>>(p);
-        else spmm_kernel<LPR, NV, VEC, EU_HEAD, true, false><<<grid, threads, 0, st>>>(p);
-    } else {
-        if (idx32) spmm_kernel<LPR, NV, VEC, EU, false, true><<<grid, threads, 0, st>>>(p);
-        else spmm_kernel<LPR, NV, VEC, EU, false, false><<<grid, threads, 0, st>>>(p);
-    }
+    // 32-bit element offsets into x when they fit; per-head weights cost registers per gathered slice: 4 edges per step
+    if (VEC >= 4 && p.n_cols * p.xs < (1ll << 32)) spmm_heads_kernel<LPR, NV, VEC, 4, true><<<grid, threads, 0, st>>>(p);
+    else spmm_heads_kernel<LPR, NV, VEC, 4, false><<<grid, threads, 0, st>>>(p);
     YITU_LAUNCH_CHECK();
-    if (reduce && p.n_chunks > 0) {
-        hub_reduce_kernel<<<static_cast<unsigned>(p.n_chunks), 128, 0, st>>>(p);
-        YITU_LAUNCH_CHECK();
-    }
-    return YITU_OK;
+    return launch_hub_reduce(p, st);
 }
 
 template <int VEC, int EU, int R>
@@ -595,16 +645,12 @@ static int launch_stream(const SpmmParams &p, cudaStream_t st) {  // always foll
         else spmm_stream_kernel<VEC, EU, R, false, false><<<grid, threads, 0, st>>>(p);
     }
     YITU_LAUNCH_CHECK();
-    if (hub) {
-        hub_reduce_kernel<<<static_cast<unsigned>(p.n_chunks), 128, 0, st>>>(p);
-        YITU_LAUNCH_CHECK();
-    }
-    return YITU_OK;
+    return launch_hub_reduce(p, st);
 }
 
 // Development switches read from the environment at every call (measurement of one kernel form against another):
-// YITU_SPMM_STREAM=0 keeps the warp-per-row kernels for every graph, =2 takes the edge-stream kernel for every graph
-// whose shape it covers (default 1: by average row length, see yitu_spmm_csr_f32); YITU_SPMM_STREAM_ROWS=8|16|31 and
+// YITU_SPMM_STREAM=0 keeps the group kernel for every graph, =2 takes the edge-stream kernel for every graph
+// whose shape it covers (default 1: by the rule in yitu_spmm_csr_f32); YITU_SPMM_STREAM_ROWS=8|16|31 and
 // YITU_SPMM_STREAM_EU pick an instantiation of the edge-stream kernel other than the default.
 static int env_int(const char *name, int dflt) {
     const char *v = getenv(name);
@@ -625,21 +671,56 @@ static int dispatch_stream(const SpmmParams &p, cudaStream_t st, int rows_dflt, 
     return launch_stream<VEC, EU_A, 16>(p, st);
 }
 
-template <int LPE, int EU>
-static int launch_wide(const SpmmParams &p, cudaStream_t st) {
+template <int RW, int LPE, int NV, int VEC, int EU>
+static int launch_group(const SpmmParams &p, cudaStream_t st, bool reduce = true) {
     const int64_t groups = p.chunk_tasks + p.row_tasks;
     if (groups == 0) return YITU_OK;
     const int threads = block_threads();
-    const int64_t gx = (groups + threads / 32 - 1) / (threads / 32);
-    YITU_REQUIRE(gx < (1ll << 31), YITU_ERR_LIMIT, "spmm grid too large (%lld)", (long long)gx);
-    if (p.n_cols * p.xs < (1ll << 32)) spmm_wide_kernel<LPE, EU, true><<<static_cast<unsigned>(gx), threads, 0, st>>>(p);
-    else spmm_wide_kernel<LPE, EU, false><<<static_cast<unsigned>(gx), threads, 0, st>>>(p);
+    const int64_t gx = (groups + threads / RW - 1) / (threads / RW);
+    const int64_t gy = (p.D + LPE * NV * VEC - 1) / (LPE * NV * VEC);
+    YITU_REQUIRE(gx < (1ll << 31) && gy <= 65535, YITU_ERR_LIMIT, "spmm grid too large (%lld x %lld)",
+                 (long long)gx, (long long)gy);
+    dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
+    if (p.n_cols * p.xs < (1ll << 32)) spmm_group_kernel<RW, LPE, NV, VEC, EU, true><<<grid, threads, 0, st>>>(p);
+    else spmm_group_kernel<RW, LPE, NV, VEC, EU, false><<<grid, threads, 0, st>>>(p);
     YITU_LAUNCH_CHECK();
-    if (p.n_chunks > 0) {
-        hub_reduce_kernel<<<static_cast<unsigned>(p.n_chunks), 128, 0, st>>>(p);
-        YITU_LAUNCH_CHECK();
-    }
-    return YITU_OK;
+    return reduce ? launch_hub_reduce(p, st) : YITU_OK;
+}
+
+// Lanes per row (RW), lanes per edge and edges per step of spmm_group_kernel by row width.  The narrowest group that
+// covers a source row wins on every graph that fills the machine: four rows of 64 floats per warp instead of one keep
+// four times as many dependent chains in flight and need no sum across lanes (uniform graph, 1 M rows x 16 edges, us, by
+// lanes per row 32 / 16 / 8: 64 floats 917 / 793 / 680; 16 floats 860 / 395 / 313).  Rows of at most 32 floats keep 8 lanes,
+// two or four edges per load instruction, so that a power-law graph's long rows do not hold up their warp (1 M rows x 15
+// edges, 32 floats: 474 us with 4 lanes, 460 with 8); below 8 edges per row and without hub rows there is nothing to hold
+// up and the narrowest group is taken (2 M rows x 4 edges: 16 floats 365 -> 266, 32 floats 440 -> 364).
+static int dispatch_group8(const SpmmParams &p, bool short_rows, cudaStream_t st, bool reduce = true) {
+    if (p.D <= 16) return short_rows ? launch_group<2, 2, 1, 8, 2>(p, st, reduce) : launch_group<8, 2, 1, 8, 2>(p, st, reduce);
+    if (p.D <= 32) return short_rows ? launch_group<4, 4, 1, 8, 4>(p, st, reduce) : launch_group<8, 4, 1, 8, 4>(p, st, reduce);
+    if (p.D <= 64) return launch_group<8, 8, 1, 8, 8>(p, st, reduce);
+    if (p.D <= 128) return launch_group<16, 16, 1, 8, 8>(p, st, reduce);
+    if (p.D <= 256) return launch_group<32, 32, 1, 8, 8>(p, st, reduce);
+    return launch_group<32, 32, 2, 8, 4>(p, st, reduce);
+}
+static int dispatch_group4(const SpmmParams &p, cudaStream_t st, bool reduce = true) {
+    if (p.D <= 16) return launch_group<8, 4, 1, 4, 4>(p, st, reduce);
+    if (p.D <= 32) return launch_group<8, 8, 1, 4, 8>(p, st, reduce);
+    if (p.D <= 64) return launch_group<16, 16, 1, 4, 8>(p, st, reduce);
+    if (p.D <= 128) return launch_group<32, 32, 1, 4, 8>(p, st, reduce);
+    if (p.D <= 256) return launch_group<32, 32, 2, 4, 8>(p, st, reduce);
+    return launch_group<32, 32, 4, 4, 4>(p, st, reduce);
+}
+// Widths that are no multiple of four, or rows that are not 16-byte aligned: scalar loads, NV of them per lane and edge
+// (41 floats, 170 k rows x 13 edges: 200 us with one warp and four masked slices per row, 134 us with 16 lanes x 3).
+static int dispatch_group1(const SpmmParams &p, cudaStream_t st) {
+    if (p.D <= 4) return launch_group<8, 4, 1, 1, 4>(p, st);
+    if (p.D <= 8) return launch_group<8, 8, 1, 1, 8>(p, st);
+    if (p.D <= 16) return launch_group<16, 16, 1, 1, 8>(p, st);
+    if (p.D <= 32) return launch_group<16, 16, 2, 1, 4>(p, st);
+    if (p.D <= 48) return launch_group<16, 16, 3, 1, 4>(p, st);
+    if (p.D <= 64) return launch_group<16, 16, 4, 1, 4>(p, st);
+    if (p.D <= 96) return launch_group<32, 32, 3, 1, 4>(p, st);
+    return launch_group<32, 32, 4, 1, 4>(p, st);
 }
 
 }  // namespace yitu
@@ -696,55 +777,47 @@ extern "C" int yitu_spmm_csr_f32(const yitu_spmm_args_t *a, yitu_stream_t stream
     const bool vec_ok = (D % 4 == 0) && (a->x_stride % 4 == 0) && (a->out_stride % 4 == 0) && aligned16(a->x) &&
                         aligned16(a->out) && (p.scratch == nullptr || aligned16(p.scratch)) &&
                         (!per_head || a->n_feats % 4 == 0);
-    if (!vec_ok) return launch<32, 4, 1, 4>(p, per_head, st);
-    // lanes per row / 128-bit slices per lane / edges gathered per step, from a sweep on B200: narrower groups
-    // than the row lose coalescing; deeper unrolling pays while it fits the register budget
-    // rows of more than 128 floats: 256-bit loads (one 1 KiB request per warp and edge) when everything is 32-byte
-    // aligned; measured 6.20 ms against 6.44 ms with 128-bit loads on the D=256 R-MAT workload.  Narrower rows would
-    // need half-warp groups, which lose more than the wider loads gain.
+    // 256-bit loads when every row starts on a 32-byte boundary
     const auto aligned32 = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 31) == 0; };
-    // YITU_SPMM_STREAM (development switch): 0 warp-per-row kernel for everything; 2 edge-stream kernel for everything it
-    // covers, hub chunks included; 3 one of the two by average row length (stream below 24 edges per row);
-    // 1 (default) both: the chunks of the hub rows go to the warp-per-row kernel - long uniform tasks, where its 32
-    // resident warps at 64 registers win - and all other rows to the edge-stream kernel, in two launches on the stream;
-    // for graphs below 64 edges per row (24 for rows of more than 128 floats), the warp-per-row kernel alone above.
-    // Measured on B200, 128 features (ms: warp per row / both / stream alone): R-MAT 16.8 M rows x 31 edges 34.70 /
-    // 32.60 / 35.00; its 8-way shards of 65 M edges each: 7.27 M rows 6.49 / 5.51 / 5.64, 3.07 M rows 4.89 / 4.61 / 4.76,
-    // 1.20 M rows 4.17 / 4.23 / 4.41, 82 k rows (795 per row) 3.43 / 3.68 / 4.03.  256 features, 2.1 M rows x 30: 6.08 /
-    // 6.17 / 6.18.  Uniform graph, 16 edges per row, no hubs: 11.83 / - / 10.74.
+    const bool vec8_ok = vec_ok && D % 8 == 0 && a->x_stride % 8 == 0 && a->out_stride % 8 == 0 && aligned32(a->x) &&
+                         aligned32(a->out) && (p.scratch == nullptr || aligned32(p.scratch)) &&
+                         (!per_head || a->n_feats % 8 == 0);
+    if (per_head) {
+        if (!vec_ok) return launch_heads<32, 4, 1>(p, st);
+        if (vec8_ok && D > 128 && D <= 512) return D <= 256 ? launch_heads<32, 1, 8>(p, st) : launch_heads<32, 2, 8>(p, st);
+        if (D <= 16) return launch_heads<4, 1, 4>(p, st);
+        if (D <= 32) return launch_heads<8, 1, 4>(p, st);
+        if (D <= 64) return launch_heads<16, 1, 4>(p, st);
+        if (D <= 128) return launch_heads<32, 1, 4>(p, st);
+        if (D <= 256) return launch_heads<32, 2, 4>(p, st);
+        return launch_heads<32, 4, 4>(p, st);
+    }
+    if (!vec_ok) return dispatch_group1(p, st);
+
+    // Edge-stream kernel, for rows of 65..256 floats.  It spares a short row its own chain of latencies, but a warp walks
+    // 16 consecutive rows, so it needs a graph of so many rows that the heavy batches of a power-law graph do not become
+    // the tail (50 k rows x 18 edges, 128 floats: 386 us against 69 us with the group kernel) and rows of few edges.
+    // Measured on B200 (us, group / stream), 128 floats: uniform 1 M rows x 16 edges 1276 / 1220, 2 M x 4 edges 1086 / 969;
+    // 256 floats: 1 M x 16 2464 / 2401, 2 M x 4 1905 / 1499, 0.5 M x 32 2163 / 2158.  With hub rows (a chunk schedule) the
+    // chunks go to the group kernel (a whole warp per chunk, two edges per load) and only the other rows are streamed: R-MAT
+    // with 128 floats (ms, group alone / stream alone / both) 16.8 M rows x 31 edges 35.7 / 36.6 / 34.3, 8 M x 8 5.52 / - /
+    // 5.23, 4 M x 15 3.93 / 4.16 / 3.87; below 2 M rows the group kernel alone.
+    // YITU_SPMM_STREAM (development switch): 0 never, 2 for everything the kernel covers, 1 (default) by this rule.
     const int stream_mode = env_int("YITU_SPMM_STREAM", 1);
-    const bool stream_shape = !per_head && g.nnz < (1ll << 31);
-    const bool stream_ok = stream_shape && (stream_mode == 2 || (stream_mode == 3 && g.nnz < 24 * g.n_rows));
-    const bool split = stream_shape && stream_mode == 1 && g.nnz < (D > 128 ? 24 : 64) * g.n_rows;
-    const bool wide256 = D > 128 && D <= 256 && D % 8 == 0 && a->x_stride % 8 == 0 && a->out_stride % 8 == 0 &&
-                         aligned32(a->x) && aligned32(a->out) && (p.scratch == nullptr || aligned32(p.scratch));
-    if (split && (wide256 || (D > 64 && D <= 128))) {
-        if (p.n_chunks > 0) {
+    const bool stream_shape = g.nnz < (1ll << 31) && D > 64 && (D <= 128 || (D <= 256 && vec8_ok));
+    const bool use_stream = stream_shape && (stream_mode == 2 || (stream_mode == 1 && (p.n_chunks > 0
+                            ? D <= 128 && g.n_rows >= (2 << 20) && g.nnz < 64 * g.n_rows
+                            : g.n_rows >= 150000 && g.nnz < 24 * g.n_rows)));
+    if (use_stream) {
+        SpmmParams r = p;
+        if (p.n_chunks > 0 && stream_mode == 1) {
             SpmmParams c = p;
             c.row_tasks = 0;  // the chunks only; the reduction follows the second launch
-            if (int rc = wide256 ? launch<32, 1, 8, 4>(c, false, st, false) : launch<32, 1, 4, 16>(c, false, st, false)) return rc;
+            if (int rc = vec8_ok ? launch_group<32, 16, 1, 8, 8>(c, st, false) : dispatch_group4(c, st, false)) return rc;
+            r.chunk_tasks = 0;  // the rows that are not cut into chunks (those are stepped over), then the reduction
         }
-        SpmmParams r = p;
-        r.chunk_tasks = 0;  // the rows that are not cut into chunks (those are stepped over), then the reduction
-        return wide256 ? dispatch_stream<8, 4, 8>(r, st, 16, 4) : dispatch_stream<4, 8, 16>(r, st, 16, 8);
+        return D > 128 ? dispatch_stream<8, 4, 8>(r, st, 16, 4) : dispatch_stream<4, 8, 16>(r, st, 16, 8);
     }
-    if (stream_ok && wide256) return dispatch_stream<8, 4, 8>(p, st, 16, 4);
-    if (stream_ok && D > 64 && D <= 128) return dispatch_stream<4, 8, 16>(p, st, 16, 8);
-    if (D > 128 && D <= 512 && D % 8 == 0 && a->x_stride % 8 == 0 && a->out_stride % 8 == 0 && aligned32(a->x) &&
-        aligned32(a->out) && (p.scratch == nullptr || aligned32(p.scratch)) && (!per_head || a->n_feats % 8 == 0)) {
-        if (D <= 256) return launch<32, 1, 8, 4>(p, per_head, st);
-        return launch<32, 2, 8, 4>(p, per_head, st);
-    }
-    // rows of 33..64 floats with scalar weights: a full warp per row, four edges per 256-bit load instruction
-    // (measured 0.350 ms against 0.392 ms for half-warp rows on the D=64 hetero workload; for 65..128 floats the same
-    // scheme lost, 37.5 ms against 34.6 ms)
-    if (!per_head && D > 32 && D <= 64 && D % 8 == 0 && a->x_stride % 8 == 0 && a->out_stride % 8 == 0 && aligned32(a->x) &&
-        aligned32(a->out) && (p.scratch == nullptr || aligned32(p.scratch)))
-        return launch_wide<8, 1>(p, st);
-    if (D <= 16) return launch<4, 1, 4, 4>(p, per_head, st);
-    if (D <= 32) return launch<8, 1, 4, 4>(p, per_head, st);
-    if (D <= 64) return launch<16, 1, 4, 4>(p, per_head, st);
-    if (D <= 128) return launch<32, 1, 4, 16>(p, per_head, st);
-    if (D <= 256) return launch<32, 2, 4, 8>(p, per_head, st);
-    return launch<32, 4, 4, 4>(p, per_head, st);
+    if (vec8_ok) return dispatch_group8(p, p.n_chunks == 0 && g.nnz < 8 * g.n_rows, st);
+    return dispatch_group4(p, st);
 }
