@@ -216,6 +216,17 @@ int yitu_spmm_csr_f32_static(const yitu_spmm_args_t *args, yitu_stream_t stream)
 int yitu_epilogue_grad_f32(int64_t n_rows, int64_t n_feats, int32_t activation, const float *y, const float *grad_y,
                            const float *row_scale, float *grad_agg, yitu_stream_t stream);
 
+/* Dense products of the layers around the aggregation, float32 in operands, sums and results.
+ * C[n,N] = A[n,K] B + bias[N] (bias NULL = none); B is [K,N], or [N,K] with b_transposed; ld* are row strides in
+ * floats.  x W^T + b of a layer, x W, and the input gradient g W. */
+int yitu_linear_f32(int64_t n, int64_t K, int64_t N, const float *a, int64_t lda, const float *b, int64_t ldb,
+                    int32_t b_transposed, const float *bias, float *c, int64_t ldc, yitu_stream_t stream);
+/* C[M,N] = A[n,M]^T B[n,N], C contiguous, and (a_sums not NULL) a_sums[M] = column sums of A in the same pass: the
+ * weight and bias gradient of a layer.  Sums are formed in a fixed order: run-to-run identical results. */
+int64_t yitu_gram_scratch_bytes(int64_t n, int64_t M, int64_t N, int32_t column_sums);
+int yitu_gram_f32(int64_t n, int64_t M, int64_t N, const float *a, int64_t lda, const float *b, int64_t ldb, float *c,
+                  float *a_sums, float *scratch, int64_t scratch_bytes, yitu_stream_t stream);
+
 /* values[e] = 1 / (number of edges of e's row that carry e's segment id): with YITU_W_EDGE over a stitched
  * graph this turns the SpMM into "mean per relation, then sum over relations" in ONE pass and one output
  * write per destination row — the mathematics of HeteroGraphConv over GCNLayer with norm = 1/in_degree

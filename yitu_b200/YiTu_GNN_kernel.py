@@ -4,7 +4,8 @@ checks, with every aggregation running in libyitu_b200.so.
 
 The neighbour-group arguments (part_pointers, part2Node, partSize, dimWorker, warpPerBlock) describe the
 reference kernel's own schedule; they are validated like the reference validates them and otherwise unused.
-The dense X*W products stay torch GEMMs, as in the reference (torch::mm, YiTu_GNN_kernel.cu:276,471-472).
+The dense X*W products (torch::mm in the reference, YiTu_GNN_kernel.cu:276,471-472) are float32 throughout: the library's
+own kernels or the library GEMM, whichever is the faster one (ops.matmul, ops.gram).
 
 BACKWARD_USES_FORWARD_CSR: the reference's backward kernels aggregate d_output with the FORWARD CSR
 (YiTu_GNN_kernel.cu:448-466, :733-745), which is the gradient only when the adjacency is symmetric.  The
@@ -54,7 +55,7 @@ def forward(input, weight, row_pointers, column_index, degrees, part_pointers, p
     ops.require_cuda(weight, "weight")
     ops.require_cuda(degrees, "degrees")
     _graph_inputs(row_pointers, column_index, part_pointers, part2Node)
-    tmp = torch.mm(input, weight)
+    tmp = ops.matmul(input, weight)
     g = _prepared(row_pointers, column_index, input.size(0))
     return [ops.spmm(g, tmp, mode=W_NODE, norm_dst=degrees, norm_src=degrees)]
 
@@ -62,6 +63,11 @@ def forward(input, weight, row_pointers, column_index, degrees, part_pointers, p
 def backward(d_output, X, W, row_pointers, column_index, degrees, part_pointers, part2Node, partSize, dimWorker,
              warpPerBlock):
     """[d_input, d_weight] (YiTu_GNN_kernel.cu:422-475): d' = A_hat^T d_output; d' W^T; X^T d'."""
+    return backward_needed(d_output, X, W, row_pointers, column_index, degrees, part_pointers, part2Node, True, True)
+
+
+def backward_needed(d_output, X, W, row_pointers, column_index, degrees, part_pointers, part2Node, need_input, need_weight):
+    """backward() without the gradients that nobody asked for (a first layer's input), which come back as None."""
     ops.require_cuda(d_output, "d_output")
     ops.require_cuda(X, "X")
     ops.require_cuda(W, "W")
@@ -69,7 +75,8 @@ def backward(d_output, X, W, row_pointers, column_index, degrees, part_pointers,
     _graph_inputs(row_pointers, column_index, part_pointers, part2Node)
     g = _prepared(row_pointers, column_index, X.size(0))
     d_prime = _aggregate(g, d_output, True, mode=W_NODE, norm_dst=degrees, norm_src=degrees)
-    return [torch.mm(d_prime, W.transpose(0, 1)), torch.mm(X.transpose(0, 1), d_prime)]
+    return [ops.matmul(d_prime, W, b_transposed=True) if need_input else None,
+            ops.gram(X, d_prime)[0] if need_weight else None]
 
 
 def forward_gin(input, weight, row_pointers, column_index, epsilon, part_pointers, part2Node, partSize, dimWorker,
@@ -80,18 +87,27 @@ def forward_gin(input, weight, row_pointers, column_index, epsilon, part_pointer
     _graph_inputs(row_pointers, column_index, part_pointers, part2Node)
     g = _prepared(row_pointers, column_index, input.size(0))
     agg = ops.spmm(g, input, mode=W_NONE, alpha=float(epsilon))
-    return [torch.mm(agg, weight), agg]
+    return [ops.matmul(agg, weight), agg]
 
 
 def backward_gin(d_output, X, W, row_pointers, column_index, epsilon, part_pointers, part2Node, partSize, dimWorker,
                  warpPerBlock):
     """[d_input, d_weight] (YiTu_GNN_kernel.cu:701-823); X is the aggregate saved by forward_gin."""
+    return backward_gin_needed(d_output, X, W, row_pointers, column_index, epsilon, part_pointers, part2Node, True, True)
+
+
+def backward_gin_needed(d_output, X, W, row_pointers, column_index, epsilon, part_pointers, part2Node, need_input,
+                        need_weight):
+    """backward_gin() without the gradients that nobody asked for: a first layer's input gradient costs a product and
+    an aggregation."""
     ops.require_cuda(d_output, "d_output")
     ops.require_cuda(X, "X")
     ops.require_cuda(W, "W")
     _graph_inputs(row_pointers, column_index, part_pointers, part2Node)
-    d_weight = torch.mm(X.transpose(0, 1), d_output)
-    d_input_prime = torch.mm(d_output, W.transpose(0, 1))
+    d_weight = ops.gram(X, d_output)[0] if need_weight else None
+    if not need_input:
+        return [None, d_weight]
+    d_input_prime = ops.matmul(d_output, W, b_transposed=True)
     g = _prepared(row_pointers, column_index, X.size(0))
     d_input = _aggregate(g, d_input_prime, True, mode=W_NONE, alpha=float(epsilon))
     return [d_input, d_weight]

@@ -23,9 +23,9 @@ class GNNAFunction(torch.autograd.Function):
     def backward(ctx, d_output):
         X, weight = ctx.saved_tensors
         info = ctx.inputInfo
-        d_input, d_weight = YiTu_GNN_kernel.backward(
+        d_input, d_weight = YiTu_GNN_kernel.backward_needed(
             d_output.contiguous(), X, weight, info.row_pointers, info.column_index, info.degrees, info.partPtr,
-            info.part2Node, info.partSize, info.dimWorker, info.warpPerBlock)
+            info.part2Node, *ctx.needs_input_grad[:2])
         return d_input, d_weight, None
 
 

@@ -22,9 +22,9 @@ class GNNAFunction_GIN(torch.autograd.Function):
     def backward(ctx, d_output):
         X_agg, weight = ctx.saved_tensors
         info = ctx.inputInfo
-        d_input, d_weight = YiTu_GNN_kernel.backward_gin(
+        d_input, d_weight = YiTu_GNN_kernel.backward_gin_needed(
             d_output.contiguous(), X_agg, weight, info.row_pointers, info.column_index, ctx.eplison, info.partPtr,
-            info.part2Node, info.partSize, info.dimWorker, info.warpPerBlock)
+            info.part2Node, *ctx.needs_input_grad[:2])
         return d_input, d_weight, None, None
 
 

@@ -18,6 +18,44 @@ def _block_of(graph):
     return graph if isinstance(graph, Block) else graph.blk
 
 
+class _LinearFunction(autograd.Function):
+    """x W^T + b with the bias added in the product's epilogue; weight and bias gradient from one pass over x and the
+    gradient (the library takes a pass each, and a slow one for a small result over many rows)."""
+
+    @staticmethod
+    def forward(ctx, x, w, b):
+        ctx.save_for_backward(x, w)
+        return ops.matmul(x, w, b_transposed=True, bias=b)
+
+    @staticmethod
+    def backward(ctx, grad):
+        x, w = ctx.saved_tensors
+        return _linear_grads(grad, x, w, ctx.needs_input_grad)
+
+
+def _linear_grads(grad, x, w, need):
+    """Gradients of x W^T + b with respect to (x, W, b), None where not needed."""
+    if torch.is_grad_enabled():  # a graph of the backward pass is wanted: operators that can be differentiated again
+        return (grad @ w if need[0] else None, grad.t() @ x if need[1] else None, grad.sum(0) if need[2] else None)
+    grad = grad.contiguous()
+    gx = ops.matmul(grad, w) if need[0] else None
+    if not need[1]:
+        return gx, None, grad.sum(0) if need[2] else None
+    return (gx, *ops.gram(grad, x, sums=need[2]))
+
+
+class Linear(nn.Linear):
+    """nn.Linear (same parameters, state and initialisation) whose float32 products on a GPU run in the framework's own
+    dense kernels; every other use is nn.Linear's."""
+
+    def forward(self, x):
+        if (type(x) in (torch.Tensor, nn.Parameter) and x.dim() == 2 and self.bias is not None and x.is_cuda and
+                x.size(1) == self.in_features and ops._dense_kernels_apply(x, self.weight) and
+                ops._dense_rows(self.bias.unsqueeze(0), x.device)):
+            return _LinearFunction.apply(x, self.weight, self.bias)
+        return nn.Linear.forward(self, x)
+
+
 class _AggregateFunction(autograd.Function):
     """y = act(row_scale * (A x) + bias) with fixed per-edge weights (or none): one SpMM with a fused epilogue
     forward; backward one element-wise pass (activation derivative and row scale) and the transposed SpMM."""
@@ -72,7 +110,7 @@ class GCNLayer(nn.Module):
 
     def __init__(self, in_features: int, out_features: int, activation: str = None):
         nn.Module.__init__(self)
-        self.fc = nn.Linear(in_features, out_features)
+        self.fc = Linear(in_features, out_features)
         self.activation = activation
 
     def forward(self, graph, norm, x):
@@ -95,9 +133,9 @@ class GATLayer(nn.Module):
     def __init__(self, in_features: int, out_features: int, n_heads: int, activation: str = None):
         nn.Module.__init__(self)
         self.n_heads, self.n_features, self.activation = n_heads, out_features, activation
-        self.linear_q = nn.Linear(n_heads * out_features, n_heads)
-        self.linear_k = nn.Linear(n_heads * out_features, n_heads)
-        self.linear_v = nn.Linear(in_features, n_heads * out_features)
+        self.linear_q = Linear(n_heads * out_features, n_heads)
+        self.linear_k = Linear(n_heads * out_features, n_heads)
+        self.linear_v = Linear(in_features, n_heads * out_features)
 
     def forward(self, graph, x):
         if isinstance(x, (list, tuple)):
@@ -146,7 +184,7 @@ class _LinearIntoFunction(autograd.Function):
         h = torch.empty(sum(rows), ws[0].size(0), dtype=xs[0].dtype, device=xs[0].device)
         off = 0
         for x, w, b, n in zip(xs, ws, bs, rows):
-            torch.addmm(b, x, w.t(), out=h[off:off + n])
+            ops.matmul(x, w, b_transposed=True, bias=b, out=h[off:off + n])
             off += n
         ctx.n_rel, ctx.rows = n_rel, rows
         ctx.save_for_backward(*xs, *ws)
@@ -162,9 +200,10 @@ class _LinearIntoFunction(autograd.Function):
         for i, (x, w, n) in enumerate(zip(xs, ws, ctx.rows)):
             g = grad_h[off:off + n]
             off += n
-            gxs.append(g @ w if ctx.needs_input_grad[1 + i] else None)
-            gws.append(g.t() @ x if ctx.needs_input_grad[1 + n_rel + i] else None)
-            gbs.append(g.sum(0) if ctx.needs_input_grad[1 + 2 * n_rel + i] else None)
+            gx, gw, gb = _linear_grads(g, x, w, [ctx.needs_input_grad[1 + k * n_rel + i] for k in range(3)])
+            gxs.append(gx)
+            gws.append(gw)
+            gbs.append(gb)
         return (None, *gxs, *gws, *gbs)
 
 
@@ -179,7 +218,7 @@ class StitchedRGCNConv(nn.Module):
         nn.Module.__init__(self)
         assert reduce in ("mean", "sum")
         self.names = [name for name, _ in relations]
-        self.fcs = nn.ModuleDict({name: nn.Linear(in_features, out_features) for name in self.names})
+        self.fcs = nn.ModuleDict({name: Linear(in_features, out_features) for name in self.names})
         self.reduce = reduce
         blocks = [blk for _, blk in relations]
         self.n_src = [blk.size[1] for blk in blocks]

@@ -251,6 +251,70 @@ def spmm(graph, x, *, n_heads=1, mode=W_NONE, edge_values=None, edge_perm=None, 
     return out
 
 
+def _dense_rows(t, device):
+    """A float32 CUDA matrix whose rows are contiguous: what the dense kernels take."""
+    return (type(t) in (torch.Tensor, torch.nn.Parameter) and t.dtype == torch.float32 and t.dim() == 2 and t.device == device and
+            t.is_cuda and t.stride(1) == 1 and t.stride(0) >= t.size(1) > 0 and not t.is_neg())
+
+
+def _dense_kernels_apply(*matrices):
+    """Whether the framework's own dense kernels may stand in for the library GEMM: plain float32 matrices, and full
+    float32 precision asked for (the default; a program that allows TF32 keeps the library's TF32 path)."""
+    device = matrices[0].device
+    return (all(_dense_rows(t, device) for t in matrices) and torch.get_float32_matmul_precision() == "highest" and
+            not torch.is_autocast_enabled("cuda"))
+
+
+def _recorded(*tensors):
+    """Whether autograd records what is done with these tensors (the kernels' results would carry no history)."""
+    return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
+
+
+def matmul(a, b, b_transposed=False, bias=None, out=None):
+    """a b (+ bias), or a b^T (+ bias) with b_transposed, for a matrix a of many rows: yitu_linear_f32, or the library
+    GEMM for other types and where it is the faster one.  Without a bias that is where both widths are large (60 k x
+    128 x 128: 59 us against 55; 20 k x 500 x 500: 256 against 205; 1 M x 64 x 64: 175 against 251); with one the
+    library adds it in a second pass (1 M x 64 x 64: 190 us against 540, 170 k x 128 x 256: 257 against 447, 20 k x 500
+    x 500: 274 against 267).  out: a matrix with contiguous rows that receives the result."""
+    K, N = a.size(-1), b.size(0 if b_transposed else -1)
+    own = min(K, N) <= 64 and max(K, N) <= 256 if bias is None else K * N <= 65536
+    if (not own or a.dim() != 2 or b.dim() != 2 or b.size(1 if b_transposed else 0) != K or not _dense_kernels_apply(a, b) or
+            _recorded(a, b, bias) or
+            (bias is not None and not (bias.dtype == torch.float32 and bias.device == a.device and bias.dim() == 1 and
+                                       bias.numel() == N and bias.is_contiguous())) or
+            (out is not None and not (_dense_rows(out, a.device) and out.size(0) == a.size(0) and out.size(1) == N))):
+        bt = b.t() if b_transposed else b
+        if bias is not None:
+            return torch.addmm(bias, a, bt, out=out)
+        return torch.mm(a, bt, out=out)
+    if out is None:
+        out = torch.empty((a.size(0), N), dtype=torch.float32, device=a.device)
+    with torch.cuda.device(a.device):
+        check(lib().yitu_linear_f32(a.size(0), K, N, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0),
+                                    int(b_transposed), None if bias is None else bias.data_ptr(), out.data_ptr(),
+                                    out.stride(0), _stream(a.device)))
+    return out
+
+
+def gram(a, b, sums=False):
+    """(a^T b, column sums of a or None) for matrices of many rows: yitu_gram_f32 in one pass over a and b; the library's
+    GEMM and reduction for other types and for results of more than 65536 values (20 k x 500 x 500: 341 us against 278;
+    1 M x 64 x 64 with sums: 206 us against 768; 170 k x 128 x 256: 247 against 350)."""
+    if (a.dim() != 2 or b.dim() != 2 or a.size(0) != b.size(0) or a.size(1) * b.size(1) > 65536 or
+            not _dense_kernels_apply(a, b) or _recorded(a, b)):
+        return torch.mm(a.t(), b), a.sum(0) if sums else None
+    n, M, N = a.size(0), a.size(1), b.size(1)
+    L = lib()
+    out = torch.empty((M, N), dtype=torch.float32, device=a.device)
+    s = torch.empty(M, dtype=torch.float32, device=a.device) if sums else None
+    nbytes = L.yitu_gram_scratch_bytes(n, M, N, int(sums))
+    scratch = torch.empty(nbytes // 4, dtype=torch.float32, device=a.device)
+    with torch.cuda.device(a.device):
+        check(L.yitu_gram_f32(n, M, N, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), out.data_ptr(),
+                              s.data_ptr() if sums else None, scratch.data_ptr(), nbytes, _stream(a.device)))
+    return out, s
+
+
 def epilogue_grad(y, grad_y, row_scale=None, activation=None):
     """grad_y * act'(y) * row_scale[r] in one pass (yitu_epilogue_grad_f32); y, grad_y are [n_rows, ...] float32."""
     n_rows = grad_y.size(0)
