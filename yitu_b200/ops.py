@@ -31,8 +31,32 @@ def _ptr(t):
     return None if t is None else C.c_void_p(t.data_ptr())
 
 
+# the raw handles behind torch.cuda.current_stream / current_device (0.1 us instead of 2); a build without them has the
+# public functions
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda i: torch.cuda.current_stream(i).cuda_stream)
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+
+
 def _stream(device):
-    return C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    return C.c_void_p(_raw_stream(device.index))
+
+
+def _addr(t):
+    """Device address of a tensor as ctypes takes it for a void pointer (None for None)."""
+    return None if t is None else t.data_ptr()
+
+
+def _launch(fn, device, *args):
+    """fn(*args, current stream of device) with device current: the guard and the stream object of torch.cuda cost more
+    than the launch itself, so the common case (the device is current) asks for the raw handles only."""
+    i = device.index
+    if _current_device() == i:
+        status = fn(*args, _raw_stream(i))
+    else:
+        with torch.cuda.device(i):
+            status = fn(*args, _raw_stream(i))
+    if status:
+        check(status)
 
 
 def require_cuda(t, name, dtype=None):
@@ -109,7 +133,7 @@ class PreparedGraph:
 
     # hub-row schedule ---------------------------------------------------------------------------
     def plan(self, chunk_edges=DEFAULT_CHUNK_EDGES):
-        """(HubPlan struct or None, tensors kept alive)."""
+        """(HubPlan struct, its two tables, pointer to the struct), or None for a graph without hub rows."""
         if chunk_edges in self._plans:
             return self._plans[chunk_edges]
         L = lib()
@@ -127,7 +151,8 @@ class PreparedGraph:
                 begins = torch.empty(n, dtype=torch.int64, device=self.device)
                 check(L.yitu_hub_plan_fill(C.byref(self.csr), chunk_edges, _ptr(ws), n, _ptr(rows), _ptr(begins),
                                            _stream(self.device)))
-                result = (HubPlan(chunk_edges, 0, n, _ptr(rows), _ptr(begins)), rows, begins)
+                plan = HubPlan(chunk_edges, 0, n, _ptr(rows), _ptr(begins))
+                result = (plan, rows, begins, C.pointer(plan))
         self._plans[chunk_edges] = result
         return result
 
@@ -174,7 +199,7 @@ def prepared(indptr, indices, n_cols, index_mask=0):
     alive (it also pins the memory, so an address cannot be reused while its entry exists), and the derived structures
     die with the last of them.  An in-place modification bumps the version counter and leads to a rebuild."""
     key = (indptr.data_ptr(), indptr.numel(), indptr._version, indices.data_ptr(), indices.numel(), indices._version,
-           str(indptr.device), indptr.dtype, int(n_cols), int(index_mask))
+           indptr.device, indptr.dtype, int(n_cols), int(index_mask))
     g = _PREPARED.get(key)
     if g is None:
         g = PreparedGraph(indptr, indices, n_cols, index_mask)
@@ -203,71 +228,74 @@ def spmm(graph, x, *, n_heads=1, mode=W_NONE, edge_values=None, edge_perm=None, 
     if not x.is_contiguous():
         x = x.contiguous()
     expect(x, "features", device=dev)
-    per_edge = {W_EDGE: graph.nnz, W_EDGE_HEAD: graph.nnz * n_heads}.get(mode)
-    if per_edge is not None and edge_values is None:
-        raise RuntimeError("this weight mode needs edge_values")
-    expect(edge_values, "edge_values", numel=per_edge, device=dev)
-    expect(edge_perm, "edge_perm", numel=graph.nnz, dtype=torch.int32, device=dev)
+    if mode == W_EDGE or mode == W_EDGE_HEAD:
+        if edge_values is None:
+            raise RuntimeError("this weight mode needs edge_values")
+        expect(edge_values, "edge_values", numel=graph.nnz * (n_heads if mode == W_EDGE_HEAD else 1), device=dev)
+    elif edge_values is not None:
+        expect(edge_values, "edge_values", device=dev)
+    if edge_perm is not None:
+        expect(edge_perm, "edge_perm", numel=graph.nnz, dtype=torch.int32, device=dev)
     if mode == W_NODE and (norm_dst is None or norm_src is None):
         raise RuntimeError("W_NODE needs norm_dst and norm_src")
-    expect(norm_dst, "norm_dst", numel=graph.n_rows, device=dev)
-    expect(norm_src, "norm_src", numel=graph.n_cols, device=dev)
-    expect(row_scale, "row_scale", numel=graph.n_rows, device=dev)
-    x2 = x.reshape(x.size(0), -1)
-    x_width = x2.size(1)
+    if norm_dst is not None:
+        expect(norm_dst, "norm_dst", numel=graph.n_rows, device=dev)
+    if norm_src is not None:
+        expect(norm_src, "norm_src", numel=graph.n_cols, device=dev)
+    if row_scale is not None:
+        expect(row_scale, "row_scale", numel=graph.n_rows, device=dev)
+    shape = x.shape
+    x_width = shape[1] if len(shape) == 2 and shape[0] else x.reshape(shape[0], -1).size(1)
     D = x_width * n_heads if x_shared_heads else x_width
     if D % n_heads:
         raise RuntimeError("feature width %d is not a multiple of n_heads=%d" % (D, n_heads))
-    expect(bias, "bias", numel=D, device=dev)
-    expect(out, "out", numel=graph.n_rows * D, device=dev)
+    if bias is not None:
+        expect(bias, "bias", numel=D, device=dev)
     if out is None:
-        shape = (graph.n_rows, n_heads, x_width) if x_shared_heads else (graph.n_rows,) + tuple(x.shape[1:])
-        out = torch.empty(shape, dtype=torch.float32, device=x.device)
+        out = x.new_empty((graph.n_rows, n_heads, x_width) if x_shared_heads else (graph.n_rows, *shape[1:]))
         accumulate = False
-    a = SpmmArgs()
-    a.graph = graph.csr
-    a.n_heads, a.n_feats = n_heads, D // n_heads
-    a.weight_mode, a.accumulate = mode, int(accumulate)
-    a.edge_values, a.edge_perm = _ptr(edge_values), _ptr(edge_perm)
-    a.norm_dst, a.norm_src, a.row_scale = _ptr(norm_dst), _ptr(norm_src), _ptr(row_scale)
-    a.alpha = float(alpha)
-    a.activation = activation_code(activation)
-    a.bias, a.x_shared_heads = _ptr(bias), int(bool(x_shared_heads))
-    a.x, a.x_stride = _ptr(x2), x_width
-    a.out, a.out_stride = _ptr(out), D
-    keep = None
+    else:
+        expect(out, "out", numel=graph.n_rows * D, device=dev)
     if chunk_edges is None:
         chunk_edges = graph.chunk_edges()
+    plan = scratch = None
+    scratch_floats = 0
     if chunk_edges:
         pl = graph.plan(chunk_edges)
         if pl is not None:
-            scratch = torch.empty(pl[0].n_chunks * D, dtype=torch.float32, device=x.device)
-            a.plan = C.pointer(pl[0])
-            a.scratch, a.scratch_bytes = _ptr(scratch), scratch.numel() * 4
-            keep = (pl, scratch)
-    with torch.cuda.device(x.device):
-        check(lib().yitu_spmm_csr_f32(C.byref(a), _stream(x.device)))
-    del keep
+            plan, scratch_floats = pl[3], pl[0].n_chunks * D
+            scratch = x.new_empty(scratch_floats)
+    a = SpmmArgs(graph.csr, n_heads, D // n_heads, mode, bool(accumulate), _addr(edge_values), _addr(edge_perm),
+                 _addr(norm_dst), _addr(norm_src), _addr(row_scale), float(alpha), activation_code(activation), x.data_ptr(),
+                 x_width, out.data_ptr(), D, plan, _addr(scratch), scratch_floats * 4, _addr(bias), bool(x_shared_heads), 0)
+    _launch(lib().yitu_spmm_csr_f32, dev, C.byref(a))
     return out
+
+
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
 
 
 def _dense_rows(t, device):
     """A float32 CUDA matrix whose rows are contiguous: what the dense kernels take."""
-    return (type(t) in (torch.Tensor, torch.nn.Parameter) and t.dtype == torch.float32 and t.dim() == 2 and t.device == device and
-            t.is_cuda and t.stride(1) == 1 and t.stride(0) >= t.size(1) > 0 and not t.is_neg())
+    if type(t) not in _PLAIN or t.dtype != torch.float32 or t.dim() != 2 or t.device != device or t.is_neg():
+        return False
+    stride, width = t.stride(), t.shape[1]
+    return stride[1] == 1 and stride[0] >= width > 0
 
 
-def _dense_kernels_apply(*matrices):
+def _dense_kernels_apply(a, b):
     """Whether the framework's own dense kernels may stand in for the library GEMM: plain float32 matrices, and full
     float32 precision asked for (the default; a program that allows TF32 keeps the library's TF32 path)."""
-    device = matrices[0].device
-    return (all(_dense_rows(t, device) for t in matrices) and torch.get_float32_matmul_precision() == "highest" and
-            not torch.is_autocast_enabled("cuda"))
+    device = a.device
+    return (device.type == "cuda" and _dense_rows(a, device) and _dense_rows(b, device) and
+            torch.get_float32_matmul_precision() == "highest" and not torch.is_autocast_enabled("cuda"))
 
 
 def _recorded(*tensors):
     """Whether autograd records what is done with these tensors (the kernels' results would carry no history)."""
-    return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
+    if not torch.is_grad_enabled():
+        return False
+    return any(t is not None and t.requires_grad for t in tensors)
 
 
 def matmul(a, b, b_transposed=False, bias=None, out=None):
@@ -287,12 +315,11 @@ def matmul(a, b, b_transposed=False, bias=None, out=None):
         if bias is not None:
             return torch.addmm(bias, a, bt, out=out)
         return torch.mm(a, bt, out=out)
+    n = a.size(0)
     if out is None:
-        out = torch.empty((a.size(0), N), dtype=torch.float32, device=a.device)
-    with torch.cuda.device(a.device):
-        check(lib().yitu_linear_f32(a.size(0), K, N, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0),
-                                    int(b_transposed), None if bias is None else bias.data_ptr(), out.data_ptr(),
-                                    out.stride(0), _stream(a.device)))
+        out = a.new_empty((n, N))
+    _launch(lib().yitu_linear_f32, a.device, n, K, N, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), b_transposed,
+            _addr(bias), out.data_ptr(), out.stride(0))
     return out
 
 
@@ -305,13 +332,12 @@ def gram(a, b, sums=False):
         return torch.mm(a.t(), b), a.sum(0) if sums else None
     n, M, N = a.size(0), a.size(1), b.size(1)
     L = lib()
-    out = torch.empty((M, N), dtype=torch.float32, device=a.device)
-    s = torch.empty(M, dtype=torch.float32, device=a.device) if sums else None
-    nbytes = L.yitu_gram_scratch_bytes(n, M, N, int(sums))
-    scratch = torch.empty(nbytes // 4, dtype=torch.float32, device=a.device)
-    with torch.cuda.device(a.device):
-        check(L.yitu_gram_f32(n, M, N, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), out.data_ptr(),
-                              s.data_ptr() if sums else None, scratch.data_ptr(), nbytes, _stream(a.device)))
+    out = a.new_empty((M, N))
+    s = a.new_empty(M) if sums else None
+    nbytes = L.yitu_gram_scratch_bytes(n, M, N, sums)
+    scratch = a.new_empty(nbytes // 4)
+    _launch(L.yitu_gram_f32, a.device, n, M, N, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0), out.data_ptr(),
+            _addr(s), scratch.data_ptr(), nbytes)
     return out, s
 
 
@@ -322,9 +348,8 @@ def epilogue_grad(y, grad_y, row_scale=None, activation=None):
     grad_y = grad_y.contiguous()
     out = torch.empty_like(grad_y)
     code = activation_code(activation)
-    with torch.cuda.device(grad_y.device):
-        check(lib().yitu_epilogue_grad_f32(n_rows, max(width, 1), code, _ptr(y) if code else None, _ptr(grad_y),
-                                           _ptr(row_scale), _ptr(out), _stream(grad_y.device)))
+    _launch(lib().yitu_epilogue_grad_f32, grad_y.device, n_rows, max(width, 1), code, y.data_ptr() if code else None,
+            grad_y.data_ptr(), _addr(row_scale), out.data_ptr())
     return out
 
 
@@ -335,7 +360,7 @@ def _hub_plan(graph, chunk_edges):
     pl = graph.plan(chunk_edges)
     if pl is None:
         return None, 0, None
-    return C.pointer(pl[0]), pl[0].n_chunks, pl
+    return pl[3], pl[0].n_chunks, pl
 
 
 def _heads_feats(graph, x, name):
@@ -384,8 +409,7 @@ def spmm_bwd(graph, values, x, grad_out, chunk_edges=DEFAULT_CHUNK_EDGES):
     if t_plan is not None:
         scratch = torch.empty(t_chunks * H * F, dtype=torch.float32, device=dev)
         a.t_plan, a.scratch, a.scratch_bytes = t_plan, _ptr(scratch), scratch.numel() * 4
-    with torch.cuda.device(dev):
-        check(lib().yitu_spmm_bwd_f32(C.byref(a), _stream(dev)))
+    _launch(lib().yitu_spmm_bwd_f32, dev, C.byref(a))
     del keep
     return grad_values, grad_x
 
@@ -474,8 +498,7 @@ def gat_fwd(graph, query, key, x, slope=0.2, head_mean=False, activation=None, c
         nbytes = L.yitu_gat_fwd_scratch_bytes(n_chunks, H, F)
         scratch = torch.empty(nbytes // 4, dtype=torch.float32, device=dev)
         a.plan, a.scratch, a.scratch_bytes = plan, _ptr(scratch), nbytes
-    with torch.cuda.device(dev):
-        check(L.yitu_gat_fwd_f32(C.byref(a), _stream(dev)))
+    _launch(L.yitu_gat_fwd_f32, dev, C.byref(a))
     del keep
     if head_mean:
         return out, row_max, row_sum, out_heads
@@ -521,8 +544,7 @@ def gat_bwd(graph, query, key, x, out, row_max, row_sum, grad_out, slope=0.2, he
     scratch = torch.empty(max(nbytes // 4, 1), dtype=torch.float32, device=dev)
     b.fwd.plan, b.t_plan = plan, t_plan
     b.scratch, b.scratch_bytes = _ptr(scratch), nbytes
-    with torch.cuda.device(dev):
-        check(L.yitu_gat_bwd_f32(C.byref(b), _stream(dev)))
+    _launch(L.yitu_gat_bwd_f32, dev, C.byref(b))
     del keep, t_keep
     return grad_q, grad_k, grad_x
 
@@ -576,9 +598,7 @@ def degree_norm(indptr, mode=DEG_SQRT):
     YiTu_GNN/data/dataset.py:131-133), 1/sqrt(d), or 1/d."""
     n = indptr.numel() - 1
     out = torch.empty(n, dtype=torch.float32, device=indptr.device)
-    with torch.cuda.device(indptr.device):
-        check(lib().yitu_degree_norm_f32(n, _ptr(indptr), int(indptr.dtype == torch.int64), mode, _ptr(out),
-                                         _stream(indptr.device)))
+    _launch(lib().yitu_degree_norm_f32, indptr.device, n, indptr.data_ptr(), indptr.dtype == torch.int64, mode, out.data_ptr())
     return out
 
 
