@@ -202,6 +202,34 @@ def test_group_kernel_dispatch_edges(oracle, monkeypatch, D, degrees):
         assert bool((out[:, D:] == 7.0).all())
 
 
+@pytest.mark.parametrize("D", [1, 4, 7, 8, 16, 20, 24, 32, 40, 41, 64, 100, 128, 200, 256, 260, 320])
+def test_rows_are_summed_in_the_order_they_are_stored(D):
+    """The order of a row's additions is fixed by its width alone (edge after edge; 33..64 floats in whole 32-byte slices: four
+    interleaved sums), so that the sign of a sum near zero does not depend on the graph around the row."""
+    from yitu_b200 import ops
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(D)
+    degs = torch.tensor([0, 1, 2, 3, 5, 8, 13, 31, 32, 33, 47, 64], device="cuda")
+    indptr = torch.zeros(degs.numel() + 1, dtype=torch.int32, device="cuda")
+    indptr[1:] = degs.cumsum(0).to(torch.int32)
+    n_cols = 300
+    indices = torch.randint(0, n_cols, (int(degs.sum()),), device="cuda", generator=gen).to(torch.int32)
+    x = torch.randn(n_cols, D, device="cuda", generator=gen)
+    g = ops.PreparedGraph(indptr, indices, n_cols)
+    out = ops.spmm(g, x)
+    four = 32 < D <= 64 and D % 8 == 0
+    for r, deg in enumerate(degs.tolist()):
+        rows = x[indices[int(indptr[r]):int(indptr[r]) + deg].long()]
+        parts = []
+        for s in range(4 if four else 1):
+            a = torch.zeros(D, device="cuda")
+            for row in rows[s::4 if four else 1]:
+                a = a + row
+            parts.append(a)
+        ref = (parts[0] + parts[1]) + (parts[2] + parts[3]) if four else parts[0]
+        assert torch.equal(out[r], ref), "D=%d, row of %d edges" % (D, deg)
+
+
 def test_infinite_features_stay_infinite():
     """Lanes behind a row's last edge gather nothing, so an infinite feature sums to infinity and not to NaN."""
     from yitu_b200 import ops

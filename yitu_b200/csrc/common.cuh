@@ -105,6 +105,92 @@ __device__ __forceinline__ void store_vec(float *p, const float (&r)[VEC]) {
     }
 }
 
+// Sums of the hub rows' chunk partials (width W, chunk c at partial + c * stride), handed to finish(row, d, sum).  A CTA of
+// 256 threads looks at eight consecutive chunks, one per warp: the warp that finds its row's first chunk adds a row of up to
+// 16 chunks by itself, longer rows are shared by the whole CTA, every group of threads taking every groups-th chunk.  Added
+// in a fixed order: run-to-run identical.  (One CTA per chunk, most of which leave at once, took 0.95 ms for the chunks of a
+// graph of 520 M edges.)  Launch with (n_chunks + 7) / 8 CTAs.
+struct HubRows {
+    const void *indptr;
+    int is64, chunk_edges;
+    int64_t n_chunks;
+    const int *chunk_row;
+    const int64_t *chunk_begin;
+};
+
+// VEC = 4 takes W, stride and the partials' address as multiples of four floats.
+template <int VEC, typename Finish>
+__device__ __forceinline__ void reduce_hub_rows(const HubRows &h, const float *partial, int64_t stride, int64_t W, Finish finish) {
+    __shared__ float s_part[256][VEC];
+    __shared__ int s_nch[8];
+    __shared__ int64_t s_row[8];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t first = static_cast<int64_t>(blockIdx.x) * 8, chunk = first + w;
+    int nch = 0;
+    int64_t row = 0;
+    if (chunk < h.n_chunks) {
+        row = __ldg(h.chunk_row + chunk);
+        const int64_t rb = load_ptr(h.indptr, h.is64, row);
+        if (__ldg(h.chunk_begin + chunk) == rb)
+            nch = static_cast<int>((load_ptr(h.indptr, h.is64, row + 1) - rb + h.chunk_edges - 1) / h.chunk_edges);
+    }
+    const auto sum = [&](const float *part, int k0, int step, int n, float (&a)[VEC]) {
+#pragma unroll
+        for (int q = 0; q < VEC; ++q) a[q] = 0.0f;
+        for (int k = k0; k < n; k += 8 * step) {
+            float v[8][VEC];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                if (k + u * step < n) {
+                    load_vec<VEC>(v[u], part + static_cast<int64_t>(k + u * step) * stride);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < VEC; ++q) v[u][q] = 0.0f;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+#pragma unroll
+                for (int q = 0; q < VEC; ++q) a[q] += v[u][q];
+        }
+    };
+    const bool alone = nch <= 16;
+    float a[VEC];
+    if (alone && nch > 0)
+        for (int64_t d = lane * VEC; d < W; d += 32 * VEC) {
+            sum(partial + chunk * stride + d, 0, 1, nch, a);
+            finish(row, d, a);
+        }
+    if (lane == 0) {
+        s_nch[w] = alone ? 0 : nch;
+        s_row[w] = row;
+    }
+    __syncthreads();
+    int cols = 8;
+    while (cols * VEC < W && cols < 256) cols <<= 1;
+    const int tx = threadIdx.x & (cols - 1), grp = threadIdx.x / cols, groups = 256 / cols;
+    for (int i = 0; i < 8; ++i) {
+        if (s_nch[i] == 0) continue;
+        for (int64_t d0 = 0; d0 < W; d0 += cols * VEC) {
+            const int64_t d = d0 + tx * VEC;
+#pragma unroll
+            for (int q = 0; q < VEC; ++q) a[q] = 0.0f;
+            if (d < W) sum(partial + (first + i) * stride + d, grp, groups, s_nch[i], a);
+            if (groups > 1) {
+#pragma unroll
+                for (int q = 0; q < VEC; ++q) s_part[threadIdx.x][q] = a[q];
+                __syncthreads();
+                if (grp == 0)
+                    for (int g = 1; g < groups; ++g)
+#pragma unroll
+                        for (int q = 0; q < VEC; ++q) a[q] += s_part[g * cols + tx][q];
+                __syncthreads();
+            }
+            if (grp == 0 && d < W) finish(s_row[i], d, a);
+        }
+    }
+}
+
 inline int validate_csr(const yitu_csr_t *g) {
     YITU_REQUIRE(g != nullptr, YITU_ERR_INVALID_ARG, "graph is NULL");
     YITU_REQUIRE(g->n_rows >= 0 && g->n_cols >= 0 && g->nnz >= 0, YITU_ERR_INVALID_ARG,

@@ -51,6 +51,7 @@ struct SpmmParams {
     float *scratch;
     const float *bias;
     int act, xshared;
+    int node_late;  // W_NODE: the destination's factor is applied to the row's sum instead of to every edge
 };
 
 // Last step of every output row: bias, then activation (both optional).
@@ -200,36 +201,38 @@ __global__ void __launch_bounds__(256) spmm_heads_kernel(const __grid_constant__
 //   What bounds it: DRAM and L2 bandwidth for wide rows; for narrow ones the chain of three dependent latencies per row
 // (row pointer, ids, gathers).  A row's edges are therefore gathered 8 to 16 at a time, and the next tile of ids is
 // requested before the current one is consumed.
-template <int RW, int LPE, int NV, int VEC, int EU, bool IDX32>
-__global__ void __launch_bounds__(128) spmm_group_kernel(const __grid_constant__ SpmmParams p) {
+template <int RW, int LPE, int NV, int VEC, int EU, bool IDX32, int CTAS>
+__global__ void __launch_bounds__(128, CTAS) spmm_group_kernel(const __grid_constant__ SpmmParams p) {
     constexpr int EPI = RW / LPE;  // edges per load instruction
     constexpr int STEP = EPI * EU;
     static_assert(RW % LPE == 0 && RW % STEP == 0, "a tile of RW ids is consumed in whole steps");
     const int lane = threadIdx.x & 31;
     const int gl = lane & (RW - 1);
     const int sub = gl / LPE, l = gl & (LPE - 1);
-    const unsigned gmask = (RW == 32) ? 0xffffffffu : (((1u << (RW & 31)) - 1u) << (lane & ~(RW - 1)));
+    constexpr unsigned FULL = 0xffffffffu;
     const int64_t gid = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / RW;
     const int64_t d0 = static_cast<int64_t>(blockIdx.y) * (LPE * NV * VEC);
-    int64_t row, eb, ee;
-    float *dst;
-    bool raw;
-    if (gid < p.chunk_tasks) {
+    const bool raw = gid < p.chunk_tasks;
+    bool store = true;  // a group without a row, or with a hub row (done by its chunks), keeps its warp company
+    int row;
+    int64_t eb;
+    uint32_t len;  // edges of the row or chunk, counted from eb (registers are what limits the warps per SM here)
+    if (raw) {
         row = __ldg(p.chunk_row + gid);
         eb = __ldg(p.chunk_begin + gid);
-        const int64_t rend = load_ptr(p.indptr, p.is64, row + 1);
-        ee = min(eb + static_cast<int64_t>(p.chunk_edges), rend);
-        dst = p.scratch + gid * p.D;
-        raw = true;
+        len = static_cast<uint32_t>(min(static_cast<int64_t>(p.chunk_edges), load_ptr(p.indptr, p.is64, row + 1) - eb));
     } else {
-        row = gid - p.chunk_tasks;
-        if (row >= p.row_tasks) return;
+        store = gid - p.chunk_tasks < p.row_tasks;
+        row = store ? static_cast<int>(gid - p.chunk_tasks) : 0;
         eb = load_ptr(p.indptr, p.is64, row);
-        ee = load_ptr(p.indptr, p.is64, row + 1);
-        if (p.n_chunks > 0 && ee - eb > p.chunk_edges) return;  // hub row: done by its chunks
-        dst = p.out + row * p.os;
-        raw = false;
+        len = static_cast<uint32_t>(load_ptr(p.indptr, p.is64, row + 1) - eb);
+        store = store && !(p.n_chunks > 0 && len > static_cast<uint32_t>(p.chunk_edges));
+        if (!store) {
+            if (RW == 32) return;
+            len = 0;
+        }
     }
+    const int *ids = p.indices + eb;
     int off[NV];
     bool valid[NV];
     float acc[NV][VEC];
@@ -241,39 +244,41 @@ __global__ void __launch_bounds__(128) spmm_group_kernel(const __grid_constant__
         for (int q = 0; q < VEC; ++q) acc[i][q] = 0.0f;
     }
     const float nd = (p.wmode == YITU_W_NODE) ? __ldg(p.norm_dst + row) : 0.0f;
+    const float nd_edge = p.node_late ? 1.0f : nd;
 
-    auto load_tile = [&](int64_t e0, int &col, float &w) {
+    auto load_tile = [&](uint32_t e, int &col, float &w) {  // e: this lane's edge of the tile
         col = 0;
         w = 0.0f;
-        const int64_t e = e0 + gl;
-        if (e < ee) {
-            const int rawidx = ld_stream(p.indices + e);
+        if (e < len) {
+            const int rawidx = ld_stream(ids + e);
             col = p.mask ? (rawidx & p.mask) : rawidx;
             if (p.wmode == YITU_W_NONE) {
                 w = 1.0f;
             } else if (p.wmode == YITU_W_NODE) {
-                w = nd * __ldg(p.norm_src + col);
+                w = nd_edge * __ldg(p.norm_src + col);
             } else {
-                const int64_t vi = p.perm ? static_cast<int64_t>(ld_stream(p.perm + e)) : e;
-                w = ld_stream(p.values + vi);
+                w = ld_stream(p.values + (p.perm ? static_cast<int64_t>(ld_stream(p.perm + eb + e)) : eb + e));
             }
         }
     };
     int my_col;
     float my_w;
-    load_tile(eb, my_col, my_w);
-    for (int64_t e0 = eb; e0 < ee; e0 += RW) {
-        const int n = static_cast<int>(min(static_cast<int64_t>(RW), ee - e0));
+    load_tile(gl, my_col, my_w);
+    // with several rows per warp every group takes the trips of the longest: groups that leave each other would execute one
+    // after the other
+    for (uint32_t e0 = 0; RW == 32 ? e0 < len : __any_sync(FULL, e0 < len); e0 += RW) {
+        const int n = e0 < len ? static_cast<int>(min(static_cast<uint32_t>(RW), len - e0)) : 0;
+        const int most = RW == 32 ? n : __reduce_max_sync(FULL, n);
         int nx_col = 0;
         float nx_w = 0.0f;
-        if (e0 + RW < ee) load_tile(e0 + RW, nx_col, nx_w);
-        for (int j = 0; j < n; j += STEP) {
+        load_tile(e0 + RW + gl, nx_col, nx_w);
+        for (int j = 0; j < most; j += STEP) {
             int c[EU];
             float w[EU];
 #pragma unroll
             for (int u = 0; u < EU; ++u) {
-                c[u] = __shfl_sync(gmask, my_col, j + u * EPI + sub, RW);
-                w[u] = __shfl_sync(gmask, my_w, j + u * EPI + sub, RW);  // 0 behind the last edge
+                c[u] = __shfl_sync(FULL, my_col, j + u * EPI + sub, RW);
+                w[u] = __shfl_sync(FULL, my_w, j + u * EPI + sub, RW);  // 0 behind the last edge
             }
             float v[EU][NV][VEC];
 #pragma unroll
@@ -318,18 +323,21 @@ __global__ void __launch_bounds__(128) spmm_group_kernel(const __grid_constant__
                     if (q < half) {
                         const float send = upper ? acc[i][q] : acc[i][q + half];
                         const float keep = upper ? acc[i][q + half] : acc[i][q];
-                        acc[i][q] = keep + __shfl_xor_sync(gmask, send, o, RW);
+                        acc[i][q] = keep + __shfl_xor_sync(FULL, send, o, RW);
                     }
             if (upper) piece_at += half;
             have = half;
         } else {
 #pragma unroll
-            for (int i = 0; i < NV; ++i) acc[i][0] += __shfl_xor_sync(gmask, acc[i][0], o, RW);
+            for (int i = 0; i < NV; ++i) acc[i][0] += __shfl_xor_sync(FULL, acc[i][0], o, RW);
             owner = owner && !upper;
         }
     }
-    if (!owner) return;
-    const float s = raw ? 1.0f : p.alpha * (p.row_scale ? __ldg(p.row_scale + row) : 1.0f);
+    if (!owner || !store) return;
+    float *dst = raw ? p.scratch + gid * p.D : p.out + row * p.os;
+    // a hub row's chunk is left unscaled, but fully weighted
+    float s = raw ? 1.0f : p.alpha * (p.row_scale ? __ldg(p.row_scale + row) : 1.0f);
+    if (p.node_late) s *= nd;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         if (!valid[i]) continue;
@@ -337,7 +345,12 @@ __global__ void __launch_bounds__(128) spmm_group_kernel(const __grid_constant__
         float r[PIECE];
 #pragma unroll
         for (int q = 0; q < PIECE; ++q) r[q] = acc[i][q];
-        if (!raw) {
+        if (raw) {
+            if (p.node_late) {
+#pragma unroll
+                for (int q = 0; q < PIECE; ++q) r[q] *= s;
+            }
+        } else {
             if (p.accumulate) {
                 float old[PIECE];
                 load_vec<PIECE>(old, dst + at);
@@ -558,49 +571,32 @@ __global__ void __launch_bounds__(128, (VEC * EU <= 32) ? 6 : 4) spmm_stream_ker
     flush(INT32_MAX);
 }
 
-// Adds the chunk partials of each hub row and applies the epilogue.  One CTA per hub row (the CTAs of a row's later
-// chunks leave at once): `cols` threads span the features and the others split the chunks, each group summing every
-// groups-th chunk; thread 0 of a feature then adds the groups in order, so the sum is the same in every run.  A serial
-// loop over the chunks made a row of a few hundred chunks the tail of the whole aggregation.
-__global__ void __launch_bounds__(256) hub_reduce_kernel(const __grid_constant__ SpmmParams p, int cols) {
-    __shared__ float s_part[256];
-    const int64_t chunk = blockIdx.x;
-    const int64_t row = __ldg(p.chunk_row + chunk);
-    const int64_t rb = load_ptr(p.indptr, p.is64, row);
-    if (__ldg(p.chunk_begin + chunk) != rb) return;  // only a row's first chunk reduces
-    const int64_t re = load_ptr(p.indptr, p.is64, row + 1);
-    const int nch = static_cast<int>((re - rb + p.chunk_edges - 1) / p.chunk_edges);
-    const float s = p.alpha * (p.row_scale ? __ldg(p.row_scale + row) : 1.0f);
-    const int tx = threadIdx.x & (cols - 1), grp = threadIdx.x / cols, groups = blockDim.x / cols;
-    const float *part = p.scratch + chunk * p.D;
-    for (int64_t d0 = 0; d0 < p.D; d0 += cols) {
-        const int64_t d = d0 + tx;
-        float a = 0.0f;
-        if (d < p.D) {
-#pragma unroll 4
-            for (int k = grp; k < nch; k += groups) a += part[k * p.D + d];
+// Adds the chunk partials of each hub row and applies the epilogue.
+template <int VEC>
+__global__ void __launch_bounds__(256) hub_reduce_kernel(const __grid_constant__ SpmmParams p) {
+    const HubRows h{p.indptr, p.is64, p.chunk_edges, p.n_chunks, p.chunk_row, p.chunk_begin};
+    reduce_hub_rows<VEC>(h, p.scratch, p.D, p.D, [&](int64_t row, int64_t d, float (&a)[VEC]) {
+        const float s = p.alpha * (p.row_scale ? __ldg(p.row_scale + row) : 1.0f);
+        float *o = p.out + row * p.os + d;
+        float r[VEC];
+        if (p.accumulate) {
+            load_vec<VEC>(r, o);
+#pragma unroll
+            for (int q = 0; q < VEC; ++q) r[q] = fmaf(s, a[q], r[q]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < VEC; ++q) r[q] = s * a[q];
         }
-        if (groups > 1) {
-            s_part[threadIdx.x] = a;
-            __syncthreads();
-            if (grp == 0)
-                for (int g = 1; g < groups && g < nch; ++g) a += s_part[g * cols + tx];
-            __syncthreads();
-        }
-        if (grp == 0 && d < p.D) {
-            float *o = p.out + row * p.os + d;
-            float r = p.accumulate ? fmaf(s, a, *o) : s * a;
-            if (p.bias) r += __ldg(p.bias + d);
-            *o = activate(r, p.act);
-        }
-    }
+        finish_vec<VEC>(r, p, d);
+        store_vec<VEC>(o, r);
+    });
 }
 
 static int launch_hub_reduce(const SpmmParams &p, cudaStream_t st) {
     if (p.n_chunks == 0) return YITU_OK;
-    int cols = 16;
-    while (cols < p.D && cols < 256) cols <<= 1;
-    hub_reduce_kernel<<<static_cast<unsigned>(p.n_chunks), 256, 0, st>>>(p, cols);
+    const unsigned grid = static_cast<unsigned>((p.n_chunks + 7) / 8);
+    if (p.D % 4 == 0 && p.os % 4 == 0 && aligned16(p.out) && aligned16(p.scratch)) hub_reduce_kernel<4><<<grid, 256, 0, st>>>(p);
+    else hub_reduce_kernel<1><<<grid, 256, 0, st>>>(p);
     YITU_LAUNCH_CHECK();
     return YITU_OK;
 }
@@ -671,7 +667,7 @@ static int dispatch_stream(const SpmmParams &p, cudaStream_t st, int rows_dflt, 
     return launch_stream<VEC, EU_A, 16>(p, st);
 }
 
-template <int RW, int LPE, int NV, int VEC, int EU>
+template <int RW, int LPE, int NV, int VEC, int EU, int CTAS = 1>
 static int launch_group(const SpmmParams &p, cudaStream_t st, bool reduce = true) {
     const int64_t groups = p.chunk_tasks + p.row_tasks;
     if (groups == 0) return YITU_OK;
@@ -681,46 +677,49 @@ static int launch_group(const SpmmParams &p, cudaStream_t st, bool reduce = true
     YITU_REQUIRE(gx < (1ll << 31) && gy <= 65535, YITU_ERR_LIMIT, "spmm grid too large (%lld x %lld)",
                  (long long)gx, (long long)gy);
     dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
-    if (p.n_cols * p.xs < (1ll << 32)) spmm_group_kernel<RW, LPE, NV, VEC, EU, true><<<grid, threads, 0, st>>>(p);
-    else spmm_group_kernel<RW, LPE, NV, VEC, EU, false><<<grid, threads, 0, st>>>(p);
+    if (p.n_cols * p.xs < (1ll << 32)) spmm_group_kernel<RW, LPE, NV, VEC, EU, true, CTAS><<<grid, threads, 0, st>>>(p);
+    else spmm_group_kernel<RW, LPE, NV, VEC, EU, false, CTAS><<<grid, threads, 0, st>>>(p);
     YITU_LAUNCH_CHECK();
     return reduce ? launch_hub_reduce(p, st) : YITU_OK;
 }
 
-// Lanes per row (RW), lanes per edge and edges per step of spmm_group_kernel by row width.  The narrowest group that
-// covers a source row wins on every graph that fills the machine: four rows of 64 floats per warp instead of one keep
-// four times as many dependent chains in flight and need no sum across lanes (uniform graph, 1 M rows x 16 edges, us, by
-// lanes per row 32 / 16 / 8: 64 floats 917 / 793 / 680; 16 floats 860 / 395 / 313).  Rows of at most 32 floats keep 8 lanes,
-// two or four edges per load instruction, so that a power-law graph's long rows do not hold up their warp (1 M rows x 15
-// edges, 32 floats: 474 us with 4 lanes, 460 with 8); below 8 edges per row and without hub rows there is nothing to hold
-// up and the narrowest group is taken (2 M rows x 4 edges: 16 floats 365 -> 266, 32 floats 440 -> 364).
-static int dispatch_group8(const SpmmParams &p, bool short_rows, cudaStream_t st, bool reduce = true) {
-    if (p.D <= 16) return short_rows ? launch_group<2, 2, 1, 8, 2>(p, st, reduce) : launch_group<8, 2, 1, 8, 2>(p, st, reduce);
-    if (p.D <= 32) return short_rows ? launch_group<4, 4, 1, 8, 4>(p, st, reduce) : launch_group<8, 4, 1, 8, 4>(p, st, reduce);
-    if (p.D <= 64) return launch_group<8, 8, 1, 8, 8>(p, st, reduce);
-    if (p.D <= 128) return launch_group<16, 16, 1, 8, 8>(p, st, reduce);
-    if (p.D <= 256) return launch_group<32, 32, 1, 8, 8>(p, st, reduce);
-    return launch_group<32, 32, 2, 8, 4>(p, st, reduce);
-}
+// Lanes per row (RW), lanes per edge, edges per step and resident CTAs of spmm_group_kernel by row width, from sweeps on B200
+// over uniform and R-MAT graphs of 16 k to 2 M rows.  What decides below 256 floats is how many dependent chains are in flight:
+// the narrowest group that covers a source row (four rows of 32 floats per warp), and few registers, so that 12 or 16 CTAs of
+// 128 threads fit an SM - a register bound that leaves one or two gathers of a chain in flight beats deeper unrolling at half
+// the warps (1 M rows x 16 edges, us: 32 floats 331 at 40 registers, 480 with two edges per step, 368 with eight and no bound;
+// R-MAT 1 M x 15, 64 floats 560 at 32 registers, 677 without the bound; 128 floats 808 at 32 registers, 910 without).
+// Rows of 33..64 floats are the exception to the narrow group: a warp per row, four edges per load, is as fast on uniform
+// graphs (660 us against 671) and faster on power-law ones, where the longest of a warp's rows holds up the others (R-MAT
+// 1 M x 15: 511 against 624).
+// Every row's edges are summed in the order the CSR stores them, rows of 33..64 floats in four interleaved sums: the order
+// does not depend on the graph's size, so a ReLU behind the sum sees the same signs whatever form is taken here.
 static int dispatch_group4(const SpmmParams &p, cudaStream_t st, bool reduce = true) {
-    if (p.D <= 16) return launch_group<8, 4, 1, 4, 4>(p, st, reduce);
-    if (p.D <= 32) return launch_group<8, 8, 1, 4, 8>(p, st, reduce);
+    if (p.D <= 16) return launch_group<4, 4, 1, 4, 4, 16>(p, st, reduce);
+    if (p.D <= 32) return launch_group<8, 8, 1, 4, 4, 12>(p, st, reduce);
     if (p.D <= 64) return launch_group<16, 16, 1, 4, 8>(p, st, reduce);
-    if (p.D <= 128) return launch_group<32, 32, 1, 4, 8>(p, st, reduce);
+    if (p.D <= 128) return launch_group<32, 32, 1, 4, 2, 12>(p, st, reduce);
     if (p.D <= 256) return launch_group<32, 32, 2, 4, 8>(p, st, reduce);
     return launch_group<32, 32, 4, 4, 4>(p, st, reduce);
 }
+static int dispatch_group8(const SpmmParams &p, cudaStream_t st, bool reduce = true) {
+    if (p.D <= 32) return dispatch_group4(p, st, reduce);
+    if (p.D <= 64) return launch_group<32, 8, 1, 8, 1, 16>(p, st, reduce);
+    if (p.D <= 128) return launch_group<16, 16, 1, 8, 2, 12>(p, st, reduce);
+    if (p.D <= 256) return launch_group<32, 32, 1, 8, 2>(p, st, reduce);
+    return launch_group<32, 32, 2, 8, 4>(p, st, reduce);
+}
 // Widths that are no multiple of four, or rows that are not 16-byte aligned: scalar loads, NV of them per lane and edge
-// (41 floats, 170 k rows x 13 edges: 200 us with one warp and four masked slices per row, 134 us with 16 lanes x 3).
+// (41 floats, 170 k rows x 13 edges: 200 us with one warp and four masked slices per row, 120 us with 16 lanes x 3).
 static int dispatch_group1(const SpmmParams &p, cudaStream_t st) {
-    if (p.D <= 4) return launch_group<8, 4, 1, 1, 4>(p, st);
-    if (p.D <= 8) return launch_group<8, 8, 1, 1, 8>(p, st);
-    if (p.D <= 16) return launch_group<16, 16, 1, 1, 8>(p, st);
-    if (p.D <= 32) return launch_group<16, 16, 2, 1, 4>(p, st);
-    if (p.D <= 48) return launch_group<16, 16, 3, 1, 4>(p, st);
-    if (p.D <= 64) return launch_group<16, 16, 4, 1, 4>(p, st);
-    if (p.D <= 96) return launch_group<32, 32, 3, 1, 4>(p, st);
-    return launch_group<32, 32, 4, 1, 4>(p, st);
+    if (p.D <= 4) return launch_group<4, 4, 1, 1, 4, 16>(p, st);
+    if (p.D <= 8) return launch_group<8, 8, 1, 1, 8, 16>(p, st);
+    if (p.D <= 16) return launch_group<16, 16, 1, 1, 8, 12>(p, st);
+    if (p.D <= 32) return launch_group<16, 16, 2, 1, 4, 12>(p, st);
+    if (p.D <= 48) return launch_group<16, 16, 3, 1, 2, 16>(p, st);
+    if (p.D <= 64) return launch_group<16, 16, 4, 1, 2, 12>(p, st);
+    if (p.D <= 96) return launch_group<32, 32, 3, 1, 2, 12>(p, st);
+    return launch_group<32, 32, 4, 1, 2, 12>(p, st);
 }
 
 }  // namespace yitu
@@ -797,8 +796,8 @@ extern "C" int yitu_spmm_csr_f32(const yitu_spmm_args_t *a, yitu_stream_t stream
     // Edge-stream kernel, for rows of 65..256 floats.  It spares a short row its own chain of latencies, but a warp walks
     // 16 consecutive rows, so it needs a graph of so many rows that the heavy batches of a power-law graph do not become
     // the tail (50 k rows x 18 edges, 128 floats: 386 us against 69 us with the group kernel) and rows of few edges.
-    // Measured on B200 (us, group / stream), 128 floats: uniform 1 M rows x 16 edges 1276 / 1220, 2 M x 4 edges 1086 / 969;
-    // 256 floats: 1 M x 16 2464 / 2401, 2 M x 4 1905 / 1499, 0.5 M x 32 2163 / 2158.  With hub rows (a chunk schedule) the
+    // Measured on B200 (us, group / stream), 128 floats: uniform 1 M rows x 16 edges 1246 / 1220, 2 M x 4 edges 908 / 969;
+    // 100 floats 1275 / 1196, 1085 / 991; 256 floats 2458 / 2396, 1640 / 1499.  With hub rows (a chunk schedule) the
     // chunks go to the group kernel (a whole warp per chunk, two edges per load) and only the other rows are streamed: R-MAT
     // with 128 floats (ms, group alone / stream alone / both) 16.8 M rows x 31 edges 35.7 / 36.6 / 34.3, 8 M x 8 5.52 / - /
     // 5.23, 4 M x 15 3.93 / 4.16 / 3.87; below 2 M rows the group kernel alone.
@@ -807,7 +806,7 @@ extern "C" int yitu_spmm_csr_f32(const yitu_spmm_args_t *a, yitu_stream_t stream
     const bool stream_shape = g.nnz < (1ll << 31) && D > 64 && (D <= 128 || (D <= 256 && vec8_ok));
     const bool use_stream = stream_shape && (stream_mode == 2 || (stream_mode == 1 && (p.n_chunks > 0
                             ? D <= 128 && g.n_rows >= (2 << 20) && g.nnz < 64 * g.n_rows
-                            : g.n_rows >= 150000 && g.nnz < 24 * g.n_rows)));
+                            : g.n_rows >= 150000 && g.nnz < 24 * g.n_rows && !(vec8_ok && D <= 128 && g.nnz < 8 * g.n_rows))));
     if (use_stream) {
         SpmmParams r = p;
         if (p.n_chunks > 0 && stream_mode == 1) {
@@ -818,6 +817,8 @@ extern "C" int yitu_spmm_csr_f32(const yitu_spmm_args_t *a, yitu_stream_t stream
         }
         return D > 128 ? dispatch_stream<8, 4, 8>(r, st, 16, 4) : dispatch_stream<4, 8, 16>(r, st, 16, 8);
     }
-    if (vec8_ok) return dispatch_group8(p, p.n_chunks == 0 && g.nnz < 8 * g.n_rows, st);
+    // rows of few edges: the destination's factor once per row, as the stream kernel does
+    p.node_late = p.wmode == YITU_W_NODE && stream_shape && g.nnz < (D > 128 ? 24 : 64) * g.n_rows;
+    if (vec8_ok) return dispatch_group8(p, st);
     return dispatch_group4(p, st);
 }
