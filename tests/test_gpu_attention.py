@@ -526,3 +526,69 @@ def test_full_size_gat_backward_sampled_rows_against_float64():
         assert float((err - 2e-5 * (truth.abs() + scale)).max()) <= 0, "%s off by %g (scale %g)" % (name, float(err.max()), scale)
         big = truth.abs() >= 0.01 * scale
         record_error("full-size-gat-backward", float(err.max()) / scale, float((err[big] / truth.abs()[big]).max()))
+
+
+GROUP_SHAPES = [(1, 4), (1, 8), (3, 4), (2, 8), (3, 8), (4, 8), (1, 12), (5, 4), (5, 8), (3, 16), (2, 24), (7, 8), (8, 8), (1, 64), (3, 20),
+                (9, 8), (5, 16), (4, 32), (6, 20), (16, 8), (10, 16), (8, 32), (5, 40), (32, 8), (8, 64), (4, 128), (32, 16), (3, 36)]
+
+
+@pytest.mark.parametrize("H,F", GROUP_SHAPES)
+@pytest.mark.parametrize("head_mean", [False, True])
+def test_fused_gat_group_widths(oracle, H, F, head_mean):
+    """Every width class of the fused kernels (lanes per row, slices per lane, lanes per head that are no power of two), rows
+    that end inside, at and behind a tile, hub rows on either side, and tensors that are only 16-byte aligned."""
+    from yitu_b200 import ops
+    rng = np.random.default_rng(100 * H + F)
+    n = 420
+    degs = [0, 1, 2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 0, 31, 32, 33, 63, 64, 65, 200, 2, 1, 0, 300]
+    degs += list(rng.integers(0, 12, n - len(degs)))
+    cols = [np.unique(np.concatenate([rng.choice(n, size=int(k), replace=False), [5, 6] if i % 2 and k else []])).astype(np.int32)
+            for i, k in enumerate(degs)]
+    indptr = np.concatenate([[0], np.cumsum([len(c) for c in cols])]).astype(np.int32)
+    indices = np.concatenate(cols).astype(np.int32)
+    q, k = (rng.standard_normal((n, H)).astype(np.float32) for _ in range(2))
+    x = rng.standard_normal((n, H, F)).astype(np.float32)
+    g_in = rng.standard_normal((n, F) if head_mean else (n, H, F)).astype(np.float32)
+    g_full = (np.repeat(g_in[:, None, :], H, axis=1) / np.float32(H)).astype(np.float32) if head_mean else g_in
+    ref_out, ref_attn = oracle.gat_forward(indptr, indices, q, k, x)
+    rgq, rgk, rgx = oracle.gat_backward(indptr, indices, q, k, x, ref_attn, g_full)
+
+    def shifted(a):  # 16 bytes behind a 32-byte boundary
+        t = torch.empty(a.size + 4, device="cuda")[4:].view(*a.shape)
+        return t.copy_(_dev(a))
+
+    for place, chunk in ((_dev, 64), (_dev, None), (shifted, 64), (_dev, 0)):
+        for dtype in (torch.int32, torch.int64):
+            graph = ops.PreparedGraph(_dev(indptr).to(dtype), _dev(indices), n)
+            dx, dg = place(x), place(g_in)
+            res = ops.gat_fwd(graph, _dev(q), _dev(k), dx, head_mean=head_mean, chunk_edges=chunk)
+            heads = res[3] if head_mean else res[0]
+            assert_close(heads.cpu().numpy(), ref_out, what="per-head %dx%d chunk=%s" % (H, F, chunk))
+            if head_mean:
+                assert_close(res[0].cpu().numpy(), ref_out.astype(np.float64).mean(axis=1), what="head mean %dx%d" % (H, F))
+            gq, gk, gx = ops.gat_bwd(graph, _dev(q), _dev(k), dx, *res[:3], dg, head_mean=head_mean,
+                                     out_heads=res[3] if head_mean else None, chunk_edges=chunk)
+            assert_close(gq.cpu().numpy(), np.asarray(rgq).reshape(gq.shape), rtol=3e-5, what="grad_query %dx%d" % (H, F))
+            assert_close(gk.cpu().numpy(), rgk, rtol=3e-5, what="grad_key %dx%d" % (H, F))
+            assert_close(gx.cpu().numpy(), rgx, rtol=3e-5, what="grad_x %dx%d" % (H, F))
+
+
+@pytest.mark.parametrize("H,F", [(2, 8), (8, 8), (8, 32)])
+def test_fused_gat_with_infinite_scores(H, F):
+    """A key of -inf takes its edges out of the softmax, wherever they stand in the row; a row of such edges alone has no
+    softmax (NaN), and a row without edges is 0."""
+    from yitu_b200 import ops
+    n, deg = 90, 70
+    indptr = torch.tensor([0, deg, deg + 40, deg + 80, deg + 80], dtype=torch.int32, device="cuda")
+    indices = torch.cat([torch.arange(deg), torch.arange(40), torch.arange(50, 90)]).to(torch.int32).cuda()
+    q, k, x = torch.randn(4, H, device="cuda"), torch.randn(n, H, device="cuda"), torch.randn(n, H, F, device="cuda")
+    k[:40] = -float("inf")
+    for chunk in (0, 64):
+        g = ops.PreparedGraph(indptr, indices, n)
+        out = ops.gat_fwd(g, q, k, x, chunk_edges=chunk)[0]
+        for row, cols in ((0, range(40, deg)), (2, range(50, 90))):
+            c = torch.tensor(list(cols), device="cuda")
+            a = torch.softmax(torch.nn.functional.leaky_relu(q[row].double() + k[c].double(), 0.2), dim=0)
+            ref = (a.unsqueeze(-1) * x[c].double()).sum(0)
+            assert float((out[row].double() - ref).abs().max()) <= 1e-5 * float(ref.abs().max()) + 1e-6
+        assert bool(torch.isnan(out[1]).all()) and float(out[3].abs().max()) == 0.0

@@ -23,9 +23,30 @@ namespace yitu {
 
 __device__ __forceinline__ int pow2_shift(int v) { return 31 - __clz(v); }
 
+// Loads that have to be issued where they stand: a plain __ldg may be sunk to its first use, behind the wait for the feature
+// row that was requested with it, which puts its latency on top of the row's.
+__device__ __forceinline__ float load_now(const float *p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+// base + row * bytes as one 32 x 32 + 64 bit multiply-add
+template <typename T>
+__device__ __forceinline__ const T *row_at(const T *base, int row, uint32_t bytes) {
+    return reinterpret_cast<const T *>(reinterpret_cast<const char *>(base) + static_cast<uint64_t>(static_cast<uint32_t>(row)) * bytes);
+}
+__device__ __forceinline__ float4 load_now(const float4 *p) {
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
 // ---------------------------------------------------------------------------------------------------------
-// Stand-alone edge softmax.  One warp per row; a lane is (edge slot, head): HB = pow2 >= min(H,32) lanes
-// span the heads (coalesced key / attn accesses), 32/HB edges advance together.
+// Stand-alone edge softmax.  A lane is (edge slot, head): HB = pow2 >= min(H,32) lanes span the heads (coalesced key / attn
+// accesses).  A warp owns a row; a hub row gets a CTA of 512 threads.  A row of up to four edges per slot is held in
+// registers: ids, segments and scores are read once, all in flight together, whatever the number of segments.  Longer rows
+// are walked four edges per slot at a time, for four segments at once.  (One edge at a time, once per segment and pass, a row was a chain of gathers: the
+// hub rows of 2.4 M edges x 4 heads in 3 segments took 368 us forward and 416 us backward.)
 // ---------------------------------------------------------------------------------------------------------
 struct SoftmaxParams {
     int64_t n_rows;
@@ -42,9 +63,12 @@ struct SoftmaxParams {
     const int64_t *chunk_begin;
 };
 
+constexpr int HUB_THREADS = 512;
+constexpr int SEGS = 4;  // segments whose sums a long row forms in one walk
+
 // Row assignment shared by the stand-alone kernels.  CTA = false: one warp per row, hub rows skipped when a schedule
-// is given.  CTA = true: one 256-thread CTA per hub row (launched with one CTA per chunk; the CTAs of a row's later
-// chunks leave at once), its 256/HB edge slots advancing together.
+// is given.  CTA = true: one CTA per hub row (launched with one CTA per chunk; the CTAs of a row's later
+// chunks leave at once), its edge slots advancing together.
 template <bool CTA>
 __device__ __forceinline__ bool softmax_row(const SoftmaxParams &p, int64_t &row, int64_t &eb, int64_t &ee) {
     if constexpr (CTA) {
@@ -62,123 +86,218 @@ __device__ __forceinline__ bool softmax_row(const SoftmaxParams &p, int64_t &row
     }
 }
 
-// Sum over the edge slots that share a head lane: shuffles inside the warp, then (CTA) across the 8 warps through
-// shared memory, every thread adding the 8 values in the same order.
-template <bool CTA>
-__device__ __forceinline__ float slot_sum(float v, int HB, float *s_red) {
-    for (int o = HB; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+// Sum (or maximum) over the edge slots that share a head lane: shuffles inside the warp, then (CTA) across the warps through
+// shared memory, every thread combining the values in the same order.
+template <bool CTA, bool MAX>
+__device__ __forceinline__ float slot_reduce(float v, int HB, float *s_red) {
+    const auto join = [](float a, float b) { return MAX ? fmaxf(a, b) : a + b; };
+    for (int o = HB; o < 32; o <<= 1) v = join(v, __shfl_xor_sync(0xffffffffu, v, o));
     if constexpr (CTA) {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, hs = lane & (HB - 1);
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, hs = lane & (HB - 1), warps = blockDim.x >> 5;
         __syncthreads();
         if (lane < HB) s_red[warp * 32 + hs] = v;
         __syncthreads();
-        v = 0.0f;
-        for (int w = 0; w < 8; ++w) v += s_red[w * 32 + hs];
+        v = s_red[hs];
+        for (int w = 1; w < warps; ++w) v = join(v, s_red[w * 32 + hs]);
     }
     return v;
 }
 
+// Four edges of a slot: position, segment (-1: none) and column.
+struct Edges4 {
+    int seg[4], col[4];
+    __device__ __forceinline__ void load(const SoftmaxParams &p, int64_t e0, int64_t ee, int ES) {
+        int raw[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) raw[u] = e0 + u * ES < ee ? __ldg(p.indices + e0 + u * ES) : 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            seg[u] = e0 + u * ES < ee ? (p.mask ? static_cast<int>(static_cast<unsigned>(raw[u]) >> 24) : 0) : -1;
+            if (seg[u] >= p.B) seg[u] = -1;  // edges of segments without a query take no part
+            col[u] = p.mask ? (raw[u] & p.mask) : raw[u];
+        }
+    }
+};
+
 template <bool CTA>
-__global__ void __launch_bounds__(256) edge_softmax_fwd_kernel(const __grid_constant__ SoftmaxParams p) {
-    __shared__ float s_red[CTA ? 2 * 8 * 32 : 1];
+__global__ void __launch_bounds__(CTA ? HUB_THREADS : 256) edge_softmax_fwd_kernel(const __grid_constant__ SoftmaxParams p) {
+    __shared__ float s_red[CTA ? HUB_THREADS : 1];
     int64_t row, eb, ee;
     if (!softmax_row<CTA>(p, row, eb, ee)) return;
     const int lane = threadIdx.x & 31;
     const int hs = lane & (p.HB - 1);
     const int slot = (CTA ? threadIdx.x : lane) >> pow2_shift(p.HB);
-    const int ES = (CTA ? 256 : 32) / p.HB;
-    for (int s = 0; s < p.B; ++s) {
-        for (int hc = 0; hc < p.H; hc += p.HB) {
-            const int h = hc + hs;
-            const bool hv = h < p.H;
-            const float qv = hv ? __ldg(p.q + (static_cast<int64_t>(s) * p.n_rows + row) * p.H + h) : 0.0f;
-            float m = -CUDART_INF_F, l = 0.0f;
-            for (int64_t e = eb + slot; e < ee; e += ES) {
-                const int raw = __ldg(p.indices + e);
-                const int bid = p.mask ? static_cast<int>(static_cast<unsigned>(raw) >> 24) : 0;
-                if (bid != s || !hv) continue;
-                const int col = p.mask ? (raw & p.mask) : raw;
-                const float z = leaky_relu(qv + __ldg(p.k + static_cast<int64_t>(col) * p.H + h), p.slope);
-                if (z > m) {
-                    l = l * expf(m - z) + 1.0f;
-                    m = z;
-                } else {
-                    l += expf(z - m);
+    const int ES = (CTA ? HUB_THREADS : 32) / p.HB;
+    const bool held = ee - eb <= 4 * ES;
+    for (int hc = 0; hc < p.H; hc += p.HB) {
+        const int h = hc + hs;
+        const bool hv = h < p.H;
+        const auto query = [&](int s) { return __ldg(p.q + (static_cast<int64_t>(s) * p.n_rows + row) * p.H + h); };
+        const auto scores = [&](const Edges4 &e, int first, int last, float (&z)[4]) {  // of the edges in segments [first, last)
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                z[u] = (hv && e.seg[u] >= first && e.seg[u] < last) ? __ldg(p.k + static_cast<int64_t>(e.col[u]) * p.H + h) : -CUDART_INF_F;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (hv && e.seg[u] >= first && e.seg[u] < last) z[u] = leaky_relu(query(e.seg[u]) + z[u], p.slope);
+        };
+        if (held) {
+            Edges4 e;
+            e.load(p, eb + slot, ee, ES);
+            float z[4];
+            scores(e, 0, p.B, z);
+            for (int s = 0; s < p.B; ++s) {
+                float m = -CUDART_INF_F, l = 0.0f;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (e.seg[u] == s) m = fmaxf(m, z[u]);
+                m = slot_reduce<CTA, true>(m, p.HB, s_red);
+                float w[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    w[u] = e.seg[u] == s ? expf(z[u] - m) : 0.0f;
+                    l += w[u];
+                }
+                l = slot_reduce<CTA, false>(l, p.HB, s_red);
+                const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (hv && e.seg[u] == s) p.attn_out[(eb + slot + u * ES) * p.H + h] = w[u] * inv;
+            }
+            continue;
+        }
+        for (int s0 = 0; s0 < p.B; s0 += SEGS) {
+            float m[SEGS], l[SEGS], z[4];
+#pragma unroll
+            for (int s = 0; s < SEGS; ++s) {
+                m[s] = -CUDART_INF_F;
+                l[s] = 0.0f;
+            }
+            Edges4 e;
+            for (int64_t e0 = eb + slot; e0 < ee; e0 += 4 * ES) {
+                e.load(p, e0, ee, ES);
+                scores(e, s0, s0 + SEGS, z);
+#pragma unroll
+                for (int s = 0; s < SEGS; ++s) {
+                    float top = m[s];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (e.seg[u] == s0 + s) top = fmaxf(top, z[u]);
+                    const float ref = top > -CUDART_INF_F ? top : 0.0f;
+                    if (top > m[s]) l[s] *= expf(m[s] - ref);
+                    m[s] = top;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (e.seg[u] == s0 + s) l[s] += expf(z[u] - ref);
                 }
             }
-            for (int o = p.HB; o < 32; o <<= 1) {
-                const float m2 = __shfl_xor_sync(0xffffffffu, m, o);
-                const float l2 = __shfl_xor_sync(0xffffffffu, l, o);
-                const float M = fmaxf(m, m2);
-                if (M > -CUDART_INF_F) l = l * expf(m - M) + l2 * expf(m2 - M);
-                m = M;
+            float inv[SEGS];
+#pragma unroll
+            for (int s = 0; s < SEGS; ++s) {
+                if (s0 + s >= p.B) break;
+                const float top = slot_reduce<CTA, true>(m[s], p.HB, s_red);
+                if (top > -CUDART_INF_F) l[s] *= expf(m[s] - top);
+                l[s] = slot_reduce<CTA, false>(l[s], p.HB, s_red);
+                m[s] = top;
+                inv[s] = l[s] > 0.0f ? 1.0f / l[s] : 0.0f;
             }
-            if constexpr (CTA) {
-                const int warp = threadIdx.x >> 5;
-                __syncthreads();
-                if (lane < p.HB) {
-                    s_red[warp * 32 + hs] = m;
-                    s_red[256 + warp * 32 + hs] = l;
-                }
-                __syncthreads();
-                float M = -CUDART_INF_F;
-                for (int w = 0; w < 8; ++w) M = fmaxf(M, s_red[w * 32 + hs]);
-                float L = 0.0f;
-                if (M > -CUDART_INF_F)
-                    for (int w = 0; w < 8; ++w) L += s_red[256 + w * 32 + hs] * expf(s_red[w * 32 + hs] - M);
-                m = M;
-                l = L;
-            }
-            const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-            for (int64_t e = eb + slot; e < ee; e += ES) {
-                const int raw = __ldg(p.indices + e);
-                const int bid = p.mask ? static_cast<int>(static_cast<unsigned>(raw) >> 24) : 0;
-                if (bid != s || !hv) continue;
-                const int col = p.mask ? (raw & p.mask) : raw;
-                const float z = leaky_relu(qv + __ldg(p.k + static_cast<int64_t>(col) * p.H + h), p.slope);
-                p.attn_out[e * p.H + h] = expf(z - m) * inv;
+            for (int64_t e0 = eb + slot; e0 < ee; e0 += 4 * ES) {
+                e.load(p, e0, ee, ES);
+                scores(e, s0, s0 + SEGS, z);
+#pragma unroll
+                for (int s = 0; s < SEGS; ++s)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (hv && e.seg[u] == s0 + s) p.attn_out[(e0 + u * ES) * p.H + h] = expf(z[u] - m[s]) * inv[s];
             }
         }
     }
 }
 
 template <bool CTA>
-__global__ void __launch_bounds__(256) edge_softmax_bwd_kernel(const __grid_constant__ SoftmaxParams p) {
-    __shared__ float s_red[CTA ? 8 * 32 : 1];
+__global__ void __launch_bounds__(CTA ? HUB_THREADS : 256, CTA ? 2 : 4) edge_softmax_bwd_kernel(const __grid_constant__ SoftmaxParams p) {
+    __shared__ float s_red[CTA ? HUB_THREADS : 1];
     int64_t row, eb, ee;
     if (!softmax_row<CTA>(p, row, eb, ee)) return;
     const int lane = threadIdx.x & 31;
     const int hs = lane & (p.HB - 1);
     const int slot = (CTA ? threadIdx.x : lane) >> pow2_shift(p.HB);
-    const int ES = (CTA ? 256 : 32) / p.HB;
-    for (int s = 0; s < p.B; ++s) {
-        for (int hc = 0; hc < p.H; hc += p.HB) {
-            const int h = hc + hs;
-            const bool hv = h < p.H;
-            const float qv = hv ? __ldg(p.q + (static_cast<int64_t>(s) * p.n_rows + row) * p.H + h) : 0.0f;
-            float t = 0.0f;  // sum over the segment of attn * grad
-            for (int64_t e = eb + slot; e < ee; e += ES) {
-                const int raw = __ldg(p.indices + e);
-                const int bid = p.mask ? static_cast<int>(static_cast<unsigned>(raw) >> 24) : 0;
-                if (bid != s || !hv) continue;
-                t = fmaf(__ldg(p.attn_in + e * p.H + h), __ldg(p.grad_attn + e * p.H + h), t);
+    const int ES = (CTA ? HUB_THREADS : 32) / p.HB;
+    const bool held = ee - eb <= 4 * ES;
+    for (int hc = 0; hc < p.H; hc += p.HB) {
+        const int h = hc + hs;
+        const bool hv = h < p.H;
+        const auto query = [&](int s) { return __ldg(p.q + (static_cast<int64_t>(s) * p.n_rows + row) * p.H + h); };
+        // attention, its gradient and the sign of the score of four edges, those in segments [first, last)
+        const auto values = [&](const Edges4 &e, int64_t e0, int first, int last, float (&a)[4], float (&g)[4], bool (&neg)[4], bool score) {
+            float kv[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const bool on = hv && e.seg[u] >= first && e.seg[u] < last;
+                a[u] = on ? __ldg(p.attn_in + (e0 + u * ES) * p.H + h) : 0.0f;
+                g[u] = on ? __ldg(p.grad_attn + (e0 + u * ES) * p.H + h) : 0.0f;
+                kv[u] = on && score ? __ldg(p.k + static_cast<int64_t>(e.col[u]) * p.H + h) : 0.0f;
             }
-            t = slot_sum<CTA>(t, p.HB, s_red);
-            float gq = 0.0f;
-            for (int64_t e = eb + slot; e < ee; e += ES) {
-                const int raw = __ldg(p.indices + e);
-                const int bid = p.mask ? static_cast<int>(static_cast<unsigned>(raw) >> 24) : 0;
-                if (bid != s || !hv) continue;
-                const int col = p.mask ? (raw & p.mask) : raw;
-                const float a = __ldg(p.attn_in + e * p.H + h);
-                const float gs = a * (__ldg(p.grad_attn + e * p.H + h) - t);
-                const float z = qv + __ldg(p.k + static_cast<int64_t>(col) * p.H + h);
-                const float gv = gs * (z < 0.0f ? p.slope : 1.0f);
-                p.edge_grad[e * p.H + h] = gv;
-                gq += gv;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                neg[u] = score && hv && e.seg[u] >= first && e.seg[u] < last && query(e.seg[u]) + kv[u] < 0.0f;
+        };
+        float a[4], g[4];
+        bool neg[4];
+        Edges4 e;
+        if (held) {
+            e.load(p, eb + slot, ee, ES);
+            values(e, eb + slot, 0, p.B, a, g, neg, true);
+        }
+        for (int s0 = 0; s0 < p.B; s0 += SEGS) {
+            float t[SEGS], gq[SEGS];  // per segment: sum of attn * grad, sum of the score gradients
+#pragma unroll
+            for (int s = 0; s < SEGS; ++s) t[s] = gq[s] = 0.0f;
+            const auto weigh = [&]() {
+#pragma unroll
+                for (int s = 0; s < SEGS; ++s)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (e.seg[u] == s0 + s) t[s] = fmaf(a[u], g[u], t[s]);
+            };
+            const auto finish = [&](int64_t e0) {
+#pragma unroll
+                for (int s = 0; s < SEGS; ++s)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (hv && e.seg[u] == s0 + s) {
+                            const float gs = a[u] * (g[u] - t[s]), gv = gs * (neg[u] ? p.slope : 1.0f);
+                            p.edge_grad[(e0 + u * ES) * p.H + h] = gv;
+                            gq[s] += gv;
+                        }
+            };
+            if (held) {
+                weigh();
+            } else {
+                for (int64_t e0 = eb + slot; e0 < ee; e0 += 4 * ES) {
+                    e.load(p, e0, ee, ES);
+                    values(e, e0, s0, s0 + SEGS, a, g, neg, false);
+                    weigh();
+                }
             }
-            gq = slot_sum<CTA>(gq, p.HB, s_red);
-            if (slot == 0 && hv) p.grad_q[(static_cast<int64_t>(s) * p.n_rows + row) * p.H + h] = gq;
+#pragma unroll
+            for (int s = 0; s < SEGS; ++s)
+                if (s0 + s < p.B) t[s] = slot_reduce<CTA, false>(t[s], p.HB, s_red);
+            if (held) {
+                finish(eb + slot);
+            } else {
+                for (int64_t e0 = eb + slot; e0 < ee; e0 += 4 * ES) {
+                    e.load(p, e0, ee, ES);
+                    values(e, e0, s0, s0 + SEGS, a, g, neg, true);
+                    finish(e0);
+                }
+            }
+#pragma unroll
+            for (int s = 0; s < SEGS; ++s) {
+                if (s0 + s >= p.B) break;
+                gq[s] = slot_reduce<CTA, false>(gq[s], p.HB, s_red);
+                if (slot == 0 && hv) p.grad_q[(static_cast<int64_t>(s0 + s) * p.n_rows + row) * p.H + h] = gq[s];
+            }
         }
     }
 }
@@ -198,27 +317,60 @@ struct GatherSumParams {
     const int64_t *chunk_begin;
 };
 
-template <bool CTA>
-__global__ void __launch_bounds__(256) edge_gather_sum_kernel(const __grid_constant__ GatherSumParams p) {
-    __shared__ float s_red[CTA ? 8 * 32 : 1];
-    int64_t c, b, e;
-    if constexpr (CTA) {
-        c = __ldg(p.chunk_row + blockIdx.x);
+// A group of RW = max(8, HB) lanes owns one column, or one chunk of a hub column whose sum goes to `partial`: RW / HB edges
+// advance together, eight values per lane in flight.  (A warp per column left most lanes idle at the end of every row: 1 M
+// rows x 16 edges x 4 heads 211 us.)  Without scratch for partial sums (n_parts = 0) hub columns get a CTA each, below.
+template <int RW>
+__global__ void __launch_bounds__(128) edge_gather_sum_kernel(const __grid_constant__ GatherSumParams p, int64_t n_parts, float *partial) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int gl = threadIdx.x & (RW - 1);
+    const int64_t gid = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / RW;
+    const int H = p.H, HB = p.HB, hs = gl & (HB - 1), slot = gl >> pow2_shift(HB), ES = RW / HB;
+    int64_t b = 0, e = 0;
+    float *dst = nullptr;
+    if (gid < n_parts) {
+        b = __ldg(p.chunk_begin + gid);
+        e = min(b + static_cast<int64_t>(p.chunk_edges), load_ptr(p.t_indptr, p.is64, __ldg(p.chunk_row + gid) + 1));
+        dst = partial + gid * H;
+    } else if (gid - n_parts < p.n_cols) {
+        const int64_t c = gid - n_parts;
         b = load_ptr(p.t_indptr, p.is64, c);
-        if (__ldg(p.chunk_begin + blockIdx.x) != b) return;
         e = load_ptr(p.t_indptr, p.is64, c + 1);
-    } else {
-        c = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-        if (c >= p.n_cols) return;
-        b = load_ptr(p.t_indptr, p.is64, c);
-        e = load_ptr(p.t_indptr, p.is64, c + 1);
-        if (p.n_chunks > 0 && e - b > p.chunk_edges) return;
+        if (p.n_chunks > 0 && e - b > p.chunk_edges) e = b;
+        else dst = p.out + c * H;
     }
+    for (int hc = 0; hc < H; hc += HB) {
+        const int h = hc + hs;
+        float a = 0.0f;
+        for (int64_t j0 = b + slot; __any_sync(FULL, j0 < e); j0 += 8 * ES) {
+            int64_t at[8];
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int64_t j = j0 + u * ES;
+                at[u] = j < e ? (p.perm ? static_cast<int64_t>(__ldg(p.perm + j)) : j) : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = (at[u] >= 0 && h < H) ? __ldg(p.vals + at[u] * H + h) : 0.0f;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) a += v[u];
+        }
+        for (int o = HB; o < RW; o <<= 1) a += __shfl_xor_sync(FULL, a, o, RW);
+        if (dst && slot == 0 && h < H) dst[h] = a;
+    }
+}
+
+__global__ void __launch_bounds__(256) edge_gather_sum_hub_kernel(const __grid_constant__ GatherSumParams p) {
+    __shared__ float s_red[8 * 32];
+    const int64_t c = __ldg(p.chunk_row + blockIdx.x);
+    const int64_t b = load_ptr(p.t_indptr, p.is64, c);
+    if (__ldg(p.chunk_begin + blockIdx.x) != b) return;
+    const int64_t e = load_ptr(p.t_indptr, p.is64, c + 1);
     const int lane = threadIdx.x & 31;
     const int H = p.H, HB = p.HB;
     const int hs = lane & (HB - 1);
-    const int slot = (CTA ? threadIdx.x : lane) >> pow2_shift(HB);
-    const int ES = (CTA ? 256 : 32) / HB;
+    const int slot = threadIdx.x >> pow2_shift(HB);
+    const int ES = 256 / HB;
     const int *perm = p.perm;
     const float *vals = p.vals;
     for (int hc = 0; hc < H; hc += HB) {
@@ -238,7 +390,7 @@ __global__ void __launch_bounds__(256) edge_gather_sum_kernel(const __grid_const
             }
             for (; j < e; j += ES) a += __ldg(vals + (perm ? static_cast<int64_t>(__ldg(perm + j)) : j) * H + h);
         }
-        a = slot_sum<CTA>(a, HB, s_red);
+        a = slot_reduce<true, false>(a, HB, s_red);
         if (slot == 0 && h < H) p.out[c * H + h] = a;
     }
 }
@@ -355,22 +507,28 @@ edge_dot_rows_kernel(int64_t n_rows, const void *indptr, int is64, const int *in
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Fused GAT forward.  One warp per destination row, tiles of 32 edges.
-//   per tile: lanes fetch 32 column ids; (edge, head) pairs are spread over the lanes to compute the scores
-//   with coalesced key reads; lane h folds the tile into head h's running (max, sum); then every lane
-//   gathers its NV 128-bit slices of each source row and accumulates p * x.  Accumulators are rescaled when
-//   the running maximum moves (online softmax), and divided by the sum once at the end.
-// Shared memory per warp: 32 column ids, 32*H scores/probabilities, H-sized scale / max / sum / query rows.
+// Fused GAT forward.  A group of RW lanes owns one destination row (or hub chunk); LPE of them cover a source row, NV slices
+// of VEC floats each, and a slice lies inside one head.  A lane therefore computes the scores of its own head's edges itself
+// (q in a register, one 4-byte key per edge, the same address for the lanes of a head) and keeps that head's running maximum
+// and sum: no score ever goes through shared memory, and the key and feature gathers of EU edges are in flight together as
+// soon as the ids are known.  The accumulators are rescaled once per step when the maximum moves (online softmax).  With
+// RW > LPE the sub-groups take different edges and are merged at the end of the row like hub chunks.
+//   Bound by gather bandwidth for wide rows; for narrow ones by the chain of three latencies per row, which is why the
+// narrowest group that covers a row is taken (four rows of 64 floats per warp).  Against a warp per row with the scores of a
+// tile in shared memory (us): uniform 1 M rows x 33 edges 8x32 6500 -> 5610 (6.3 TB/s gathered), 1 M x 17 8x8 2250 -> 756,
+// 4x32 2150 -> 1360, R-MAT 1 M x 16 4x16 1920 -> 753, 131 k x 19 8x8 350 -> 119.
+//   EU and the register bound: four edges per step at 80 registers for up to 128 floats (8x8 uniform: 752; at 64 registers
+// 942, at 94 without a bound 981; two edges 807, eight 1006); wider rows run unbounded (5570; 5860 at 80 registers).
 // ---------------------------------------------------------------------------------------------------------
 struct GatParams {
     int64_t n_rows;
     const void *indptr;
     const int *indices;
-    int is64, H, F, hshift;  // hshift = log2(H) if H is a power of two, else -1
+    int is64, H, F;
     float slope;
     const float *q, *k, *x;
     float *out, *row_max, *row_sum;
-    int head_mean, act, stage;  // stage = floats of per-warp staging for the head mean (H*F or 0)
+    int head_mean, act;
     float *out_heads;           // head_mean: optional per-head result [n_rows,H,F]
     // hub rows: chunk c covers edges [chunk_begin[c], +chunk_edges) of row chunk_row[c]; its unnormalised sums, running
     // maxima and sums go to partial[c] = {H*F, H, H} floats and gat_fwd_merge_kernel finishes the row
@@ -381,255 +539,238 @@ struct GatParams {
     float *partial;
 };
 
-// edges per tile of the fused forward (64: 6.52 against 6.56 ms on the uniform 8x32 layer, but 5.87 against 5.16 ms on the
-// power-law graph, whose many short rows pay for the larger shared-memory footprint)
-constexpr int FWD_TILE = 32;
-__host__ __device__ __forceinline__ int warp_smem_floats_fwd(int H, int stage) {
-    return FWD_TILE + FWD_TILE * H + 4 * 32 + stage;
-}
+// floats of one hub chunk's partial result: H*F sums, then H maxima and H sums (padded so that chunks stay 32-byte aligned
+// when the sums are whole 32-byte slices)
+__host__ __device__ __forceinline__ int64_t fwd_partial_stride(int64_t H, int64_t F) { return H * F + ((2 * H + 7) & ~7ll); }
 
-// floats of one hub chunk's partial result: H*F sums, then H maxima and H sums (padded so that chunks stay 16-byte aligned)
-__host__ __device__ __forceinline__ int64_t fwd_partial_stride(int64_t H, int64_t F) { return H * F + ((2 * H + 3) & ~3ll); }
-
-template <int NV, bool MEAN, bool PLAN>
-__device__ __forceinline__ void gat_fwd_body(const GatParams &p) {
-    extern __shared__ float smem[];
-    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t gid = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + wib;
+template <int RW, int LPE, int NV, int VEC, int EU, int MINB = 1>
+__global__ void __launch_bounds__(128, MINB) gat_fwd_kernel(const __grid_constant__ GatParams p) {
+    constexpr int EPI = RW / LPE, STEP = EPI * EU;
+    static_assert(RW % STEP == 0, "a tile of RW ids is consumed in whole steps");
+    extern __shared__ __align__(16) float smem[];  // head_mean: H*F floats per group
+    const int lane = threadIdx.x & 31, gl = lane & (RW - 1), sub = gl / LPE, l_in = gl & (LPE - 1);
+    constexpr unsigned FULL_WARP = 0xffffffffu;
+    const int64_t gid = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / RW;
     int64_t row, eb, ee;
-    bool chunk = false;  // PLAN = false is the kernel for graphs without hub rows: no schedule logic at all
-    if constexpr (PLAN) {
-        chunk = gid < p.n_chunks;
-        if (chunk) {
-            row = __ldg(p.chunk_row + gid);
-            eb = __ldg(p.chunk_begin + gid);
-            ee = min(eb + static_cast<int64_t>(p.chunk_edges), load_ptr(p.indptr, p.is64, row + 1));
-        } else {
-            row = gid - p.n_chunks;
-            if (row >= p.n_rows) return;
-            eb = load_ptr(p.indptr, p.is64, row);
-            ee = load_ptr(p.indptr, p.is64, row + 1);
-            if (ee - eb > p.chunk_edges) return;  // hub row: done by its chunks
-        }
+    const bool chunk = gid < p.n_chunks;
+    bool store = true;  // a group without a row, or with a hub row (done by its chunks), keeps its warp company
+    if (chunk) {
+        row = __ldg(p.chunk_row + gid);
+        eb = __ldg(p.chunk_begin + gid);
+        ee = min(eb + static_cast<int64_t>(p.chunk_edges), load_ptr(p.indptr, p.is64, row + 1));
     } else {
-        row = gid;
-        if (row >= p.n_rows) return;
+        store = gid - p.n_chunks < p.n_rows;
+        row = store ? gid - p.n_chunks : 0;
         eb = load_ptr(p.indptr, p.is64, row);
         ee = load_ptr(p.indptr, p.is64, row + 1);
+        store = store && !(p.n_chunks > 0 && ee - eb > p.chunk_edges);
+        if (!store) {
+            if (RW == 32) return;
+            ee = eb;
+        }
     }
-    const int H = p.H;
-    float *base = smem + wib * warp_smem_floats_fwd(H, p.stage);
-    int *s_col = reinterpret_cast<int *>(base);
-    float *s_p = base + FWD_TILE;
-    float *s_scale = s_p + FWD_TILE * H;
-    float *s_m = s_scale + 32;
-    float *s_q = s_m + 32;
-    float *s_l = s_q + 32;
-
-    const int64_t D = static_cast<int64_t>(H) * p.F;
-    int hd[NV];
-    bool valid[NV];
-    int64_t off[NV];
+    const int H = p.H, F = p.F, D = H * F;
+    int off[NV], hd[NV];
+    bool valid[NV];  // lanes behind the row's end repeat its first slice and store nothing
+    const float *kp[NV], *xp[NV];
+    float q[NV], m[NV], l[NV], acc[NV][VEC];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-        off[i] = static_cast<int64_t>(i * 32 + lane) * 4;
+        off[i] = (i * LPE + l_in) * VEC;
         valid[i] = off[i] < D;
-        hd[i] = valid[i] ? static_cast<int>(off[i] / p.F) : 0;
+        if (!valid[i]) off[i] = 0;
+        hd[i] = off[i] / F;
+        q[i] = __ldg(p.q + row * H + hd[i]);
+        kp[i] = p.k + hd[i];
+        xp[i] = p.x + off[i];
+        m[i] = -CUDART_INF_F;
+        l[i] = 0.0f;
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) acc[i][v] = 0.0f;
     }
-    float acc[NV][4];
+    const uint32_t k_bytes = static_cast<uint32_t>(H) * 4u, x_bytes = static_cast<uint32_t>(D) * 4u;
+    int my_col = eb + gl < ee ? ld_stream(p.indices + eb + gl) : 0;
+    // EU edges of this lane's sub-group, starting at position j of the tile; FULL: all STEP positions carry an edge
+    auto step = [&](int j, int n, auto full) {
+        constexpr bool FULL = decltype(full)::value;
+        float s[EU][NV], x[EU][NV][VEC];
 #pragma unroll
-    for (int i = 0; i < NV; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
-
-    if (lane < H) s_q[lane] = __ldg(p.q + row * H + lane);
-    float m_run = -CUDART_INF_F, l_run = 0.0f;  // lane h owns head h
-    __syncwarp();
-
-    for (int64_t e0 = eb; e0 < ee; e0 += FWD_TILE) {
-        const int n = static_cast<int>(min(static_cast<int64_t>(FWD_TILE), ee - e0));
-        int my_col[FWD_TILE / 32];
+        for (int u = 0; u < EU; ++u) {
+            const int at = j + u * EPI + sub;
+            const int c = __shfl_sync(FULL_WARP, my_col, at, RW);
 #pragma unroll
-        for (int t = 0; t < FWD_TILE / 32; ++t) my_col[t] = t * 32 + lane < n ? ld_stream(p.indices + e0 + t * 32 + lane) : 0;
-        const int c_first = __shfl_sync(0xffffffffu, my_col[0], 0);
+            for (int i = 0; i < NV; ++i) {
+                if (FULL || at < n) {
+                    s[u][i] = load_now(row_at(kp[i], c, k_bytes));
+                    load_vec<VEC>(x[u][i], row_at(xp[i], c, x_bytes));
+                } else {
+                    s[u][i] = -CUDART_INF_F;
 #pragma unroll
-        for (int t = 0; t < FWD_TILE / 32; ++t) s_col[t * 32 + lane] = t * 32 + lane < n ? my_col[t] : c_first;
-        __syncwarp();
-        const int npairs = n * H;
-        for (int idx = lane; idx < npairs; idx += 32) {
-            const int e = p.hshift >= 0 ? (idx >> p.hshift) : (idx / H);
-            const int h = idx - e * H;
-            s_p[idx] = leaky_relu(s_q[h] + __ldg(p.k + static_cast<int64_t>(s_col[e]) * H + h), p.slope);
-        }
-        __syncwarp();
-        const int n4 = (n + 3) & ~3;
-        if (p.hshift >= 0) {
-            // H a power of two: a lane's pairs idx = lane + 32t all belong to head lane % H, so the tile's maximum and
-            // sum are butterflies over the lanes of equal lane % H; every lane keeps the running statistics of that head
-            float tm = -CUDART_INF_F;
-            for (int idx = lane; idx < npairs; idx += 32) tm = fmaxf(tm, s_p[idx]);
-            for (int o = H; o < 32; o <<= 1) tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, o));
-            const float m_new = fmaxf(m_run, tm);
-            const float sc = expf(m_run - m_new);  // 0 on the first tile (m_run = -inf)
-            if (lane < H) s_scale[lane] = sc;
-            float ls = 0.0f;
-            for (int idx = lane; idx < n4 * H; idx += 32) {
-                const float v = idx < npairs ? expf(s_p[idx] - m_new) : 0.0f;
-                s_p[idx] = v;
-                ls += v;
+                    for (int v = 0; v < VEC; ++v) x[u][i][v] = 0.0f;
+                }
             }
-            for (int o = H; o < 32; o <<= 1) ls += __shfl_xor_sync(0xffffffffu, ls, o);
-            l_run = l_run * sc + ls;
-            m_run = m_new;
-            __syncwarp();
+        }
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            float top = m[i];
+#pragma unroll
+            for (int u = 0; u < EU; ++u) {
+                if (FULL || j + u * EPI + sub < n) s[u][i] = leaky_relu(q[i] + s[u][i], p.slope);
+                top = fmaxf(top, s[u][i]);
+            }
+            // a lane that has met no finite score yet subtracts 0: exp(-inf - 0) = 0 and not NaN
+            const float ref = top > -CUDART_INF_F ? top : 0.0f;
+            const float scale = expf(m[i] - ref);
+            m[i] = top;
+            l[i] *= scale;
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) acc[i][v] *= scale;
+#pragma unroll
+            for (int u = 0; u < EU; ++u) {
+                const float w = expf(s[u][i] - ref);
+                l[i] += w;
+#pragma unroll
+                for (int v = 0; v < VEC; ++v) acc[i][v] = fmaf(w, x[u][i][v], acc[i][v]);
+            }
+        }
+    };
+    // a warp per row walks whole steps without predicates; with several rows per warp every group takes the predicated form
+    // and the trips of the longest, because groups that leave each other execute one after the other
+    for (int64_t e0 = eb; RW == 32 ? e0 < ee : __any_sync(FULL_WARP, e0 < ee); e0 += RW) {
+        const int n = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(RW), ee - e0)));
+        const int nx_col = e0 + RW + gl < ee ? ld_stream(p.indices + e0 + RW + gl) : 0;
+        int j = 0;
+        if constexpr (RW == 32) {
+            for (; j + STEP <= n; j += STEP) step(j, n, std::true_type{});
+            if (j < n) step(j, n, std::false_type{});
         } else {
-            if (lane < H) {
-                float tm = -CUDART_INF_F;
-                for (int e = 0; e < n; ++e) tm = fmaxf(tm, s_p[e * H + lane]);
-                const float m_new = fmaxf(m_run, tm);
-                const float sc = expf(m_run - m_new);  // 0 on the first tile (m_run = -inf)
-                s_scale[lane] = sc;
-                s_m[lane] = m_new;
-                l_run *= sc;
-                m_run = m_new;
-            }
-            __syncwarp();
-            for (int idx = lane; idx < n4 * H; idx += 32) {
-                const int e = idx / H;
-                const int h = idx - e * H;
-                s_p[idx] = idx < npairs ? expf(s_p[idx] - s_m[h]) : 0.0f;
-            }
-            __syncwarp();
-            if (lane < H) {
-                float ls = 0.0f;
-                for (int e = 0; e < n; ++e) ls += s_p[e * H + lane];
-                l_run += ls;
-            }
+            const int most = __reduce_max_sync(FULL_WARP, n);
+            for (; j < most; j += STEP) step(j, n, std::false_type{});
         }
+        my_col = nx_col;
+    }
+    // merge the sub-groups (fixed order: deterministic)
+#pragma unroll
+    for (int o = LPE; o < RW; o <<= 1)
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
-            const float sc = s_scale[hd[i]];
-            acc[i][0] *= sc; acc[i][1] *= sc; acc[i][2] *= sc; acc[i][3] *= sc;
+            const float m2 = __shfl_xor_sync(FULL_WARP, m[i], o, RW), l2 = __shfl_xor_sync(FULL_WARP, l[i], o, RW);
+            const float top = fmaxf(m[i], m2), ref = top > -CUDART_INF_F ? top : 0.0f;
+            const float mine = expf(m[i] - ref), other = expf(m2 - ref);
+            m[i] = top;
+            l[i] = l[i] * mine + l2 * other;
+#pragma unroll
+            for (int v = 0; v < VEC; ++v)
+                acc[i][v] = acc[i][v] * mine + __shfl_xor_sync(FULL_WARP, acc[i][v], o, RW) * other;
         }
-        for (int j = 0; j < n4; j += 4) {
-            float4 v[4][NV];
-            float w[4][NV];
+    if (chunk) {
+        float *part = p.partial + gid * fwd_partial_stride(H, F);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float *xr = p.x + static_cast<int64_t>(s_col[j + u]) * D;
-#pragma unroll
-                for (int i = 0; i < NV; ++i) {
-                    if (valid[i]) {
-                        v[u][i] = __ldg(reinterpret_cast<const float4 *>(xr + off[i]));
-                        w[u][i] = s_p[(j + u) * H + hd[i]];
-                    } else {
-                        v[u][i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        w[u][i] = 0.0f;
-                    }
-                }
+        for (int i = 0; i < NV; ++i) {
+            if (!valid[i] || sub != 0) continue;
+            store_vec<VEC>(part + off[i], acc[i]);
+            if (off[i] == hd[i] * F) {
+                part[D + hd[i]] = m[i];
+                part[D + H + hd[i]] = l[i];
             }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int i = 0; i < NV; ++i) {
-                    acc[i][0] = fmaf(w[u][i], v[u][i].x, acc[i][0]);
-                    acc[i][1] = fmaf(w[u][i], v[u][i].y, acc[i][1]);
-                    acc[i][2] = fmaf(w[u][i], v[u][i].z, acc[i][2]);
-                    acc[i][3] = fmaf(w[u][i], v[u][i].w, acc[i][3]);
-                }
         }
-        __syncwarp();
     }
-    if (PLAN && chunk) {
-        float *part = p.partial + gid * fwd_partial_stride(H, p.F);
+    store = store && !chunk;
+    float *stage = smem + static_cast<int64_t>(threadIdx.x / RW) * D;
 #pragma unroll
-        for (int i = 0; i < NV; ++i)
-            if (valid[i])
-                *reinterpret_cast<float4 *>(part + off[i]) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-        if (lane < H) {
-            part[D + lane] = m_run;
-            part[D + H + lane] = l_run;
+    for (int i = 0; i < NV; ++i) {
+        if (sub != 0 || !valid[i] || !store) continue;
+        // every score of the row is -inf: the softmax is not defined
+        if (ee > eb && m[i] == -CUDART_INF_F) l[i] = CUDART_NAN_F;
+        const float inv = l[i] > 0.0f ? 1.0f / l[i] : (ee > eb ? CUDART_NAN_F : 0.0f);
+        float r[VEC];
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) r[v] = acc[i][v] * inv;
+        if (p.head_mean) {
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) stage[off[i] + v] = r[v];
+            if (p.out_heads) store_vec<VEC>(p.out_heads + row * D + off[i], r);
+        } else {
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) r[v] = activate(r[v], p.act);
+            store_vec<VEC>(p.out + row * D + off[i], r);
         }
-        return;
+        if (off[i] == hd[i] * F) {
+            p.row_max[row * H + hd[i]] = m[i];
+            p.row_sum[row * H + hd[i]] = l[i];
+        }
     }
-    if (lane < H) {
-        s_l[lane] = l_run;
-        p.row_max[row * H + lane] = m_run;
-        p.row_sum[row * H + lane] = l_run;
-    }
+    if (!p.head_mean) return;
+    // the layer's mean over heads: the H values of a feature are added in head order (fixed order: deterministic)
     __syncwarp();
-    if constexpr (MEAN) {
-        // the layer's mean over heads: stage the H*F results, then lane f adds the H values of feature f in head
-        // order (fixed order: deterministic) — the [n_rows,H,F] tensor is never written
-        float *s_o = s_l + 32;
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            if (!valid[i]) continue;
-            const float l = s_l[hd[i]];
-            const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-            const float4 r = make_float4(acc[i][0] * inv, acc[i][1] * inv, acc[i][2] * inv, acc[i][3] * inv);
-            *reinterpret_cast<float4 *>(s_o + off[i]) = r;
-            if (p.out_heads) *reinterpret_cast<float4 *>(p.out_heads + row * D + off[i]) = r;
-        }
-        __syncwarp();
-        const float inv_h = 1.0f / static_cast<float>(H);
-        for (int f = lane; f < p.F; f += 32) {
-            float a = 0.0f;
-            for (int h = 0; h < H; ++h) a += s_o[h * p.F + f];
-            p.out[row * p.F + f] = activate(a * inv_h, p.act);
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            if (!valid[i]) continue;
-            const float l = s_l[hd[i]];
-            const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-            *reinterpret_cast<float4 *>(p.out + row * D + off[i]) =
-                make_float4(activate(acc[i][0] * inv, p.act), activate(acc[i][1] * inv, p.act),
-                            activate(acc[i][2] * inv, p.act), activate(acc[i][3] * inv, p.act));
-        }
+    if (!store) return;
+    const float inv_h = 1.0f / static_cast<float>(H);
+    for (int f = gl; f < F; f += RW) {
+        float a = 0.0f;
+        for (int h = 0; h < H; ++h) a += stage[h * F + f];
+        p.out[row * F + f] = activate(a * inv_h, p.act);
     }
 }
 
-template <int NV, bool MEAN, bool PLAN>
-__global__ void __launch_bounds__(256) gat_fwd_kernel(const __grid_constant__ GatParams p) {
-    gat_fwd_body<NV, MEAN, PLAN>(p);
-}
-
-// The same body held to 64 registers (four 256-thread CTAs per SM).  Left to itself the compiler settles on 48
-// registers for the two-slice head-mean variant and serialises the gathers: 7.2 ms against 6.5 ms on the 8x32 layer.
-template <int NV, bool MEAN, bool PLAN>
-__global__ void __launch_bounds__(256, 4) gat_fwd_kernel_r64(const __grid_constant__ GatParams p) {
-    gat_fwd_body<NV, MEAN, PLAN>(p);
-}
-
-// Finishes the hub rows of the fused forward: combines the chunks' (maximum, sum, unnormalised aggregate) in chunk
-// order.  One CTA per chunk; only the first chunk of a row works.
-__global__ void __launch_bounds__(128) gat_fwd_merge_kernel(const __grid_constant__ GatParams p) {
-    __shared__ float s_m[32], s_inv[32], s_o[512];
+// Finishes the hub rows of the fused forward: combines the chunks' (maximum, sum, unnormalised aggregate).  One CTA per hub
+// row (the CTAs of a row's later chunks leave at once).  The threads split the chunks: `groups` of them share a head (or a
+// feature), each taking every groups-th chunk, and are added in order, so that a row of hundreds of chunks is no serial tail.
+__global__ void __launch_bounds__(256) gat_fwd_merge_kernel(const __grid_constant__ GatParams p) {
+    __shared__ float s_red[256], s_m[32], s_inv[32], s_o[512];
     const int64_t c0 = blockIdx.x;
     const int64_t row = __ldg(p.chunk_row + c0);
     const int64_t rb = load_ptr(p.indptr, p.is64, row);
     if (__ldg(p.chunk_begin + c0) != rb) return;
     const int64_t re = load_ptr(p.indptr, p.is64, row + 1);
     const int nch = static_cast<int>((re - rb + p.chunk_edges - 1) / p.chunk_edges);
-    const int H = p.H, F = p.F, D = H * F;
+    const int H = p.H, F = p.F, D = H * F, t = threadIdx.x;
     const int64_t stride = fwd_partial_stride(H, F);
     const float *part = p.partial + c0 * stride;
-    if (threadIdx.x < H) {
-        const int h = threadIdx.x;
+    {
+        int hb = 1;
+        while (hb < H) hb <<= 1;
+        const int h = t & (hb - 1), g = t / hb, groups = 256 / hb;
         float m = -CUDART_INF_F;
-        for (int c = 0; c < nch; ++c) m = fmaxf(m, part[c * stride + D + h]);
+        if (h < H)
+            for (int c = g; c < nch; c += groups) m = fmaxf(m, part[c * stride + D + h]);
+        s_red[t] = m;
+        __syncthreads();
+        if (g == 0 && h < H) {
+            for (int k = 1; k < groups && k < nch; ++k) m = fmaxf(m, s_red[k * hb + h]);
+            s_m[h] = m;
+        }
+        __syncthreads();
         float l = 0.0f;
-        for (int c = 0; c < nch; ++c) l += part[c * stride + D + H + h] * expf(part[c * stride + D + h] - m);
-        s_m[h] = m;
-        s_inv[h] = l > 0.0f ? 1.0f / l : 0.0f;
-        p.row_max[row * H + h] = m;
-        p.row_sum[row * H + h] = l;
+        if (h < H)
+            for (int c = g; c < nch; c += groups) l += part[c * stride + D + H + h] * expf(part[c * stride + D + h] - s_m[h]);
+        s_red[t] = l;
+        __syncthreads();
+        if (g == 0 && h < H) {
+            for (int k = 1; k < groups && k < nch; ++k) l += s_red[k * hb + h];
+            s_inv[h] = l > 0.0f ? 1.0f / l : CUDART_NAN_F;
+            p.row_max[row * H + h] = s_m[h];
+            p.row_sum[row * H + h] = l;
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    for (int d = threadIdx.x; d < D; d += blockDim.x) {
-        const int h = d / F;
+    int cols = 8;
+    while (cols < D && cols < 256) cols <<= 1;
+    const int tx = t & (cols - 1), g = t / cols, groups = 256 / cols;
+    for (int d0 = 0; d0 < D; d0 += cols) {
+        const int d = d0 + tx, h = d < D ? d / F : 0;
         float a = 0.0f;
-        for (int c = 0; c < nch; ++c) a = fmaf(part[c * stride + d], expf(part[c * stride + D + h] - s_m[h]), a);
+        if (d < D) {
+#pragma unroll 4
+            for (int c = g; c < nch; c += groups) a = fmaf(part[c * stride + d], expf(part[c * stride + D + h] - s_m[h]), a);
+        }
+        if (groups > 1) {
+            s_red[t] = a;
+            __syncthreads();
+            if (g == 0)
+                for (int k = 1; k < groups && k < nch; ++k) a += s_red[k * cols + tx];
+            __syncthreads();
+        }
+        if (g != 0 || d >= D) continue;
         const float v = a * s_inv[h];
         if (p.head_mean) {
             s_o[d] = v;
@@ -641,7 +782,7 @@ __global__ void __launch_bounds__(128) gat_fwd_merge_kernel(const __grid_constan
     if (!p.head_mean) return;
     __syncthreads();
     const float inv_h = 1.0f / static_cast<float>(H);
-    for (int f = threadIdx.x; f < F; f += blockDim.x) {
+    for (int f = t; f < F; f += 256) {
         float a = 0.0f;
         for (int h = 0; h < H; ++h) a += s_o[h * F + f];
         p.out[row * F + f] = activate(a * inv_h, p.act);
@@ -810,7 +951,6 @@ struct GatSrcParams {
     const int *t_rows, *t_perm;
     int H, F;
     float slope;
-    int hshift;             // log2(H) if H is a power of two, else -1
     const float4 *rowpack;  // [n_rows, H]: (query, row max + log row sum, D, unused)
     const float *k, *x;
     const float *g;
@@ -826,229 +966,214 @@ struct GatSrcParams {
     float *grad_values;            // GIVEN: d weight [nnz, H] in CSR order
 };
 
-// rowpack[r,h] = (q, M + log L, <g[r,h,:], out[r,h,:]>, 0); warp per row, 128-bit slices, butterfly inside a head
+// rowpack[r,h] = (q, M + log L, <g[r,h,:], out[r,h,:]>, 0).  One thread per 128-bit slice, the rows end to end; the F / 4
+// lanes of a head are added by a butterfly, or one after the other when their number is no power of two (then LPH divides
+// the 32 / LPH * LPH lanes that are used of a warp).  Streams g and out once (1 M rows x 64 floats: 258 us with a warp per
+// row, which left half of the lanes without a slice).
 __global__ void __launch_bounds__(256)
 gat_rowpack_kernel(int64_t n_rows, int H, int F, const float *q, const float *row_max, const float *row_sum,
                    const float *g, int g_shared, float g_scale, const float *out_heads, float4 *rowpack) {
-    const int64_t row = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    if (row >= n_rows) return;
-    const int lane = threadIdx.x & 31;
-    const int64_t D = static_cast<int64_t>(H) * F;
-    const int LPH = F >> 2;
-    float d[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int64_t off = static_cast<int64_t>(i * 32 + lane) * 4;
-        d[i] = 0.0f;
-        if (off < D) {
-            const int64_t goff = g_shared ? off % F : off;
-            const float4 gv = __ldg(reinterpret_cast<const float4 *>(g + row * (g_shared ? F : D) + goff));
-            const float4 ov = __ldg(reinterpret_cast<const float4 *>(out_heads + row * D + off));
-            d[i] = gv.x * ov.x + gv.y * ov.y + gv.z * ov.z + gv.w * ov.w;
-        }
+    const int lane = threadIdx.x & 31, LPH = F >> 2;
+    const int per_warp = 32 / LPH;  // heads per warp
+    const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int64_t rh = warp * per_warp + lane / LPH;  // row * H + head
+    const int k = lane % LPH;
+    const bool valid = lane < per_warp * LPH && rh < n_rows * H;
+    float d = 0.0f;
+    if (valid) {
+        const float4 gv = __ldg(reinterpret_cast<const float4 *>(g + (g_shared ? rh / H : rh) * F) + k);
+        const float4 ov = __ldg(reinterpret_cast<const float4 *>(out_heads + rh * F) + k);
+        d = gv.x * ov.x + gv.y * ov.y + gv.z * ov.z + gv.w * ov.w;
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int64_t off = static_cast<int64_t>(i * 32 + lane) * 4;
-        for (int o = LPH >> 1; o > 0; o >>= 1) d[i] += __shfl_xor_sync(0xffffffffu, d[i], o);
-        if (off < D && (lane & (LPH - 1)) == 0) {
-            const int64_t h = off / F;
-            // p = exp(score - M) / L = exp(score - (M + log L)); rows without edges are never looked up
-            const float l = __ldg(row_sum + row * H + h);
-            rowpack[row * H + h] = make_float4(__ldg(q + row * H + h), __ldg(row_max + row * H + h) + logf(fmaxf(l, 1e-38f)),
-                                               d[i] * g_scale, 0.0f);
-        }
+    if ((LPH & (LPH - 1)) == 0) {
+        for (int o = LPH >> 1; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+    } else {
+        const float mine = d;
+        for (int o = 1; o < LPH; ++o) d += __shfl_sync(0xffffffffu, mine, (lane + o) & 31);  // right in each head's first lane
+    }
+    if (valid && k == 0) {
+        // p = exp(score - M) / L = exp(score - (M + log L)); rows without edges are never looked up
+        const float l = __ldg(row_sum + rh);
+        rowpack[rh] = make_float4(__ldg(q + rh), __ldg(row_max + rh) + logf(fmaxf(l, 1e-38f)), d * g_scale, 0.0f);
     }
 }
 
-// Edges are taken in tiles of SRC_TILE.  Shared memory per warp: SRC_TILE destination ids and CSR positions, H keys of
-// the source, and per (edge, head) of the tile the attention p, p * LeakyReLU' and the destination's D.  (Tiles of 64,
-// which spare rows of 33..64 edges a second chain of dependent loads, were measured slower on the 8x32 layer, 10.5 ms
-// against 8.95 ms: the doubled shared memory costs more than the shorter chain gains.)
-constexpr int SRC_TILE = 32;
-__host__ __device__ __forceinline__ int src_smem_floats(int H) { return 2 * SRC_TILE + 32 + 3 * SRC_TILE * H; }
-
+// Lanes and groups as in the forward: a slice of a lane lies inside one head, so the lane that holds x[c], k[c] and g[r] for
+// its head also reads that head's record of the destination and forms p and ds itself, after a butterfly of log2(F / VEC)
+// steps for dp.  The record, weight and gradient gathers of EU edges are in flight together.
 // GIVEN = true is the backward of a multi-head SpMM with stored edge values (graph_ext.spmm_backward): the weights are
 // read instead of rebuilt, and the by-product is d value = <g[r], x[c]> per edge and head.
-template <int NV, int VEC, int EU, bool GIVEN>
-__device__ __forceinline__ void gat_bwd_src_body(const GatSrcParams &p) {
-    extern __shared__ float smem[];
-    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t gid = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+template <int RW, int LPE, int NV, int VEC, int EU, bool GIVEN, int LPH_T, int MINB = 1>
+__global__ void __launch_bounds__(128, MINB) gat_bwd_src_kernel(const __grid_constant__ GatSrcParams p) {
+    constexpr int EPI = RW / LPE, STEP = EPI * EU;
+    static_assert(RW % STEP == 0, "a tile of RW ids is consumed in whole steps");
+    const int lane = threadIdx.x & 31, gl = lane & (RW - 1), sub = gl / LPE, l_in = gl & (LPE - 1);
+    constexpr unsigned FULL_WARP = 0xffffffffu;
+    const int64_t gid = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / RW;
     int64_t c, eb, ee;
     const bool chunk = gid < p.n_chunks;
+    bool store = true;
     if (chunk) {
         c = __ldg(p.chunk_row + gid);
         eb = __ldg(p.chunk_begin + gid);
         ee = min(eb + static_cast<int64_t>(p.chunk_edges), load_ptr(p.t_indptr, p.is64, c + 1));
     } else {
-        c = gid - p.n_chunks;
-        if (c >= p.n_cols) return;
+        store = gid - p.n_chunks < p.n_cols;
+        c = store ? gid - p.n_chunks : 0;
         eb = load_ptr(p.t_indptr, p.is64, c);
         ee = load_ptr(p.t_indptr, p.is64, c + 1);
-        if (p.n_chunks > 0 && ee - eb > p.chunk_edges) return;
+        store = store && !(p.n_chunks > 0 && ee - eb > p.chunk_edges);
+        if (!store) {
+            if (RW == 32) return;
+            ee = eb;
+        }
     }
-    const int H = p.H, F = p.F;
-    const int D = H * F;
-    const int LPH = F / VEC;  // lanes per head: a power of two <= 32
-    const bool leader = (lane & (LPH - 1)) == 0;
-    const int64_t gstride = p.g_shared ? F : D;
-    float *base = smem + wib * src_smem_floats(H);
-    int *s_r = reinterpret_cast<int *>(base), *s_pos = s_r + SRC_TILE;
-    float *s_k = base + 2 * SRC_TILE, *s_p = s_k + 32, *s_pf = s_p + SRC_TILE * H, *s_d = s_pf + SRC_TILE * H;
-    if (!GIVEN && lane < H) s_k[lane] = __ldg(p.k + c * H + lane);
-    int hd[NV], off[NV], goff[NV];  // offsets inside a row: H*F <= 512
-    bool valid[NV];
-    float xr[NV][VEC], acc[NV][VEC];
-    float gk_lane = 0.0f;  // partial sum of the score gradients of head lane % H (lane h of head h when H is not 2^k)
+    const int H = p.H, F = p.F, D = H * F;
+    const int LPH = LPH_T ? LPH_T : F / VEC;  // lanes per head, at most 32; any number only with one slice per lane
+    const bool pow2 = (LPH & (LPH - 1)) == 0;
+    const int head_lane = sub * LPE + l_in / LPH * LPH;  // read only in the other case
+    const uint32_t g_bytes = static_cast<uint32_t>(p.g_shared ? F : D) * 4u, rec_bytes = static_cast<uint32_t>(H) * 16u,
+                   edge_bytes = static_cast<uint32_t>(H) * 4u;
+    int hd[NV], off[NV];
+    bool valid[NV], first[NV];  // lanes behind the row's end repeat its first slice and store nothing; first lane of a head
+    const float *gp[NV];
+    const float4 *rp[NV];
+    float xr[NV][VEC], acc[NV][VEC], kk[NV], gk[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-        off[i] = (i * 32 + lane) * VEC;
+        off[i] = (i * LPE + l_in) * VEC;
         valid[i] = off[i] < D;
-        hd[i] = valid[i] ? off[i] / F : 0;
-        goff[i] = p.g_shared ? off[i] - hd[i] * F : off[i];
-        if (valid[i]) {
-            load_vec<VEC>(xr[i], p.x + c * D + off[i]);
+        if (!valid[i]) off[i] = 0;
+        hd[i] = off[i] / F;
+        first[i] = valid[i] && off[i] == hd[i] * F;
+        gp[i] = p.g + (p.g_shared ? off[i] - hd[i] * F : off[i]);
+        rp[i] = p.rowpack + hd[i];
+        kk[i] = GIVEN ? 0.0f : __ldg(p.k + c * H + hd[i]);
+        gk[i] = 0.0f;
+        load_vec<VEC>(xr[i], p.x + c * D + off[i]);
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) {
+            xr[i][v] *= p.g_scale;
+            acc[i][v] = 0.0f;
+        }
+    }
+    int my_r = 0, my_pos = 0;
+    if (eb + gl < ee) {
+        my_r = ld_stream(p.t_rows + eb + gl);
+        my_pos = ld_stream(p.t_perm + eb + gl);
+    }
+    // EU edges of this lane's sub-group, starting at position j of the tile; FULL: all STEP positions carry an edge
+    auto step = [&](int j, int n, auto full) {
+        constexpr bool FULL = decltype(full)::value;
+        float gv[EU][NV][VEC], w[EU][NV];
+        float4 rec[EU][NV];
+        int pos[EU];
+#pragma unroll
+        for (int u = 0; u < EU; ++u) {
+            const int at = j + u * EPI + sub;
+            const int r = __shfl_sync(FULL_WARP, my_r, at, RW);
+            pos[u] = __shfl_sync(FULL_WARP, my_pos, at, RW);
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                if (FULL || at < n) {
+                    if constexpr (GIVEN) w[u][i] = load_now(row_at(p.values + hd[i], pos[u], edge_bytes));
+                    else rec[u][i] = load_now(row_at(rp[i], r, rec_bytes));
+                    load_vec<VEC>(gv[u][i], row_at(gp[i], r, g_bytes));
+                } else {
+                    w[u][i] = 0.0f;
+                    rec[u][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int v = 0; v < VEC; ++v) gv[u][i][v] = 0.0f;
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < EU; ++u) {
+            const bool live = FULL || j + u * EPI + sub < n;
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                float dp = 0.0f;
+#pragma unroll
+                for (int v = 0; v < VEC; ++v) dp = fmaf(gv[u][i][v], xr[i][v], dp);
+                if (LPH_T || pow2) {
+#pragma unroll
+                    for (int o = LPE >> 1; o > 0; o >>= 1)
+                        if (o < LPH) dp += __shfl_xor_sync(FULL_WARP, dp, o, RW);
+                } else {  // every lane adds the head's lanes in the same order
+                    const float mine = dp;
+                    dp = 0.0f;
+                    for (int o = 0; o < LPH; ++o) dp += __shfl_sync(FULL_WARP, mine, head_lane + o, RW);
+                }
+                float out = dp, pr = 0.0f;
+                if constexpr (GIVEN) {
+                    pr = w[u][i];
+                } else {
+                    const float sc = rec[u][i].x + kk[i];
+                    pr = expf(leaky_relu(sc, p.slope) - rec[u][i].y);
+                    if (!live) pr = 0.0f;
+                    out = (sc < 0.0f ? pr * p.slope : pr) * (dp - rec[u][i].z);
+                    gk[i] += out;
+                }
+#pragma unroll
+                for (int v = 0; v < VEC; ++v) acc[i][v] = fmaf(pr, gv[u][i][v], acc[i][v]);
+                // the head's first lane writes the score gradient (or d value) to the edge's CSR position
+                if (live && first[i])
+                    *const_cast<float *>(row_at((GIVEN ? p.grad_values : p.edge_grad) + hd[i], pos[u], edge_bytes)) = out;
+            }
+        }
+    };
+    for (int64_t e0 = eb; RW == 32 ? e0 < ee : __any_sync(FULL_WARP, e0 < ee); e0 += RW) {  // as in the forward
+        const int n = static_cast<int>(max(static_cast<int64_t>(0), min(static_cast<int64_t>(RW), ee - e0)));
+        int nx_r = 0, nx_pos = 0;
+        if (e0 + RW + gl < ee) {
+            nx_r = ld_stream(p.t_rows + e0 + RW + gl);
+            nx_pos = ld_stream(p.t_perm + e0 + RW + gl);
+        }
+        int j = 0;
+        if constexpr (RW == 32) {
+            for (; j + STEP <= n; j += STEP) step(j, n, std::true_type{});
+            if (j < n) step(j, n, std::false_type{});
         } else {
-#pragma unroll
-            for (int v = 0; v < VEC; ++v) xr[i][v] = 0.0f;
+            const int most = __reduce_max_sync(FULL_WARP, n);
+            for (; j < most; j += STEP) step(j, n, std::false_type{});
         }
-#pragma unroll
-        for (int v = 0; v < VEC; ++v) acc[i][v] = 0.0f;
+        my_r = nx_r;
+        my_pos = nx_pos;
     }
-    for (int64_t e0 = eb; e0 < ee; e0 += SRC_TILE) {
-        const int n = static_cast<int>(min(static_cast<int64_t>(SRC_TILE), ee - e0));
-        int my_r[SRC_TILE / 32], my_pos[SRC_TILE / 32];
 #pragma unroll
-        for (int t = 0; t < SRC_TILE / 32; ++t) {
-            my_r[t] = my_pos[t] = 0;
-            if (t * 32 + lane < n) {
-                my_r[t] = ld_stream(p.t_rows + e0 + t * 32 + lane);
-                my_pos[t] = ld_stream(p.t_perm + e0 + t * 32 + lane);
-            }
+    for (int o = LPE; o < RW; o <<= 1)
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            gk[i] += __shfl_xor_sync(FULL_WARP, gk[i], o, RW);
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) acc[i][v] += __shfl_xor_sync(FULL_WARP, acc[i][v], o, RW);
         }
-        const int r_first = __shfl_sync(0xffffffffu, my_r[0], 0);
-#pragma unroll
-        for (int t = 0; t < SRC_TILE / 32; ++t) {
-            s_r[t * 32 + lane] = t * 32 + lane < n ? my_r[t] : r_first;  // padding edges repeat the first one, attention 0
-            s_pos[t * 32 + lane] = my_pos[t];
-        }
-        __syncwarp();
-        // attention and its factors for the tile's (edge, head) pairs: one 16-byte record of the destination each
-        const int n_up = (n + EU - 1) & ~(EU - 1);
-        for (int idx = lane; idx < n_up * H; idx += 32) {
-            const int e = p.hshift >= 0 ? (idx >> p.hshift) : (idx / H);
-            const int h = idx - e * H;
-            float pr = 0.0f, pf = 0.0f, dv = 0.0f;
-            if constexpr (GIVEN) {
-                if (e < n) pr = __ldg(p.values + static_cast<int64_t>(s_pos[e]) * H + h);
-            } else if (e < n) {
-                const float4 rp = __ldg(p.rowpack + static_cast<int64_t>(s_r[e]) * H + h);
-                const float sc = rp.x + s_k[h];
-                pr = expf(leaky_relu(sc, p.slope) - rp.y);
-                pf = sc < 0.0f ? pr * p.slope : pr;
-                dv = rp.z;
-            }
-            s_p[idx] = pr;
-            if constexpr (!GIVEN) {
-                s_pf[idx] = pf;
-                s_d[idx] = dv;
-            }
-        }
-        __syncwarp();
-        for (int j = 0; j < n_up; j += EU) {
-            float gv[EU][NV][VEC];
-#pragma unroll
-            for (int u = 0; u < EU; ++u) {
-                const float *gr = p.g + static_cast<int64_t>(s_r[j + u]) * gstride;
-#pragma unroll
-                for (int i = 0; i < NV; ++i) {
-                    if (valid[i]) {
-                        load_vec<VEC>(gv[u][i], gr + goff[i]);
-                    } else {
-#pragma unroll
-                        for (int v = 0; v < VEC; ++v) gv[u][i][v] = 0.0f;
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < EU; ++u) {
-#pragma unroll
-                for (int i = 0; i < NV; ++i) {
-                    float dp = 0.0f;
-#pragma unroll
-                    for (int v = 0; v < VEC; ++v) dp = fmaf(gv[u][i][v], xr[i][v], dp);
-                    for (int o = LPH >> 1; o > 0; o >>= 1) dp += __shfl_xor_sync(0xffffffffu, dp, o);
-                    const int slot = (j + u) * H + hd[i];
-                    const float w = valid[i] ? s_p[slot] * p.g_scale : 0.0f;
-#pragma unroll
-                    for (int v = 0; v < VEC; ++v) acc[i][v] = fmaf(w, gv[u][i][v], acc[i][v]);
-                    // the head's leader lane leaves dp (minus the destination's D) for the pass over the pairs below
-                    if (leader && valid[i]) s_d[slot] = dp * p.g_scale - (GIVEN ? 0.0f : s_d[slot]);
-                }
-            }
-        }
-        __syncwarp();
-        // score gradients (or d value) of the tile, spread over (edge, head) pairs: scattered to the edges' CSR positions
-        for (int idx = lane; idx < n * H; idx += 32) {
-            const int e = p.hshift >= 0 ? (idx >> p.hshift) : (idx / H);
-            const int h = idx - e * H;
-            if constexpr (GIVEN) {
-                p.grad_values[static_cast<int64_t>(s_pos[e]) * H + h] = s_d[idx];
-            } else {
-                const float ds = s_pf[idx] * s_d[idx];
-                p.edge_grad[static_cast<int64_t>(s_pos[e]) * H + h] = ds;
-                if (p.hshift >= 0) gk_lane += ds;  // H a power of two: this lane always meets head lane % H
-                else s_pf[idx] = ds;
-            }
-        }
-        if (!GIVEN && p.hshift < 0) {
-            __syncwarp();
-            if (lane < H)
-                for (int e = 0; e < n; ++e) gk_lane += s_pf[e * H + lane];
-        }
-        __syncwarp();
-    }
+    if (sub != 0 || !store) return;
     float *xdst = chunk ? p.x_partial + gid * D : p.grad_x + c * D;
     float *kdst = chunk ? p.k_partial + gid * H : p.grad_k + c * H;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         if (!valid[i]) continue;
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) acc[i][v] *= p.g_scale;
         store_vec<VEC>(xdst + off[i], acc[i]);
-    }
-    if constexpr (!GIVEN) {
-        if (p.hshift >= 0)
-            for (int o = H; o < 32; o <<= 1) gk_lane += __shfl_xor_sync(0xffffffffu, gk_lane, o);
-        if (lane < H) kdst[lane] = gk_lane;
+        if (!GIVEN && first[i]) kdst[hd[i]] = gk[i];
     }
 }
 
-template <int NV, int VEC, int EU, bool GIVEN>
-__global__ void __launch_bounds__(256) gat_bwd_src_kernel(const __grid_constant__ GatSrcParams p) {
-    gat_bwd_src_body<NV, VEC, EU, GIVEN>(p);
+// out[row, :W] = sum of the row's chunk partials
+template <int VEC>
+__global__ void __launch_bounds__(256) chunk_sum_kernel(const __grid_constant__ HubRows h, int W, const float *partial, float *out) {
+    reduce_hub_rows<VEC>(h, partial, W, W, [&](int64_t row, int64_t d, float (&a)[VEC]) { store_vec<VEC>(out + row * W + d, a); });
 }
 
-// the same body held to 64 registers, four CTAs per SM: 8.95 ms against 9.58 ms at 80 registers for the backward of the
-// 8x32 layer (the few spilled values cost less than the lost warps)
-template <int NV, int VEC, int EU, bool GIVEN>
-__global__ void __launch_bounds__(256, 4) gat_bwd_src_kernel_r64(const __grid_constant__ GatSrcParams p) {
-    gat_bwd_src_body<NV, VEC, EU, GIVEN>(p);
-}
-
-// out[row, :W] = sum of the row's chunk partials, in chunk order (one CTA per chunk, the row's first chunk works)
-__global__ void __launch_bounds__(128)
-chunk_sum_kernel(const void *indptr, int is64, int chunk_edges, const int *chunk_row, const int64_t *chunk_begin, int W,
-                 const float *partial, float *out) {
-    const int64_t c0 = blockIdx.x;
-    const int64_t row = __ldg(chunk_row + c0);
-    const int64_t rb = load_ptr(indptr, is64, row);
-    if (__ldg(chunk_begin + c0) != rb) return;
-    const int64_t nch = (load_ptr(indptr, is64, row + 1) - rb + chunk_edges - 1) / chunk_edges;
-    for (int d = threadIdx.x; d < W; d += blockDim.x) {
-        float a = 0.0f;
-        for (int64_t c = 0; c < nch; ++c) a += partial[(c0 + c) * W + d];
-        out[row * W + d] = a;
-    }
+static int launch_chunk_sum(const HubRows &h, int64_t W, const float *partial, float *out, cudaStream_t st) {
+    if (h.n_chunks == 0) return YITU_OK;
+    const unsigned grid = static_cast<unsigned>((h.n_chunks + 7) / 8);
+    if (W % 4 == 0 && aligned16(partial) && aligned16(out)) chunk_sum_kernel<4><<<grid, 256, 0, st>>>(h, static_cast<int>(W), partial, out);
+    else chunk_sum_kernel<1><<<grid, 256, 0, st>>>(h, static_cast<int>(W), partial, out);
+    YITU_LAUNCH_CHECK();
+    return YITU_OK;
 }
 
 static int head_block(int64_t H) {
@@ -1101,7 +1226,7 @@ extern "C" int yitu_edge_softmax_fwd_f32(const yitu_csr_t *g, int32_t n_segments
     edge_softmax_fwd_kernel<false><<<static_cast<unsigned>((g->n_rows + 7) / 8), 256, 0, st>>>(p);
     YITU_LAUNCH_CHECK();
     if (p.n_chunks > 0) {  // hub rows: one CTA each
-        edge_softmax_fwd_kernel<true><<<static_cast<unsigned>(p.n_chunks), 256, 0, st>>>(p);
+        edge_softmax_fwd_kernel<true><<<static_cast<unsigned>(p.n_chunks), HUB_THREADS, 0, st>>>(p);
         YITU_LAUNCH_CHECK();
     }
     return YITU_OK;
@@ -1125,9 +1250,34 @@ extern "C" int yitu_edge_softmax_bwd_f32(const yitu_csr_t *g, int32_t n_segments
     edge_softmax_bwd_kernel<false><<<static_cast<unsigned>((g->n_rows + 7) / 8), 256, 0, st>>>(p);
     YITU_LAUNCH_CHECK();
     if (p.n_chunks > 0) {
-        edge_softmax_bwd_kernel<true><<<static_cast<unsigned>(p.n_chunks), 256, 0, st>>>(p);
+        edge_softmax_bwd_kernel<true><<<static_cast<unsigned>(p.n_chunks), HUB_THREADS, 0, st>>>(p);
         YITU_LAUNCH_CHECK();
     }
+    return YITU_OK;
+}
+
+// partial: scratch of n_chunks * H floats for the hub columns' chunk sums, or NULL (a CTA per hub column)
+static int gather_sum(int64_t n_cols, const void *t_indptr, int32_t indptr_is64, const int32_t *t_perm, int64_t n_heads,
+                      const float *edge_vals, float *out, const yitu_hub_plan_t *t_plan, float *partial, cudaStream_t st) {
+    if (n_cols == 0) return YITU_OK;
+    GatherSumParams p{};
+    p.n_cols = n_cols; p.t_indptr = t_indptr; p.is64 = indptr_is64; p.perm = t_perm;
+    p.H = static_cast<int>(n_heads); p.HB = head_block(n_heads); p.vals = edge_vals; p.out = out;
+    if (int rc = fill_plan(t_plan, &p.n_chunks, &p.chunk_edges, &p.chunk_row, &p.chunk_begin)) return rc;
+    const int64_t n_parts = partial ? p.n_chunks : 0;
+    const int rw = p.HB < 8 ? 8 : p.HB;
+    const unsigned grid = static_cast<unsigned>((n_cols + n_parts + 128 / rw - 1) / (128 / rw));
+    if (rw == 8) edge_gather_sum_kernel<8><<<grid, 128, 0, st>>>(p, n_parts, partial);
+    else if (rw == 16) edge_gather_sum_kernel<16><<<grid, 128, 0, st>>>(p, n_parts, partial);
+    else edge_gather_sum_kernel<32><<<grid, 128, 0, st>>>(p, n_parts, partial);
+    YITU_LAUNCH_CHECK();
+    if (p.n_chunks == 0) return YITU_OK;
+    if (partial) {
+        const HubRows h{t_indptr, indptr_is64, p.chunk_edges, p.n_chunks, p.chunk_row, p.chunk_begin};
+        return launch_chunk_sum(h, n_heads, partial, out, st);
+    }
+    edge_gather_sum_hub_kernel<<<static_cast<unsigned>(p.n_chunks), 256, 0, st>>>(p);
+    YITU_LAUNCH_CHECK();
     return YITU_OK;
 }
 
@@ -1137,18 +1287,8 @@ extern "C" int yitu_edge_gather_sum_f32(int64_t n_cols, const void *t_indptr, in
     YITU_REQUIRE(n_cols >= 0 && n_heads >= 1 && t_indptr, YITU_ERR_INVALID_ARG, "bad argument");
     if (n_cols == 0) return YITU_OK;
     YITU_REQUIRE(out, YITU_ERR_INVALID_ARG, "out is NULL");
-    GatherSumParams p{};
-    p.n_cols = n_cols; p.t_indptr = t_indptr; p.is64 = indptr_is64; p.perm = t_perm;
-    p.H = static_cast<int>(n_heads); p.HB = head_block(n_heads); p.vals = edge_vals; p.out = out;
-    if (int rc = fill_plan(t_plan, &p.n_chunks, &p.chunk_edges, &p.chunk_row, &p.chunk_begin)) return rc;
-    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    edge_gather_sum_kernel<false><<<static_cast<unsigned>((n_cols + 7) / 8), 256, 0, st>>>(p);
-    YITU_LAUNCH_CHECK();
-    if (p.n_chunks > 0) {
-        edge_gather_sum_kernel<true><<<static_cast<unsigned>(p.n_chunks), 256, 0, st>>>(p);
-        YITU_LAUNCH_CHECK();
-    }
-    return YITU_OK;
+    return gather_sum(n_cols, t_indptr, indptr_is64, t_perm, n_heads, edge_vals, out, t_plan, nullptr,
+                      reinterpret_cast<cudaStream_t>(stream));
 }
 
 // grad_shared: grad_out is [n_rows,F] and stands for every head (scaled by grad_scale) — the gradient of a mean
@@ -1221,22 +1361,19 @@ static int check_gat(const yitu_gat_args_t *a, bool backward) {
 static void fill_gat(GatParams &p, const yitu_gat_args_t *a) {
     p.n_rows = a->graph.n_rows; p.indptr = a->graph.indptr; p.indices = a->graph.indices;
     p.is64 = a->graph.indptr_is64; p.H = static_cast<int>(a->n_heads); p.F = static_cast<int>(a->n_feats);
-    p.hshift = (p.H & (p.H - 1)) == 0 ? 31 - __builtin_clz(p.H) : -1;
     p.slope = a->slope; p.q = a->query; p.k = a->key; p.x = a->x;
     p.out = a->out; p.row_max = a->row_max; p.row_sum = a->row_sum;
     p.head_mean = a->head_mean ? 1 : 0; p.act = a->activation;
-    p.stage = p.head_mean ? p.H * p.F : 0;
     p.out_heads = p.head_mean ? a->out_heads : nullptr;
 }
 
-template <typename K>
-static int launch_rows(K kernel, const GatParams &p, int smem_floats_per_warp, cudaStream_t st) {
-    const int warps = 8;
-    const size_t smem = static_cast<size_t>(warps) * smem_floats_per_warp * sizeof(float);
-    if (smem > 48 * 1024)
-        YITU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+template <int RW, int LPE, int NV, int VEC, int EU, int MINB = 1>
+static int launch_gat_fwd(const GatParams &p, cudaStream_t st) {
+    const int groups_per_cta = 128 / RW;
+    const size_t smem = p.head_mean ? static_cast<size_t>(groups_per_cta) * p.H * p.F * sizeof(float) : 0;
     const int64_t groups = p.n_rows + p.n_chunks;
-    kernel<<<static_cast<unsigned>((groups + warps - 1) / warps), warps * 32, smem, st>>>(p);
+    const unsigned grid = static_cast<unsigned>((groups + groups_per_cta - 1) / groups_per_cta);
+    gat_fwd_kernel<RW, LPE, NV, VEC, EU, MINB><<<grid, 128, smem, st>>>(p);
     YITU_LAUNCH_CHECK();
     return YITU_OK;
 }
@@ -1270,48 +1407,74 @@ extern "C" int yitu_gat_fwd_f32(const yitu_gat_args_t *a, yitu_stream_t stream) 
         p.partial = a->scratch;
     }
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const int sm = warp_smem_floats_fwd(p.H, p.stage);
-    const auto pick = [&](auto mean, auto plan) -> int {
-        constexpr bool M = decltype(mean)::value, P = decltype(plan)::value;
-        if (D <= 128) return launch_rows(gat_fwd_kernel<1, M, P>, p, sm, st);
-        if (D <= 256) return launch_rows(gat_fwd_kernel_r64<2, M, P>, p, sm, st);
-        return launch_rows(gat_fwd_kernel<4, M, P>, p, sm, st);
-    };
-    using T = std::true_type;
-    using Fl = std::false_type;
-    const int rc = p.head_mean ? (p.n_chunks > 0 ? pick(T{}, T{}) : pick(T{}, Fl{}))
-                               : (p.n_chunks > 0 ? pick(Fl{}, T{}) : pick(Fl{}, Fl{}));
+    // 256-bit gathers when a head spans whole 32-byte slices and every row starts on a 32-byte boundary
+    const auto a32 = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 31) == 0; };
+    const bool wide = p.F % 8 == 0 && a32(a->x) && a32(a->out) && a32(p.out_heads) && a32(p.partial);
+    int rc;
+    if (wide) {
+        if (D <= 8) rc = launch_gat_fwd<8, 1, 1, 8, 1>(p, st);
+        else if (D <= 16) rc = launch_gat_fwd<8, 2, 1, 8, 2>(p, st);
+        else if (D <= 32) rc = launch_gat_fwd<8, 4, 1, 8, 4>(p, st);
+        else if (D <= 64) rc = launch_gat_fwd<8, 8, 1, 8, 4, 6>(p, st);
+        else if (D <= 128) rc = launch_gat_fwd<16, 16, 1, 8, 4, 6>(p, st);
+        else if (D <= 256) rc = launch_gat_fwd<32, 32, 1, 8, 4>(p, st);
+        else rc = launch_gat_fwd<32, 32, 2, 8, 2>(p, st);
+    } else {
+        if (D <= 16) rc = launch_gat_fwd<8, 4, 1, 4, 4>(p, st);
+        else if (D <= 32) rc = launch_gat_fwd<8, 8, 1, 4, 4>(p, st);
+        else if (D <= 64) rc = launch_gat_fwd<16, 16, 1, 4, 8>(p, st);
+        else if (D <= 128) rc = launch_gat_fwd<32, 32, 1, 4, 8>(p, st);
+        else if (D <= 256) rc = launch_gat_fwd<32, 32, 2, 4, 4>(p, st);
+        else rc = launch_gat_fwd<32, 32, 4, 4, 2>(p, st);
+    }
     if (rc) return rc;
     if (p.n_chunks > 0) {
-        gat_fwd_merge_kernel<<<static_cast<unsigned>(p.n_chunks), 128, 0, st>>>(p);
+        gat_fwd_merge_kernel<<<static_cast<unsigned>(p.n_chunks), 256, 0, st>>>(p);
         YITU_LAUNCH_CHECK();
     }
     return YITU_OK;
 }
 
 // Launches the source-side pass (attention rebuilt, or GIVEN edge values); the caller merges hub chunks afterwards.
+template <int RW, int LPE, int NV, int VEC, int EU, bool GIVEN, int MINB = 1>
+static int launch_src_as(const GatSrcParams &p, cudaStream_t st) {
+    const int groups_per_cta = 128 / RW;
+    const unsigned grid = static_cast<unsigned>((p.n_cols + p.n_chunks + groups_per_cta - 1) / groups_per_cta);
+    // the butterfly over the lanes of a head is unrolled for the wide loads; the others (heads of four floats, misaligned
+    // tensors) branch over its steps
+    switch (VEC == 8 ? p.F / VEC : 0) {
+        case 1: gat_bwd_src_kernel<RW, LPE, NV, VEC, EU, GIVEN, 1, MINB><<<grid, 128, 0, st>>>(p); break;
+        case 2: if constexpr (VEC == 8 && LPE >= 2) gat_bwd_src_kernel<RW, LPE, NV, VEC, EU, GIVEN, 2, MINB><<<grid, 128, 0, st>>>(p); break;
+        case 4: if constexpr (VEC == 8 && LPE >= 4) gat_bwd_src_kernel<RW, LPE, NV, VEC, EU, GIVEN, 4, MINB><<<grid, 128, 0, st>>>(p); break;
+        case 8: if constexpr (VEC == 8 && LPE >= 8) gat_bwd_src_kernel<RW, LPE, NV, VEC, EU, GIVEN, 8, MINB><<<grid, 128, 0, st>>>(p); break;
+        case 16: if constexpr (VEC == 8 && LPE >= 16) gat_bwd_src_kernel<RW, LPE, NV, VEC, EU, GIVEN, 16, MINB><<<grid, 128, 0, st>>>(p); break;
+        case 32: if constexpr (VEC == 8 && LPE >= 32) gat_bwd_src_kernel<RW, LPE, NV, VEC, EU, GIVEN, 32, MINB><<<grid, 128, 0, st>>>(p); break;
+        default: gat_bwd_src_kernel<RW, LPE, NV, VEC, EU, GIVEN, 0, MINB><<<grid, 128, 0, st>>>(p); break;
+    }
+    YITU_LAUNCH_CHECK();
+    return YITU_OK;
+}
+
 template <bool GIVEN>
-static int launch_src(GatSrcParams &sp, int64_t t_chunks, const float *x, const float *grad_out, float *grad_x,
-                      float *x_partial, cudaStream_t st) {
-    const int D = sp.H * sp.F;
-    sp.hshift = (sp.H & (sp.H - 1)) == 0 ? 31 - __builtin_clz(sp.H) : -1;
-    const unsigned blocks = static_cast<unsigned>((sp.n_cols + t_chunks + 7) / 8);
-    const size_t smem = 8 * static_cast<size_t>(src_smem_floats(sp.H)) * sizeof(float);
-    auto run = [&](auto kernel) -> int {
-        if (smem > 48 * 1024)
-            YITU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-        kernel<<<blocks, 256, smem, st>>>(sp);
-        YITU_LAUNCH_CHECK();
-        return YITU_OK;
-    };
+static int launch_src(const GatSrcParams &p, cudaStream_t st) {
+    const int D = p.H * p.F;
     // 256-bit gathers when a head spans whole 32-byte slices and every row starts on a 32-byte boundary
     const auto a32 = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 31) == 0; };
-    const bool wide = sp.F % 8 == 0 && a32(x) && a32(grad_out) && a32(grad_x) && a32(x_partial);
-    if (wide && D > 128)
-        return D <= 256 ? run(gat_bwd_src_kernel_r64<1, 8, 4, GIVEN>) : run(gat_bwd_src_kernel<2, 8, 2, GIVEN>);
-    if (D <= 128) return run(gat_bwd_src_kernel<1, 4, 4, GIVEN>);
-    if (D <= 256) return run(gat_bwd_src_kernel<2, 4, 4, GIVEN>);
-    return run(gat_bwd_src_kernel<4, 4, 2, GIVEN>);
+    if (p.F % 8 == 0 && a32(p.x) && a32(p.g) && a32(p.grad_x) && a32(p.x_partial)) {
+        if (D <= 8) return launch_src_as<8, 1, 1, 8, 1, GIVEN>(p, st);
+        if (D <= 16) return launch_src_as<8, 2, 1, 8, 2, GIVEN>(p, st);
+        if (D <= 32) return launch_src_as<8, 4, 1, 8, 4, GIVEN>(p, st);
+        if (D <= 64) return launch_src_as<8, 8, 1, 8, 2, GIVEN, 6>(p, st);
+        if (D <= 128) return launch_src_as<16, 16, 1, 8, 4, GIVEN, 4>(p, st);
+        if (D <= 256) return launch_src_as<32, 32, 1, 8, 4, GIVEN, 4>(p, st);
+        return launch_src_as<32, 32, 2, 8, 2, GIVEN>(p, st);
+    }
+    if (D <= 16) return launch_src_as<8, 4, 1, 4, 4, GIVEN>(p, st);
+    if (D <= 32) return launch_src_as<8, 8, 1, 4, 4, GIVEN>(p, st);
+    if (D <= 64) return launch_src_as<16, 16, 1, 4, 4, GIVEN>(p, st);
+    if (D <= 128) return launch_src_as<32, 32, 1, 4, 4, GIVEN>(p, st);
+    if (D <= 256) return launch_src_as<32, 32, 2, 4, 4, GIVEN>(p, st);
+    return launch_src_as<32, 32, 4, 4, 2, GIVEN>(p, st);
 }
 
 extern "C" int yitu_gat_bwd_f32(const yitu_gat_bwd_args_t *b, yitu_stream_t stream) {
@@ -1349,13 +1512,15 @@ extern "C" int yitu_gat_bwd_f32(const yitu_gat_bwd_args_t *b, yitu_stream_t stre
     float *k_partial = q_partial + up256f(p.n_chunks * H);
     float *x_partial = k_partial + up256f(t_chunks * H);
     const int64_t lph = F / 4;
-    const bool one_pass = lph <= 32 && (lph & (lph - 1)) == 0 && aligned16(a->x) && aligned16(out_heads);
+    // lanes per head: a power of two, or any number when a row is one slice per lane
+    const bool one_pass = lph <= 32 && ((lph & (lph - 1)) == 0 || D <= 128) && aligned16(a->x) && aligned16(out_heads);
 
     if (one_pass) {
         // (1) per-destination constants, (2) everything else in one pass over the transposed graph, (3) grad_query as
         // the row sum of the scattered score gradients
         if (g.n_rows > 0) {
-            gat_rowpack_kernel<<<static_cast<unsigned>((g.n_rows + 7) / 8), 256, 0, st>>>(
+            const int64_t heads_per_cta = 8 * (32 / lph);
+            gat_rowpack_kernel<<<static_cast<unsigned>((g.n_rows * H + heads_per_cta - 1) / heads_per_cta), 256, 0, st>>>(
                 g.n_rows, static_cast<int>(H), static_cast<int>(F), a->query, a->row_max, a->row_sum, b->grad_out, shared,
                 gscale, out_heads, reinterpret_cast<float4 *>(rowpack));
             YITU_LAUNCH_CHECK();
@@ -1369,21 +1534,13 @@ extern "C" int yitu_gat_bwd_f32(const yitu_gat_bwd_args_t *b, yitu_stream_t stre
             sp.grad_x = b->grad_x; sp.grad_k = b->grad_key; sp.edge_grad = b->edge_grad;
             sp.n_chunks = t_chunks; sp.chunk_edges = t_chunk_edges; sp.chunk_row = t_chunk_row;
             sp.chunk_begin = t_chunk_begin; sp.x_partial = x_partial; sp.k_partial = k_partial;
-            int rc = launch_src<false>(sp, t_chunks, a->x, b->grad_out, b->grad_x, x_partial, st);
-            if (rc) return rc;
-            if (t_chunks > 0) {
-                chunk_sum_kernel<<<static_cast<unsigned>(t_chunks), 128, 0, st>>>(
-                    b->t_indptr, g.indptr_is64, t_chunk_edges, t_chunk_row, t_chunk_begin, static_cast<int>(D), x_partial,
-                    b->grad_x);
-                YITU_LAUNCH_CHECK();
-                chunk_sum_kernel<<<static_cast<unsigned>(t_chunks), 128, 0, st>>>(
-                    b->t_indptr, g.indptr_is64, t_chunk_edges, t_chunk_row, t_chunk_begin, static_cast<int>(H), k_partial,
-                    b->grad_key);
-                YITU_LAUNCH_CHECK();
-            }
+            if (int rc = launch_src<false>(sp, st)) return rc;
+            const HubRows h{b->t_indptr, g.indptr_is64, t_chunk_edges, t_chunks, t_chunk_row, t_chunk_begin};
+            if (int rc = launch_chunk_sum(h, D, x_partial, b->grad_x, st)) return rc;
+            if (int rc = launch_chunk_sum(h, H, k_partial, b->grad_key, st)) return rc;
         }
-        return yitu_edge_gather_sum_f32(g.n_rows, g.indptr, g.indptr_is64, nullptr, H, b->edge_grad, b->grad_query,
-                                        p.n_chunks > 0 ? a->plan : nullptr, stream);
+        return gather_sum(g.n_rows, g.indptr, g.indptr_is64, nullptr, H, b->edge_grad, b->grad_query,
+                          p.n_chunks > 0 ? a->plan : nullptr, q_partial, st);
     }
 
     // Head widths whose lanes-per-head count is not a power of two (or exceeds a warp): destination side as a gather
@@ -1410,11 +1567,8 @@ extern "C" int yitu_gat_bwd_f32(const yitu_gat_bwd_args_t *b, yitu_stream_t stre
                                            static_cast<int>(smem)));
         gat_bwd_score_kernel<<<static_cast<unsigned>((g.n_rows + p.n_chunks + warps - 1) / warps), warps * 32, smem, st>>>(p);
         YITU_LAUNCH_CHECK();
-        if (p.n_chunks > 0) {
-            chunk_sum_kernel<<<static_cast<unsigned>(p.n_chunks), 128, 0, st>>>(
-                g.indptr, g.indptr_is64, p.chunk_edges, p.chunk_row, p.chunk_begin, p.H, q_partial, b->grad_query);
-            YITU_LAUNCH_CHECK();
-        }
+        const HubRows h{g.indptr, g.indptr_is64, p.chunk_edges, p.n_chunks, p.chunk_row, p.chunk_begin};
+        if (int rc = launch_chunk_sum(h, H, q_partial, b->grad_query, st)) return rc;
     }
     yitu_hub_plan_t tp{};
     yitu_spmm_args_t s{};
@@ -1432,8 +1586,8 @@ extern "C" int yitu_gat_bwd_f32(const yitu_gat_bwd_args_t *b, yitu_stream_t stre
     }
     if (int rc = yitu_spmm_csr_f32(&s, stream)) return rc;
     if (g.n_cols == 0) return YITU_OK;
-    return yitu_edge_gather_sum_f32(g.n_cols, b->t_indptr, g.indptr_is64, b->t_perm, H, b->edge_grad, b->grad_key,
-                                    t_chunks > 0 ? b->t_plan : nullptr, stream);
+    return gather_sum(g.n_cols, b->t_indptr, g.indptr_is64, b->t_perm, H, b->edge_grad, b->grad_key,
+                      t_chunks > 0 ? b->t_plan : nullptr, k_partial, st);
 }
 
 extern "C" int yitu_spmm_bwd_f32(const yitu_spmm_bwd_args_t *a, yitu_stream_t stream) {
@@ -1463,12 +1617,7 @@ extern "C" int yitu_spmm_bwd_f32(const yitu_spmm_bwd_args_t *a, yitu_stream_t st
     sp.g_scale = 1.0f; sp.grad_x = a->grad_x; sp.n_chunks = t_chunks; sp.x_partial = a->scratch;
     sp.values = a->edge_values; sp.grad_values = a->grad_values;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (int rc = launch_src<true>(sp, t_chunks, a->x, a->grad_out, a->grad_x, a->scratch, st)) return rc;
-    if (t_chunks > 0) {
-        chunk_sum_kernel<<<static_cast<unsigned>(t_chunks), 128, 0, st>>>(a->t_indptr, g.indptr_is64, sp.chunk_edges,
-                                                                          sp.chunk_row, sp.chunk_begin,
-                                                                          static_cast<int>(D), a->scratch, a->grad_x);
-        YITU_LAUNCH_CHECK();
-    }
-    return YITU_OK;
+    if (int rc = launch_src<true>(sp, st)) return rc;
+    const HubRows h{a->t_indptr, g.indptr_is64, sp.chunk_edges, t_chunks, sp.chunk_row, sp.chunk_begin};
+    return launch_chunk_sum(h, D, a->scratch, a->grad_x, st);
 }

@@ -354,7 +354,10 @@ def epilogue_grad(y, grad_y, row_scale=None, activation=None):
 
 
 def _hub_plan(graph, chunk_edges):
-    """(pointer to the HubPlan struct or None, number of chunks, objects to keep alive)."""
+    """(pointer to the HubPlan struct or None, number of chunks, objects to keep alive); chunk_edges None: the graph's own,
+    0: no schedule."""
+    if chunk_edges is None:
+        chunk_edges = graph.chunk_edges()
     if not chunk_edges:
         return None, 0, None
     pl = graph.plan(chunk_edges)
@@ -371,7 +374,7 @@ def _heads_feats(graph, x, name):
     return x.size(1), x.size(2)
 
 
-def edge_dot(graph, grad_out, x, chunk_edges=DEFAULT_CHUNK_EDGES):
+def edge_dot(graph, grad_out, x, chunk_edges=None):
     """grad_a[e,h] = <grad_out[row_e,h,:], x[col_e,h,:]>; grad_out [n_rows,H,F], x [n_cols,H,F]."""
     H, F = _heads_feats(graph, x, "x")
     expect(grad_out, "grad_out", shape=(graph.n_rows, H, F), device=graph.device)
@@ -389,7 +392,7 @@ def spmm_bwd_supported(n_heads, n_feats):
     return n_heads <= 32 and n_feats % 4 == 0 and n_heads * n_feats <= 512 and lph <= 32 and (lph & (lph - 1)) == 0
 
 
-def spmm_bwd(graph, values, x, grad_out, chunk_edges=DEFAULT_CHUNK_EDGES):
+def spmm_bwd(graph, values, x, grad_out, chunk_edges=None):
     """(grad_values [nnz,H], grad_x [n_cols,H,F]) of the multi-head SpMM with per-edge values, in one pass over the
     transposed graph (yitu_spmm_bwd_f32); shapes outside spmm_bwd_supported take edge_dot + the transposed spmm."""
     H, F = _heads_feats(graph, x, "x")
@@ -427,7 +430,7 @@ def _query_key(graph, query, key, batched):
     return B, H
 
 
-def edge_softmax_fwd(graph, query, key, slope=0.2, chunk_edges=DEFAULT_CHUNK_EDGES):
+def edge_softmax_fwd(graph, query, key, slope=0.2, chunk_edges=None):
     """attn [nnz,H]; query [B,n_rows,H], key [n_cols,H]."""
     B, H = _query_key(graph, query, key, batched=True)
     attn = torch.zeros((graph.nnz, H), dtype=torch.float32, device=key.device)
@@ -439,7 +442,7 @@ def edge_softmax_fwd(graph, query, key, slope=0.2, chunk_edges=DEFAULT_CHUNK_EDG
     return attn
 
 
-def edge_softmax_bwd(graph, query, key, attn, grad_attn, slope=0.2, chunk_edges=DEFAULT_CHUNK_EDGES):
+def edge_softmax_bwd(graph, query, key, attn, grad_attn, slope=0.2, chunk_edges=None):
     """(grad_query [B,n_rows,H], grad_key [n_cols,H])."""
     B, H = _query_key(graph, query, key, batched=True)
     expect(attn, "attn", shape=(graph.nnz, H), device=graph.device)
@@ -476,12 +479,11 @@ def gat_fused_supported(graph, n_heads, n_feats, backward=True):
     return graph.index_mask == 0 and n_heads <= 32 and n_feats % 4 == 0 and n_heads * n_feats <= 512
 
 
-def gat_fwd(graph, query, key, x, slope=0.2, head_mean=False, activation=None, chunk_edges=DEFAULT_CHUNK_EDGES,
-            keep_heads=True):
+def gat_fwd(graph, query, key, x, slope=0.2, head_mean=False, activation=None, chunk_edges=None, keep_heads=True):
     """Fused scores + edge softmax + aggregation: (out [n_rows,H,F], row_max [n_rows,H], row_sum [n_rows,H]).
     head_mean: out is act(mean over heads), [n_rows,F], and a fourth tensor comes back: the per-head result
     [n_rows,H,F] that gat_bwd needs (None with keep_heads=False: inference, nothing is written but the mean).
-    Rows longer than chunk_edges are split over several warps (0: never)."""
+    Rows longer than chunk_edges are split over several warps (0: never, default: the graph's own length)."""
     H, F = _heads_feats(graph, x, "x")
     if _query_key(graph, query, key, batched=False)[1] != H:
         raise RuntimeError("query / key have %d heads, x has %d" % (key.size(1), H))
@@ -506,7 +508,7 @@ def gat_fwd(graph, query, key, x, slope=0.2, head_mean=False, activation=None, c
 
 
 def gat_bwd(graph, query, key, x, out, row_max, row_sum, grad_out, slope=0.2, head_mean=False, out_heads=None,
-            chunk_edges=DEFAULT_CHUNK_EDGES):
+            chunk_edges=None):
     """(grad_query, grad_key, grad_x) of gat_fwd; grad_out is the gradient of the pre-activation output
     ([n_rows,F] with head_mean, which also needs out_heads, the fourth result of gat_fwd)."""
     H, F = _heads_feats(graph, x, "x")
@@ -530,7 +532,7 @@ def gat_bwd(graph, query, key, x, out, row_max, row_sum, grad_out, slope=0.2, he
     grad_k = torch.empty_like(key)
     grad_x = torch.empty_like(x)
     lph = F // 4
-    one_pass = lph <= 32 and (lph & (lph - 1)) == 0
+    one_pass = lph <= 32 and ((lph & (lph - 1)) == 0 or H * F <= 128)
     edge_attn = None if one_pass else torch.empty((graph.nnz, H), dtype=torch.float32, device=dev)
     edge_grad = torch.empty((graph.nnz, H), dtype=torch.float32, device=dev)
     b.grad_out = _ptr(grad_out)
