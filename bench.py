@@ -68,25 +68,33 @@ def load_traffic(key, kernel):
     return rec["bytes"], rec.get("source")
 
 
-def spmm_kernel_name(nnz, n_rows, d):
-    """The SpMM instantiation that yitu_spmm_csr_f32 picks for scalar weights and aligned rows of d floats: below 64
-    edges per row on average (24 for rows of more than 128 floats) the edge-stream kernel, with the chunks of hub rows
-    on the warp-per-row kernel; above, the warp-per-row kernel alone."""
-    split = nnz < (24 if d > 128 else 64) * n_rows and 64 < d <= 256
-    if d > 128:
-        return "spmm_stream_kernel<8,4,16,true,true> (+ spmm_kernel<32,1,8,4,false,true> on hub chunks)" if split \
-            else "spmm_kernel<32,1,8,4,false,true>"
-    return "spmm_stream_kernel<4,8,16,true,true> (+ spmm_kernel<32,1,4,16,false,true> on hub chunks)" if split \
-        else "spmm_kernel<32,1,4,16,false,true>"
+def spmm_form(nnz, n_rows, d, has_hub_plan):
+    """The form that yitu_spmm_csr_f32 picks for scalar weights and aligned rows of d floats: "split" (edge-stream kernel, the
+    chunks of hub rows on the group kernel), "stream" or "group"."""
+    if not 64 < d <= 256 or nnz >= 1 << 31:
+        return "group"
+    if has_hub_plan:
+        return "split" if d <= 128 and n_rows >= 2 << 20 and nnz < 64 * n_rows else "group"
+    short = d <= 128 and nnz < 8 * n_rows
+    return "stream" if n_rows >= 150000 and nnz < 24 * n_rows and not short else "group"
+
+
+def spmm_kernel_name(nnz, n_rows, d, has_hub_plan=True):
+    """The instantiation(s) behind spmm_form, for 32-byte aligned rows of 33 to 256 floats."""
+    form = spmm_form(nnz, n_rows, d, has_hub_plan)
+    if form == "group":
+        return "spmm_group_kernel<32,8,1,8,1,true,16>" if d <= 64 else \
+            "spmm_group_kernel<16,16,1,8,2,true,12>" if d <= 128 else "spmm_group_kernel<32,32,1,8,2,true,1>"
+    stream = "spmm_stream_kernel<%s,16,%s,true>" % ("8,4" if d > 128 else "4,8", "true" if form == "split" else "false")
+    return stream + (" (+ spmm_group_kernel<32,16,1,8,8,true,1> on hub chunks)" if form == "split" else "")
 
 
 def spmm_launches(nnz, n_rows, d, has_hub_plan):
     """Kernels one scalar-weight SpMM call launches: the aggregation (two kernels where hub chunks and ordinary rows
-    go to different kernels, see spmm_kernel_name) and, with a hub schedule, the reduction of the chunk partials."""
+    go to different kernels, see spmm_form) and, with a hub schedule, the reduction of the chunk partials."""
     if not has_hub_plan:
         return 1
-    split = nnz < (24 if d > 128 else 64) * n_rows and 64 < d <= 256
-    return 3 if split else 2
+    return 3 if spmm_form(nnz, n_rows, d, True) == "split" else 2
 
 
 def roofline(kernel, algorithmic_bytes, avg_launch_ms, traffic_key, compulsory_bytes=None):
@@ -184,7 +192,7 @@ class SpmmWorkload:
         self.kernel_bytes = self.nnz * (4 * d + 8) + (n + 1) * 4 + 4 * n * d
         self.compulsory_bytes = self.nnz * 8 + (n + 1) * 4 + 2 * 4 * n * d  # every source row and output row once
         self.traffic_key = "spmm_rmat_d256"
-        self.dominant_kernel = spmm_kernel_name(self.nnz, n, d)
+        self.dominant_kernel = spmm_kernel_name(self.nnz, n, d, bool(self.g.plan()))
 
     def step(self, kernel_events=None):
         t, ops = self.torch, self.ops
@@ -281,7 +289,7 @@ class SpmmWorkload:
 class GatWorkload:
     """fused GAT layer core forward + backward."""
     name = "gat_uniform_n1048576_e33554432_h8_f32_fwd_bwd"
-    dominant_kernel = "gat_fwd_kernel_r64<2,false,false>"
+    dominant_kernel = "gat_fwd_kernel<32,32,1,8,4,1>"
 
     def __init__(self, device, n=1 << 20, e=1 << 25, H=8, F=32):
         import torch
@@ -351,7 +359,7 @@ class GatWorkload:
 class RgcnWorkload:
     """hetero RGCN aggregation: per destination type one pass over the stitched relations."""
     name = "rgcn_4types_8rel_x4M_d64"
-    dominant_kernel = "spmm_wide_kernel<8,1,true>"
+    dominant_kernel = "spmm_group_kernel<32,8,1,8,1,true,16>"
 
     def __init__(self, device, d=64):
         import torch
@@ -443,7 +451,7 @@ class UniformWorkload:
         self.kernel_bytes = self.nnz * (4 * d + 8) + (n + 1) * 8 + 4 * n * d
         self.compulsory_bytes = self.nnz * 8 + (n + 1) * 8 + 2 * 4 * n * d
         self.traffic_key = "spmm_uniform_d128"
-        self.dominant_kernel = spmm_kernel_name(self.nnz, n, d)
+        self.dominant_kernel = spmm_kernel_name(self.nnz, n, d, bool(self.g.plan()))
         self.launches_per_step = spmm_launches(self.nnz, n, d, bool(self.g.plan()))
         self.kernel_launches_per_step = 1
 

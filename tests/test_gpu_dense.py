@@ -66,6 +66,18 @@ def test_empty_and_refused_operands():
         ops.matmul(torch.randn(4, 5, device="cuda"), w, b_transposed=True)
     # other types take the library's product and keep their type
     assert ops.matmul(torch.randn(4, 16, device="cuda").half(), w.half(), b_transposed=True).dtype == torch.float16
+    # a program that allows TF32, by the older or the newer switch, keeps the library's product
+    assert ops._dense_kernels_apply(w, w)
+    for allow, back in ((lambda: torch.set_float32_matmul_precision("high"), lambda: torch.set_float32_matmul_precision("highest")),
+                        (lambda: setattr(torch.backends.cuda.matmul, "fp32_precision", "tf32"),
+                         lambda: setattr(torch.backends.cuda.matmul, "fp32_precision", "ieee"))):
+        allow()
+        try:
+            assert not ops._dense_kernels_apply(w, w)
+            assert ops.matmul(torch.randn(4, 16, device="cuda"), w, b_transposed=True).shape == (4, 8)
+        finally:
+            back()
+    assert ops._dense_kernels_apply(w, w)
     # what autograd records stays recorded
     wr = w.clone().requires_grad_(True)
     assert ops.matmul(torch.randn(4, 16, device="cuda"), wr, b_transposed=True).requires_grad

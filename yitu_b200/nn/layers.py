@@ -44,6 +44,11 @@ def _linear_grads(grad, x, w, need):
     return (gx, *ops.gram(grad, x, sums=need[2]))
 
 
+def _transformed():
+    """Whether a functorch transform or forward-mode differentiation is at work: the functions here know neither."""
+    return torch._C._are_functorch_transforms_active() or autograd.forward_ad._current_level >= 0
+
+
 class Linear(nn.Linear):
     """nn.Linear (same parameters, state and initialisation) whose float32 products on a GPU run in the framework's own
     dense kernels; every other use is nn.Linear's."""
@@ -51,7 +56,7 @@ class Linear(nn.Linear):
     def forward(self, x):
         if (type(x) in (torch.Tensor, nn.Parameter) and x.dim() == 2 and self.bias is not None and x.is_cuda and
                 x.size(1) == self.in_features and ops._dense_kernels_apply(x, self.weight) and
-                ops._dense_rows(self.bias.unsqueeze(0), x.device)):
+                ops._dense_rows(self.bias.unsqueeze(0), x.device) and not _transformed()):
             return _LinearFunction.apply(x, self.weight, self.bias)
         return nn.Linear.forward(self, x)
 

@@ -12,7 +12,7 @@ from . import _lib
 from ._lib import (ACT_ELU, ACT_NONE, ACT_RELU, Csr, GatArgs, GatBwdArgs, HubPlan, SpmmArgs, SpmmBwdArgs, W_EDGE,
                    W_EDGE_HEAD, W_NODE, W_NONE, check, lib)
 
-DEFAULT_CHUNK_EDGES = 512
+DEFAULT_CHUNK_EDGES = 512  # longest chunk of a hub row; short graphs take shorter ones (PreparedGraph.chunk_edges)
 MIN_CHUNK_EDGES = 64
 STITCH_MASK = 0xFFFFFF
 ACTIVATIONS = {None: ACT_NONE, "none": ACT_NONE, "relu": ACT_RELU, "elu": ACT_ELU}
@@ -132,8 +132,11 @@ class PreparedGraph:
         return min(max(1 << (share.bit_length() - 1), MIN_CHUNK_EDGES), DEFAULT_CHUNK_EDGES)
 
     # hub-row schedule ---------------------------------------------------------------------------
-    def plan(self, chunk_edges=DEFAULT_CHUNK_EDGES):
-        """(HubPlan struct, its two tables, pointer to the struct), or None for a graph without hub rows."""
+    def plan(self, chunk_edges=None):
+        """(HubPlan struct, its two tables, pointer to the struct), or None for a graph without hub rows;
+        chunk_edges None: the graph's own length."""
+        if chunk_edges is None:
+            chunk_edges = self.chunk_edges()
         if chunk_edges in self._plans:
             return self._plans[chunk_edges]
         L = lib()
@@ -256,11 +259,9 @@ def spmm(graph, x, *, n_heads=1, mode=W_NONE, edge_values=None, edge_perm=None, 
         accumulate = False
     else:
         expect(out, "out", numel=graph.n_rows * D, device=dev)
-    if chunk_edges is None:
-        chunk_edges = graph.chunk_edges()
     plan = scratch = None
     scratch_floats = 0
-    if chunk_edges:
+    if chunk_edges != 0:
         pl = graph.plan(chunk_edges)
         if pl is not None:
             plan, scratch_floats = pl[3], pl[0].n_chunks * D
@@ -283,12 +284,23 @@ def _dense_rows(t, device):
     return stride[1] == 1 and stride[0] >= width > 0
 
 
+_fp32_precision = getattr(torch._C, "_get_fp32_precision_getter", None)
+
+
+def _full_float32():
+    """Whether float32 products on a GPU are to be formed in float32.  Asked of the setting itself: the older
+    get_float32_matmul_precision() raises in a program that sets torch.backends.cuda.matmul.fp32_precision."""
+    if _fp32_precision is not None:
+        return _fp32_precision("cuda", "matmul") in ("ieee", "none")
+    return torch.get_float32_matmul_precision() == "highest"
+
+
 def _dense_kernels_apply(a, b):
     """Whether the framework's own dense kernels may stand in for the library GEMM: plain float32 matrices, and full
     float32 precision asked for (the default; a program that allows TF32 keeps the library's TF32 path)."""
     device = a.device
     return (device.type == "cuda" and _dense_rows(a, device) and _dense_rows(b, device) and
-            torch.get_float32_matmul_precision() == "highest" and not torch.is_autocast_enabled("cuda"))
+            _full_float32() and not torch.is_autocast_enabled("cuda"))
 
 
 def _recorded(*tensors):
@@ -356,9 +368,7 @@ def epilogue_grad(y, grad_y, row_scale=None, activation=None):
 def _hub_plan(graph, chunk_edges):
     """(pointer to the HubPlan struct or None, number of chunks, objects to keep alive); chunk_edges None: the graph's own,
     0: no schedule."""
-    if chunk_edges is None:
-        chunk_edges = graph.chunk_edges()
-    if not chunk_edges:
+    if chunk_edges == 0:
         return None, 0, None
     pl = graph.plan(chunk_edges)
     if pl is None:
