@@ -55,7 +55,7 @@ def load_peaks():
 def load_traffic(key, kernel):
     """DRAM bytes per launch of a workload's dominant kernel from the committed ncu captures
     (profiles/dram_traffic.json): (bytes, provenance), or (None, why) when there is no capture of THIS kernel on
-    this workload - a figure taken with another kernel is not reported."""
+    this workload - a figure taken with another kernel, or another instantiation of it, is not reported."""
     path = os.path.join(ROOT, "profiles", "dram_traffic.json")
     if key is None or not os.path.exists(path):
         return None, "no capture"
@@ -63,7 +63,7 @@ def load_traffic(key, kernel):
         rec = json.load(f).get(key)
     if not isinstance(rec, dict):
         return None, "no capture"
-    if rec.get("kernel", "").split("<")[0] != kernel.split("<")[0].split(" ")[0]:
+    if rec.get("kernel") != kernel:
         return None, "the capture on file is of %s" % rec.get("kernel")
     return rec["bytes"], rec.get("source")
 

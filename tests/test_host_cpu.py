@@ -343,3 +343,19 @@ def test_fused_gat_route_is_closed_for_stitched_blocks():
     assert stitch_csr([a]).is_stitched() is False
     raw = Block(st.size, [st.adj_sparse[0].clone(), st.adj_sparse[1].clone()])
     assert raw.stitched is None and raw.is_stitched() is True
+
+
+def test_bench_reports_dram_traffic_of_the_kernels_that_run_only(tmp_path, monkeypatch):
+    """A capture counts for the complete name it was taken under: instantiation and companion kernels included."""
+    import bench
+
+    (tmp_path / "profiles").mkdir()
+    names = [bench.spmm_kernel_name(520_000_000, 1 << 24, 128), bench.spmm_kernel_name(63_000_000, 1 << 21, 256),
+             bench.spmm_kernel_name(30_000_000, 1 << 22, 64), bench.spmm_kernel_name(134_000_000, 1 << 23, 128, False)]
+    assert len(set(names)) == 4
+    for name in names:
+        (tmp_path / "profiles" / "dram_traffic.json").write_text(json.dumps({"w": {"bytes": 7, "kernel": name, "source": "s"}}))
+        monkeypatch.setattr(bench, "ROOT", str(tmp_path))
+        assert bench.load_traffic("w", name) == (7, "s")
+        for other in [n for n in names if n != name] + [name.split(" ")[0] + "x", name.replace("true", "false"), name.split("<")[0]]:
+            assert bench.load_traffic("w", other)[0] is None
