@@ -592,3 +592,35 @@ def test_fused_gat_with_infinite_scores(H, F):
             ref = (a.unsqueeze(-1) * x[c].double()).sum(0)
             assert float((out[row].double() - ref).abs().max()) <= 1e-5 * float(ref.abs().max()) + 1e-6
         assert bool(torch.isnan(out[1]).all()) and float(out[3].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("head_mean", [False, True])
+@pytest.mark.parametrize("H,F", [(1, 4), (2, 8), (3, 20), (4, 16), (8, 8), (4, 32), (8, 32), (8, 64)])
+def test_fused_gat_backward_of_unused_sources_is_zero(H, F, head_mean):
+    """A source without out-edges has zero gradients whatever its features hold (padded rows of uninitialised memory are such
+    sources), and changes no other source's; it shares its warp with sources that have edges."""
+    from yitu_b200 import ops
+    n_dst, n_src = 40, 67
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(H * 100 + F)
+    used = torch.tensor([c for c in range(n_src) if c % 3], dtype=torch.int32, device="cuda")
+    degs = torch.arange(n_dst, device="cuda") % 9
+    indptr = torch.zeros(n_dst + 1, dtype=torch.int32, device="cuda")
+    indptr[1:] = degs.cumsum(0).to(torch.int32)
+    indices = used[torch.randint(0, used.numel(), (int(degs.sum()),), device="cuda", generator=gen)]
+    q, k = (torch.randn(n, H, device="cuda", generator=gen) for n in (n_dst, n_src))
+    x = torch.randn(n_src, H, F, device="cuda", generator=gen)
+    grad = torch.randn(*((n_dst, F) if head_mean else (n_dst, H, F)), device="cuda", generator=gen)
+
+    def gradients(x):
+        g = ops.PreparedGraph(indptr, indices, n_src)
+        res = ops.gat_fwd(g, q, k, x, head_mean=head_mean)
+        return ops.gat_bwd(g, q, k, x, *res[:3], grad, head_mean=head_mean, out_heads=res[3] if head_mean else None)
+
+    want = gradients(x)
+    odd = x.clone()
+    odd[0::9], odd[3::9], odd[6::9] = float("inf"), float("nan"), -float("inf")
+    got = gradients(odd)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    assert float(got[1][0::3].abs().max()) == 0.0 and float(got[2][0::3].abs().max()) == 0.0

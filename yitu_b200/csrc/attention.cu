@@ -1112,7 +1112,7 @@ __global__ void __launch_bounds__(128, MINB) gat_bwd_src_kernel(const __grid_con
                     pr = expf(leaky_relu(sc, p.slope) - rec[u][i].y);
                     if (!live) pr = 0.0f;
                     out = (sc < 0.0f ? pr * p.slope : pr) * (dp - rec[u][i].z);
-                    gk[i] += out;
+                    if (live) gk[i] += out;  // without an edge dp is 0 * x[c]: NaN where x[c] is not finite
                 }
 #pragma unroll
                 for (int v = 0; v < VEC; ++v) acc[i][v] = fmaf(pr, gv[u][i][v], acc[i][v]);
