@@ -136,3 +136,22 @@ def test_first_layer_skips_the_input_gradient():
         conv.weights.requires_grad_(False)
         gx2, = torch.autograd.grad(conv(xr, info).square().sum(), [xr])
         assert torch.equal(gx, gx2)
+
+
+@pytest.mark.parametrize("M,N", [(5, 12), (16, 64), (33, 40), (64, 64), (100, 128), (80, 9)])
+def test_column_sums_with_infinite_values(M, N):
+    """Infinite, overflowing and undefined columns end as they do in torch.sum; the others do not see them."""
+    from yitu_b200 import ops
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(M)
+    n = 20011
+    g, x = torch.randn(n, M, device="cuda", generator=gen), torch.randn(n, N, device="cuda", generator=gen)
+    clean = ops.gram(g, x, sums=True)[1]
+    g[7000, 0] = float("inf")
+    g[0, 1] = -float("inf")
+    g[n - 1, 1] = float("inf")
+    g[11, 2] = float("nan")
+    g[:40, 3] = 3e38
+    sums = ops.gram(g, x, sums=True)[1]
+    assert float(sums[0]) == float("inf") and bool(torch.isnan(sums[1:3]).all()) and float(sums[3]) == float("inf")
+    assert torch.equal(sums[4:], clean[4:])

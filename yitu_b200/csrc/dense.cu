@@ -2,6 +2,8 @@
 //   yitu_linear_f32  C[n,N] = A[n,K] B (+ bias): the layer's x W^T + b, x W, and the input gradient g W
 //   yitu_gram_f32    C[M,N] = A[n,M]^T B[n,N] and, from the same pass, the column sums of A: weight and bias gradient
 // Plain float32 multiply-adds throughout: no operand or partial sum is held in fewer bits.
+#include <math_constants.h>
+
 #include "common.cuh"
 
 namespace yitu {
@@ -275,11 +277,12 @@ __global__ void __launch_bounds__(256, 2) gram_kernel(const __grid_constant__ Gr
     const bool sums = (p.sum_of == 1 && tb == 0) || (p.sum_of == 2 && ta == 0);
     const int sw = p.sum_of == 2 ? TB : TA, sum_off = p.sum_of == 2 ? BK * TA : 0;
     const int sum_c = (tid % (sw / 4)) * 4, sum_r = tid / (sw / 4), sum_step = 256 / (sw / 4);
-    // compensated: a split's column is a chain of thousands of additions, and the library's sums are trees
+    // compensated: a split's column is a chain of thousands of additions, and the library's sums are trees.  A sum that has
+    // become infinite (an infinite value, or overflow) goes on without: the compensation would be inf - inf
     float4 cs = make_float4(0.f, 0.f, 0.f, 0.f), cc = cs;
     const auto add = [](float v, float &sum, float &comp) {
         const float y = __fsub_rn(v, comp), t = __fadd_rn(sum, y);
-        comp = __fsub_rn(__fsub_rn(t, sum), y);
+        comp = fabsf(t) < CUDART_INF_F ? __fsub_rn(__fsub_rn(t, sum), y) : 0.0f;
         sum = t;
     };
 
