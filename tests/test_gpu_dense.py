@@ -155,3 +155,27 @@ def test_column_sums_with_infinite_values(M, N):
     sums = ops.gram(g, x, sums=True)[1]
     assert float(sums[0]) == float("inf") and bool(torch.isnan(sums[1:3]).all()) and float(sums[3]) == float("inf")
     assert torch.equal(sums[4:], clean[4:])
+
+
+def test_linear_saves_what_its_backward_reads():
+    """As with torch's own product, a weight whose input needs no gradient may be updated before the backward pass, and so may
+    the input of a frozen weight."""
+    from yitu_b200.nn.layers import Linear
+    lin, x, g = Linear(24, 12).cuda(), torch.randn(500, 24, device="cuda"), torch.randn(500, 12, device="cuda")
+    want = g.t() @ x
+    out = lin(x)
+    with torch.no_grad():
+        lin.weight.zero_()
+    gw, gb = torch.autograd.grad(out, [lin.weight, lin.bias], g)
+    assert float((gw - want).abs().max()) <= 1e-4 * float(want.abs().max())
+    lin.weight.requires_grad_(False)
+    with torch.no_grad():
+        lin.weight.normal_()
+    leaf = torch.randn(500, 24, device="cuda", requires_grad=True)
+    x = leaf * 2
+    out = lin(x)
+    x.data.zero_()
+    with torch.no_grad():
+        x.add_(1.0)
+    gx, gb = torch.autograd.grad(out, [leaf, lin.bias], g)
+    assert float((gx - 2 * g @ lin.weight).abs().max()) <= 1e-4 * float(gx.abs().max())

@@ -24,7 +24,8 @@ class _LinearFunction(autograd.Function):
 
     @staticmethod
     def forward(ctx, x, w, b):
-        ctx.save_for_backward(x, w)
+        # only what the backward reads, as torch's own product does: the other operand may be written to in between
+        ctx.save_for_backward(x if ctx.needs_input_grad[1] else None, w if ctx.needs_input_grad[0] else None)
         return ops.matmul(x, w, b_transposed=True, bias=b)
 
     @staticmethod
