@@ -179,3 +179,19 @@ def test_linear_saves_what_its_backward_reads():
         x.add_(1.0)
     gx, gb = torch.autograd.grad(out, [leaf, lin.bias], g)
     assert float((gx - 2 * g @ lin.weight).abs().max()) <= 1e-4 * float(gx.abs().max())
+
+
+def test_linear_is_seen_by_tracers_and_dispatch_modes():
+    """A traced or counted Linear is nn.Linear's product, not a constant of the example input."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from torch.utils.flop_counter import FlopCounterMode
+    from yitu_b200.nn.layers import Linear
+    lin = Linear(24, 12).cuda().requires_grad_(False)
+    x, y = torch.randn(50, 24, device="cuda"), torch.randn(50, 24, device="cuda")
+    want = torch.nn.functional.linear(y, lin.weight, lin.bias)
+    compiled = torch.compile(lin, backend="eager", fullgraph=True)
+    for f in (make_fx(lin)(x), torch.jit.trace(lin, x), compiled):
+        assert float((f(y) - want).abs().max()) <= 1e-5 * float(want.abs().max())
+    with FlopCounterMode(display=False) as counter:
+        lin(x)
+    assert counter.get_total_flops() == 2 * 50 * 24 * 12

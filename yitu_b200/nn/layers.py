@@ -46,8 +46,11 @@ def _linear_grads(grad, x, w, need):
 
 
 def _transformed():
-    """Whether a functorch transform or forward-mode differentiation is at work: the functions here know neither."""
-    return torch._C._are_functorch_transforms_active() or autograd.forward_ad._current_level >= 0
+    """Whether something other than plain execution is at work, which a kernel launch on raw addresses would be hidden from: a
+    functorch transform, forward-mode differentiation, a tracer, a compiler or a dispatch mode (make_fx, FLOP counters)."""
+    return (torch.compiler.is_compiling() or torch._C._are_functorch_transforms_active() or
+            autograd.forward_ad._current_level >= 0 or torch._C._get_tracing_state() is not None or
+            torch._C._len_torch_dispatch_stack() > 0)
 
 
 class Linear(nn.Linear):
@@ -55,9 +58,9 @@ class Linear(nn.Linear):
     dense kernels; every other use is nn.Linear's."""
 
     def forward(self, x):
-        if (type(x) in (torch.Tensor, nn.Parameter) and x.dim() == 2 and self.bias is not None and x.is_cuda and
-                x.size(1) == self.in_features and ops._dense_kernels_apply(x, self.weight) and
-                ops._dense_rows(self.bias.unsqueeze(0), x.device) and not _transformed()):
+        if (not _transformed() and type(x) in (torch.Tensor, nn.Parameter) and x.dim() == 2 and self.bias is not None and
+                x.is_cuda and x.size(1) == self.in_features and ops._dense_kernels_apply(x, self.weight) and
+                ops._dense_rows(self.bias.unsqueeze(0), x.device)):
             return _LinearFunction.apply(x, self.weight, self.bias)
         return nn.Linear.forward(self, x)
 
