@@ -557,7 +557,7 @@ def test_fused_gat_group_widths(oracle, H, F, head_mean):
         t = torch.empty(a.size + 4, device="cuda")[4:].view(*a.shape)
         return t.copy_(_dev(a))
 
-    for place, chunk in ((_dev, 64), (_dev, None), (shifted, 64), (_dev, 0)):
+    for place, chunk in ((_dev, 64), (_dev, ops.OWN_CHUNKS), (shifted, 64), (_dev, 0)):
         for dtype in (torch.int32, torch.int64):
             graph = ops.PreparedGraph(_dev(indptr).to(dtype), _dev(indices), n)
             dx, dg = place(x), place(g_in)

@@ -180,7 +180,7 @@ def test_group_kernel_dispatch_edges(oracle, monkeypatch, D, degrees):
     ref = oracle.spmm(indptr, indices, x, wmode=oracle.W_EDGE, values=vals)
     ref_acc = np.maximum(oracle.spmm(indptr, indices, x, alpha=0.5, out=base) + bias, 0)
     g = ops.PreparedGraph(_dev(indptr, torch.int32), _dev(indices), n_cols)
-    for chunk in (0, 64, None):
+    for chunk in (0, 64, ops.OWN_CHUNKS):
         got = ops.spmm(g, _dev(x), mode=ops.W_EDGE, edge_values=_dev(vals), chunk_edges=chunk)
         assert_close(got.cpu().numpy(), ref, what="group %s D=%d chunk=%s" % (degrees, D, chunk))
         out = _dev(base).clone()
@@ -427,3 +427,33 @@ def test_partitioned_config_on_one_gpu_sampled_rows_against_float64():
     from conftest import record_error
     big = truth.abs() >= 0.01 * scale
     record_error("partitioned-config-1gpu", float(err.max()) / scale, float((err[big] / truth.abs()[big]).max()))
+
+
+def test_no_chunks_means_no_schedule():
+    """chunk_edges 0 and None: rows are not split and no schedule is built, so a first call may be captured in a CUDA graph."""
+    from yitu_b200 import ops
+    n, deg = 50, 700
+    indptr = torch.arange(0, (n + 1) * deg, deg, dtype=torch.int32, device="cuda")
+    indices = torch.randint(0, n, (n * deg,), device="cuda").to(torch.int32)
+    x, q, k = torch.randn(n, 2, 8, device="cuda"), torch.randn(n, 2, device="cuda"), torch.randn(n, 2, device="cuda")
+    attn = torch.rand(n * deg, 2, device="cuda")
+    grad = torch.randn(n, 2, 8, device="cuda")
+
+    def calls(g, chunk):
+        gat = ops.gat_fwd(g, q, k, x, chunk_edges=chunk)
+        ops.gat_bwd(g, q, k, x, *gat, grad, chunk_edges=chunk)
+        ops.edge_dot(g, grad, x, chunk_edges=chunk)
+        ops.spmm_bwd(g, attn, x, grad, chunk_edges=chunk)
+        ops.edge_softmax_bwd(g, q[None], k, ops.edge_softmax_fwd(g, q[None], k, chunk_edges=chunk), attn, chunk_edges=chunk)
+        return ops.spmm(g, x, chunk_edges=chunk)
+
+    want = calls(ops.PreparedGraph(indptr, indices, n), 0)
+    for chunk in (0, None):
+        g = ops.PreparedGraph(indptr, indices, n)
+        g.t_prepared()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = calls(g, chunk)
+        assert not g._plans and not g.t_prepared()._plans
+        graph.replay()
+        assert torch.equal(out, want)

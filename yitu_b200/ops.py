@@ -14,6 +14,7 @@ from ._lib import (ACT_ELU, ACT_NONE, ACT_RELU, Csr, GatArgs, GatBwdArgs, HubPla
 
 DEFAULT_CHUNK_EDGES = 512  # longest chunk of a hub row; short graphs take shorter ones (PreparedGraph.chunk_edges)
 MIN_CHUNK_EDGES = 64
+OWN_CHUNKS = "own"  # chunk_edges: the graph's own length, PreparedGraph.chunk_edges(); 0 or None: rows are never split
 STITCH_MASK = 0xFFFFFF
 ACTIVATIONS = {None: ACT_NONE, "none": ACT_NONE, "relu": ACT_RELU, "elu": ACT_ELU}
 
@@ -132,10 +133,9 @@ class PreparedGraph:
         return min(max(1 << (share.bit_length() - 1), MIN_CHUNK_EDGES), DEFAULT_CHUNK_EDGES)
 
     # hub-row schedule ---------------------------------------------------------------------------
-    def plan(self, chunk_edges=None):
-        """(HubPlan struct, its two tables, pointer to the struct), or None for a graph without hub rows;
-        chunk_edges None: the graph's own length."""
-        if chunk_edges is None:
+    def plan(self, chunk_edges=OWN_CHUNKS):
+        """(HubPlan struct, its two tables, pointer to the struct), or None for a graph without hub rows."""
+        if chunk_edges == OWN_CHUNKS:
             chunk_edges = self.chunk_edges()
         if chunk_edges in self._plans:
             return self._plans[chunk_edges]
@@ -216,13 +216,13 @@ def prepared(indptr, indices, n_cols, index_mask=0):
 
 
 def spmm(graph, x, *, n_heads=1, mode=W_NONE, edge_values=None, edge_perm=None, norm_dst=None, norm_src=None,
-         row_scale=None, alpha=1.0, out=None, accumulate=False, chunk_edges=None, bias=None, activation=None,
+         row_scale=None, alpha=1.0, out=None, accumulate=False, chunk_edges=OWN_CHUNKS, bias=None, activation=None,
          x_shared_heads=False):
     """out[r,h,k] = act(alpha*row_scale[r] * sum_e w(e,h) * x[col_e,h,k] + bias[h,k]) through yitu_spmm_csr_f32.
 
     x: [n_cols, H*F] or [n_cols, H, F] float32 CUDA; returns a tensor shaped like x with n_rows rows.
     x_shared_heads (per-head edge values only): x is [n_cols, F] and every head reads the same row; the result is
-    [n_rows, H, F].  Rows longer than chunk_edges are split (0: never; default: the graph's own chunk_edges())."""
+    [n_rows, H, F].  Rows longer than chunk_edges are split (0 or None: never; default: the graph's own length)."""
     if not isinstance(x, torch.Tensor) or x.dtype != torch.float32:
         raise RuntimeError("features must be a float32 tensor, got %s" % getattr(x, "dtype", type(x).__name__))
     if x.dim() < 2 or x.size(0) != graph.n_cols:
@@ -261,7 +261,7 @@ def spmm(graph, x, *, n_heads=1, mode=W_NONE, edge_values=None, edge_perm=None, 
         expect(out, "out", numel=graph.n_rows * D, device=dev)
     plan = scratch = None
     scratch_floats = 0
-    if chunk_edges != 0:
+    if chunk_edges:
         pl = graph.plan(chunk_edges)
         if pl is not None:
             plan, scratch_floats = pl[3], pl[0].n_chunks * D
@@ -366,9 +366,8 @@ def epilogue_grad(y, grad_y, row_scale=None, activation=None):
 
 
 def _hub_plan(graph, chunk_edges):
-    """(pointer to the HubPlan struct or None, number of chunks, objects to keep alive); chunk_edges None: the graph's own,
-    0: no schedule."""
-    if chunk_edges == 0:
+    """(pointer to the HubPlan struct or None, number of chunks, objects to keep alive)."""
+    if not chunk_edges:
         return None, 0, None
     pl = graph.plan(chunk_edges)
     if pl is None:
@@ -384,7 +383,7 @@ def _heads_feats(graph, x, name):
     return x.size(1), x.size(2)
 
 
-def edge_dot(graph, grad_out, x, chunk_edges=None):
+def edge_dot(graph, grad_out, x, chunk_edges=OWN_CHUNKS):
     """grad_a[e,h] = <grad_out[row_e,h,:], x[col_e,h,:]>; grad_out [n_rows,H,F], x [n_cols,H,F]."""
     H, F = _heads_feats(graph, x, "x")
     expect(grad_out, "grad_out", shape=(graph.n_rows, H, F), device=graph.device)
@@ -402,7 +401,7 @@ def spmm_bwd_supported(n_heads, n_feats):
     return n_heads <= 32 and n_feats % 4 == 0 and n_heads * n_feats <= 512 and lph <= 32 and (lph & (lph - 1)) == 0
 
 
-def spmm_bwd(graph, values, x, grad_out, chunk_edges=None):
+def spmm_bwd(graph, values, x, grad_out, chunk_edges=OWN_CHUNKS):
     """(grad_values [nnz,H], grad_x [n_cols,H,F]) of the multi-head SpMM with per-edge values, in one pass over the
     transposed graph (yitu_spmm_bwd_f32); shapes outside spmm_bwd_supported take edge_dot + the transposed spmm."""
     H, F = _heads_feats(graph, x, "x")
@@ -440,7 +439,7 @@ def _query_key(graph, query, key, batched):
     return B, H
 
 
-def edge_softmax_fwd(graph, query, key, slope=0.2, chunk_edges=None):
+def edge_softmax_fwd(graph, query, key, slope=0.2, chunk_edges=OWN_CHUNKS):
     """attn [nnz,H]; query [B,n_rows,H], key [n_cols,H]."""
     B, H = _query_key(graph, query, key, batched=True)
     attn = torch.zeros((graph.nnz, H), dtype=torch.float32, device=key.device)
@@ -452,7 +451,7 @@ def edge_softmax_fwd(graph, query, key, slope=0.2, chunk_edges=None):
     return attn
 
 
-def edge_softmax_bwd(graph, query, key, attn, grad_attn, slope=0.2, chunk_edges=None):
+def edge_softmax_bwd(graph, query, key, attn, grad_attn, slope=0.2, chunk_edges=OWN_CHUNKS):
     """(grad_query [B,n_rows,H], grad_key [n_cols,H])."""
     B, H = _query_key(graph, query, key, batched=True)
     expect(attn, "attn", shape=(graph.nnz, H), device=graph.device)
@@ -489,11 +488,11 @@ def gat_fused_supported(graph, n_heads, n_feats, backward=True):
     return graph.index_mask == 0 and n_heads <= 32 and n_feats % 4 == 0 and n_heads * n_feats <= 512
 
 
-def gat_fwd(graph, query, key, x, slope=0.2, head_mean=False, activation=None, chunk_edges=None, keep_heads=True):
+def gat_fwd(graph, query, key, x, slope=0.2, head_mean=False, activation=None, chunk_edges=OWN_CHUNKS, keep_heads=True):
     """Fused scores + edge softmax + aggregation: (out [n_rows,H,F], row_max [n_rows,H], row_sum [n_rows,H]).
     head_mean: out is act(mean over heads), [n_rows,F], and a fourth tensor comes back: the per-head result
     [n_rows,H,F] that gat_bwd needs (None with keep_heads=False: inference, nothing is written but the mean).
-    Rows longer than chunk_edges are split over several warps (0: never, default: the graph's own length)."""
+    Rows longer than chunk_edges are split over several warps (0 or None: never, default: the graph's own length)."""
     H, F = _heads_feats(graph, x, "x")
     if _query_key(graph, query, key, batched=False)[1] != H:
         raise RuntimeError("query / key have %d heads, x has %d" % (key.size(1), H))
@@ -518,7 +517,7 @@ def gat_fwd(graph, query, key, x, slope=0.2, head_mean=False, activation=None, c
 
 
 def gat_bwd(graph, query, key, x, out, row_max, row_sum, grad_out, slope=0.2, head_mean=False, out_heads=None,
-            chunk_edges=None):
+            chunk_edges=OWN_CHUNKS):
     """(grad_query, grad_key, grad_x) of gat_fwd; grad_out is the gradient of the pre-activation output
     ([n_rows,F] with head_mean, which also needs out_heads, the fourth result of gat_fwd)."""
     H, F = _heads_feats(graph, x, "x")
