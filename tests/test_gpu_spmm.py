@@ -457,3 +457,30 @@ def test_no_chunks_means_no_schedule():
         assert not g._plans and not g.t_prepared()._plans
         graph.replay()
         assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("D", [1, 8, 24, 41, 64, 100, 128, 200, 256, 264])
+def test_node_weights_do_not_depend_on_the_graph_around_a_row(monkeypatch, D):
+    """norm_dst[r] * sum of norm_src[c] x[c] is rounded the same way in every graph and kernel, and a row without edges is 0
+    even where its factor is infinite (1 / sqrt(0))."""
+    from yitu_b200 import ops
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(D)
+    degs = torch.tensor([3, 0, 30, 7, 0, 60], device="cuda")
+    n_cols = 200
+    indices = torch.randint(0, n_cols, (int(degs.sum()),), device="cuda", generator=gen).to(torch.int32)
+    x, ns = torch.randn(n_cols, D, device="cuda", generator=gen), torch.rand(n_cols, device="cuda", generator=gen)
+    nd = torch.rand(degs.numel(), device="cuda", generator=gen)
+    nd[degs == 0] = float("inf")
+    results = []
+    for stream in ("0", "1", "2"):
+        monkeypatch.setenv("YITU_SPMM_STREAM", stream)
+        for pad in (0, 600):  # empty rows behind: the average row of the graph is short or long
+            indptr = torch.zeros(degs.numel() + pad + 1, dtype=torch.int32, device="cuda")
+            indptr[1:] = torch.cat([degs, degs.new_zeros(pad)]).cumsum(0).to(torch.int32)
+            g = ops.PreparedGraph(indptr, indices, n_cols)
+            norm = torch.cat([nd, nd.new_full((pad,), float("inf"))])
+            results.append(ops.spmm(g, x, mode=ops.W_NODE, norm_dst=norm, norm_src=ns)[:degs.numel()])
+            assert float(results[-1][degs == 0].abs().max()) == 0.0
+    for r in results[1:]:
+        assert torch.equal(r, results[0])

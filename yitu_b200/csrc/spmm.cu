@@ -51,7 +51,6 @@ struct SpmmParams {
     float *scratch;
     const float *bias;
     int act, xshared;
-    int node_late;  // W_NODE: the destination's factor is applied to the row's sum instead of to every edge
 };
 
 // Last step of every output row: bias, then activation (both optional).
@@ -243,8 +242,6 @@ __global__ void __launch_bounds__(128, CTAS) spmm_group_kernel(const __grid_cons
 #pragma unroll
         for (int q = 0; q < VEC; ++q) acc[i][q] = 0.0f;
     }
-    const float nd = (p.wmode == YITU_W_NODE) ? __ldg(p.norm_dst + row) : 0.0f;
-    const float nd_edge = p.node_late ? 1.0f : nd;
 
     auto load_tile = [&](uint32_t e, int &col, float &w) {  // e: this lane's edge of the tile
         col = 0;
@@ -255,7 +252,7 @@ __global__ void __launch_bounds__(128, CTAS) spmm_group_kernel(const __grid_cons
             if (p.wmode == YITU_W_NONE) {
                 w = 1.0f;
             } else if (p.wmode == YITU_W_NODE) {
-                w = nd_edge * __ldg(p.norm_src + col);
+                w = __ldg(p.norm_src + col);  // the destination's factor is applied once per row, at the end
             } else {
                 w = ld_stream(p.values + (p.perm ? static_cast<int64_t>(ld_stream(p.perm + eb + e)) : eb + e));
             }
@@ -335,9 +332,10 @@ __global__ void __launch_bounds__(128, CTAS) spmm_group_kernel(const __grid_cons
     }
     if (!owner || !store) return;
     float *dst = raw ? p.scratch + gid * p.D : p.out + row * p.os;
-    // a hub row's chunk is left unscaled, but fully weighted
+    // a hub row's chunk is left unscaled, but fully weighted; a row without edges is 0 whatever its factor
+    const bool node = p.wmode == YITU_W_NODE && len > 0;
     float s = raw ? 1.0f : p.alpha * (p.row_scale ? __ldg(p.row_scale + row) : 1.0f);
-    if (p.node_late) s *= nd;
+    if (node) s *= __ldg(p.norm_dst + row);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
         if (!valid[i]) continue;
@@ -346,7 +344,7 @@ __global__ void __launch_bounds__(128, CTAS) spmm_group_kernel(const __grid_cons
 #pragma unroll
         for (int q = 0; q < PIECE; ++q) r[q] = acc[i][q];
         if (raw) {
-            if (p.node_late) {
+            if (node) {
 #pragma unroll
                 for (int q = 0; q < PIECE; ++q) r[q] *= s;
             }
@@ -459,7 +457,7 @@ __global__ void __launch_bounds__(128, (VEC * EU <= 32) ? 6 : 4) spmm_stream_ker
                 const bool had = cur_end > cur_begin;
                 if (valid && (had || !p.accumulate || p.bias || p.act)) {
                     float s = p.alpha * (p.row_scale ? __ldg(p.row_scale + row) : 1.0f);
-                    if (p.wmode == YITU_W_NODE) s *= __ldg(p.norm_dst + row);
+                    if (p.wmode == YITU_W_NODE && had) s *= __ldg(p.norm_dst + row);
                     float *dst = p.out + row * p.os + off;
                     float r[VEC];
                     if (p.accumulate) {
@@ -817,8 +815,6 @@ extern "C" int yitu_spmm_csr_f32(const yitu_spmm_args_t *a, yitu_stream_t stream
         }
         return D > 128 ? dispatch_stream<8, 4, 8>(r, st, 16, 4) : dispatch_stream<4, 8, 16>(r, st, 16, 8);
     }
-    // rows of few edges: the destination's factor once per row, as the stream kernel does
-    p.node_late = p.wmode == YITU_W_NODE && stream_shape && g.nnz < (D > 128 ? 24 : 64) * g.n_rows;
     if (vec8_ok) return dispatch_group8(p, st);
     return dispatch_group4(p, st);
 }
