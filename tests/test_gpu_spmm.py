@@ -484,3 +484,23 @@ def test_node_weights_do_not_depend_on_the_graph_around_a_row(monkeypatch, D):
             assert float(results[-1][degs == 0].abs().max()) == 0.0
     for r in results[1:]:
         assert torch.equal(r, results[0])
+
+
+@pytest.mark.parametrize("D", [1, 4, 8, 12, 32, 41, 48, 64, 96, 128, 200, 256, 264])
+def test_long_rows_in_pieces(oracle, monkeypatch, D):
+    """Rows whose edges do not fit 32 bits are walked in pieces; here the pieces are 64 edges, so that rows end inside, at and
+    behind a piece, next to rows of one piece and to chunks of a schedule."""
+    from yitu_b200 import ops
+    monkeypatch.setenv("YITU_SPMM_STREAM", "0")
+    rng = np.random.default_rng(D)
+    n_cols = 700
+    indptr, indices = _csr_from_degrees(rng, [0, 1, 63, 64, 65, 128, 129, 3, 300, 500, 0, 640, 7], n_cols)
+    x, vals = rng.standard_normal((n_cols, D)).astype(np.float32), rng.standard_normal(indices.shape[0]).astype(np.float32)
+    g = ops.PreparedGraph(_dev(indptr, torch.int64), _dev(indices), n_cols)
+    for chunk in (0, 256):
+        whole = ops.spmm(g, _dev(x), mode=ops.W_EDGE, edge_values=_dev(vals), chunk_edges=chunk)
+        monkeypatch.setenv("YITU_SPMM_PIECE", "64")
+        got = ops.spmm(g, _dev(x), mode=ops.W_EDGE, edge_values=_dev(vals), chunk_edges=chunk)
+        monkeypatch.delenv("YITU_SPMM_PIECE")
+        assert torch.equal(got, whole)
+        assert_close(got.cpu().numpy(), oracle.spmm(indptr, indices, x, wmode=oracle.W_EDGE, values=vals), what="pieces D=%d" % D)

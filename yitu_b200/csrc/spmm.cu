@@ -30,7 +30,7 @@
 namespace yitu {
 
 struct SpmmParams {
-    int64_t n_rows, n_cols, D, H, F;
+    int64_t n_rows, n_cols, nnz, D, H, F;
     const void *indptr;
     const int *indices;
     int is64, mask, wmode, accumulate;
@@ -51,6 +51,7 @@ struct SpmmParams {
     float *scratch;
     const float *bias;
     int act, xshared;
+    uint32_t piece;  // spmm_group_kernel without SMALL walks longer rows in pieces of this many edges
 };
 
 // Last step of every output row: bias, then activation (both optional).
@@ -200,8 +201,9 @@ __global__ void __launch_bounds__(256) spmm_heads_kernel(const __grid_constant__
 //   What bounds it: DRAM and L2 bandwidth for wide rows; for narrow ones the chain of three dependent latencies per row
 // (row pointer, ids, gathers).  A row's edges are therefore gathered 8 to 16 at a time, and the next tile of ids is
 // requested before the current one is consumed.
-template <int RW, int LPE, int NV, int VEC, int EU, bool IDX32, int CTAS>
-__global__ void __launch_bounds__(128, CTAS) spmm_group_kernel(const __grid_constant__ SpmmParams p) {
+//   SMALL: element offsets into x and the edges of a row fit 32 bits.
+template <int RW, int LPE, int NV, int VEC, int EU, bool SMALL, int CTAS>
+__global__ void __launch_bounds__(128, SMALL || CTAS < 16 ? CTAS : 12) spmm_group_kernel(const __grid_constant__ SpmmParams p) {
     constexpr int EPI = RW / LPE;  // edges per load instruction
     constexpr int STEP = EPI * EU;
     static_assert(RW % LPE == 0 && RW % STEP == 0, "a tile of RW ids is consumed in whole steps");
@@ -215,7 +217,8 @@ __global__ void __launch_bounds__(128, CTAS) spmm_group_kernel(const __grid_cons
     bool store = true;  // a group without a row, or with a hub row (done by its chunks), keeps its warp company
     int row;
     int64_t eb;
-    uint32_t len;  // edges of the row or chunk, counted from eb (registers are what limits the warps per SM here)
+    uint32_t len;  // edges of the row or chunk, counted from eb, in 32 bits (registers are what limits the warps per SM here):
+                   // without SMALL a longer row (int64 row pointers) is walked in pieces of 2^31
     if (raw) {
         row = __ldg(p.chunk_row + gid);
         eb = __ldg(p.chunk_begin + gid);
@@ -224,8 +227,9 @@ __global__ void __launch_bounds__(128, CTAS) spmm_group_kernel(const __grid_cons
         store = gid - p.chunk_tasks < p.row_tasks;
         row = store ? static_cast<int>(gid - p.chunk_tasks) : 0;
         eb = load_ptr(p.indptr, p.is64, row);
-        len = static_cast<uint32_t>(load_ptr(p.indptr, p.is64, row + 1) - eb);
-        store = store && !(p.n_chunks > 0 && len > static_cast<uint32_t>(p.chunk_edges));
+        const int64_t edges = load_ptr(p.indptr, p.is64, row + 1) - eb;
+        len = static_cast<uint32_t>(SMALL ? edges : min(edges, static_cast<int64_t>(p.piece)));
+        store = store && !(p.n_chunks > 0 && edges > p.chunk_edges);
         if (!store) {
             if (RW == 32) return;
             len = 0;
@@ -258,51 +262,60 @@ __global__ void __launch_bounds__(128, CTAS) spmm_group_kernel(const __grid_cons
             }
         }
     };
-    int my_col;
-    float my_w;
-    load_tile(gl, my_col, my_w);
-    // with several rows per warp every group takes the trips of the longest: groups that leave each other would execute one
-    // after the other
-    for (uint32_t e0 = 0; RW == 32 ? e0 < len : __any_sync(FULL, e0 < len); e0 += RW) {
-        const int n = e0 < len ? static_cast<int>(min(static_cast<uint32_t>(RW), len - e0)) : 0;
-        const int most = RW == 32 ? n : __reduce_max_sync(FULL, n);
-        int nx_col = 0;
-        float nx_w = 0.0f;
-        load_tile(e0 + RW + gl, nx_col, nx_w);
-        for (int j = 0; j < most; j += STEP) {
-            int c[EU];
-            float w[EU];
+    const bool empty = len == 0;
+    while (true) {
+        int my_col;
+        float my_w;
+        load_tile(gl, my_col, my_w);
+        // with several rows per warp every group takes the trips of the longest: groups that leave each other would execute one
+        // after the other
+        for (uint32_t e0 = 0; RW == 32 ? e0 < len : __any_sync(FULL, e0 < len); e0 += RW) {
+            const int n = e0 < len ? static_cast<int>(min(static_cast<uint32_t>(RW), len - e0)) : 0;
+            const int most = RW == 32 ? n : __reduce_max_sync(FULL, n);
+            int nx_col = 0;
+            float nx_w = 0.0f;
+            load_tile(e0 + RW + gl, nx_col, nx_w);
+            for (int j = 0; j < most; j += STEP) {
+                int c[EU];
+                float w[EU];
 #pragma unroll
-            for (int u = 0; u < EU; ++u) {
-                c[u] = __shfl_sync(FULL, my_col, j + u * EPI + sub, RW);
-                w[u] = __shfl_sync(FULL, my_w, j + u * EPI + sub, RW);  // 0 behind the last edge
-            }
-            float v[EU][NV][VEC];
+                for (int u = 0; u < EU; ++u) {
+                    c[u] = __shfl_sync(FULL, my_col, j + u * EPI + sub, RW);
+                    w[u] = __shfl_sync(FULL, my_w, j + u * EPI + sub, RW);  // 0 behind the last edge
+                }
+                float v[EU][NV][VEC];
 #pragma unroll
-            for (int u = 0; u < EU; ++u) {
-                const bool live = j + u * EPI + sub < n;
+                for (int u = 0; u < EU; ++u) {
+                    const bool live = j + u * EPI + sub < n;
 #pragma unroll
-                for (int i = 0; i < NV; ++i) {
-                    if (live && valid[i]) {
-                        if constexpr (IDX32)
-                            load_vec<VEC>(v[u][i], p.x + (static_cast<uint32_t>(c[u]) * static_cast<uint32_t>(p.xs) + static_cast<uint32_t>(off[i])));
-                        else
-                            load_vec<VEC>(v[u][i], p.x + static_cast<int64_t>(c[u]) * p.xs + off[i]);
-                    } else {
+                    for (int i = 0; i < NV; ++i) {
+                        if (live && valid[i]) {
+                            if constexpr (SMALL)
+                                load_vec<VEC>(v[u][i], p.x + (static_cast<uint32_t>(c[u]) * static_cast<uint32_t>(p.xs) + static_cast<uint32_t>(off[i])));
+                            else
+                                load_vec<VEC>(v[u][i], p.x + static_cast<int64_t>(c[u]) * p.xs + off[i]);
+                        } else {
 #pragma unroll
-                        for (int q = 0; q < VEC; ++q) v[u][i][q] = 0.0f;
+                            for (int q = 0; q < VEC; ++q) v[u][i][q] = 0.0f;
+                        }
                     }
                 }
+#pragma unroll
+                for (int u = 0; u < EU; ++u)
+#pragma unroll
+                    for (int i = 0; i < NV; ++i)
+#pragma unroll
+                        for (int q = 0; q < VEC; ++q) acc[i][q] = fmaf(w[u], v[u][i][q], acc[i][q]);
             }
-#pragma unroll
-            for (int u = 0; u < EU; ++u)
-#pragma unroll
-                for (int i = 0; i < NV; ++i)
-#pragma unroll
-                    for (int q = 0; q < VEC; ++q) acc[i][q] = fmaf(w[u], v[u][i][q], acc[i][q]);
+            my_col = nx_col;
+            my_w = nx_w;
         }
-        my_col = nx_col;
-        my_w = nx_w;
+        if constexpr (SMALL) break;
+        const bool more = !raw && len == p.piece;
+        if (RW == 32 ? !more : !__any_sync(FULL, more)) break;
+        eb += len;
+        ids += len;
+        len = more ? static_cast<uint32_t>(min(load_ptr(p.indptr, p.is64, row + 1) - eb, static_cast<int64_t>(p.piece))) : 0;
     }
     // reduce-scatter over the sub-groups (fixed order: deterministic); piece = floats of a slice that this lane ends up with
     constexpr int PIECE = (VEC >= EPI) ? VEC / EPI : 1;
@@ -333,7 +346,7 @@ __global__ void __launch_bounds__(128, CTAS) spmm_group_kernel(const __grid_cons
     if (!owner || !store) return;
     float *dst = raw ? p.scratch + gid * p.D : p.out + row * p.os;
     // a hub row's chunk is left unscaled, but fully weighted; a row without edges is 0 whatever its factor
-    const bool node = p.wmode == YITU_W_NODE && len > 0;
+    const bool node = p.wmode == YITU_W_NODE && !empty;
     float s = raw ? 1.0f : p.alpha * (p.row_scale ? __ldg(p.row_scale + row) : 1.0f);
     if (node) s *= __ldg(p.norm_dst + row);
 #pragma unroll
@@ -645,7 +658,8 @@ static int launch_stream(const SpmmParams &p, cudaStream_t st) {  // always foll
 // Development switches read from the environment at every call (measurement of one kernel form against another):
 // YITU_SPMM_STREAM=0 keeps the group kernel for every graph, =2 takes the edge-stream kernel for every graph
 // whose shape it covers (default 1: by the rule in yitu_spmm_csr_f32); YITU_SPMM_STREAM_ROWS=8|16|31 and
-// YITU_SPMM_STREAM_EU pick an instantiation of the edge-stream kernel other than the default.
+// YITU_SPMM_STREAM_EU pick an instantiation of the edge-stream kernel other than the default; YITU_SPMM_PIECE=<multiple of 32> is the
+// length of the pieces in which the group kernel walks a row (default 2^31).
 static int env_int(const char *name, int dflt) {
     const char *v = getenv(name);
     return (v && *v) ? atoi(v) : dflt;
@@ -675,7 +689,10 @@ static int launch_group(const SpmmParams &p, cudaStream_t st, bool reduce = true
     YITU_REQUIRE(gx < (1ll << 31) && gy <= 65535, YITU_ERR_LIMIT, "spmm grid too large (%lld x %lld)",
                  (long long)gx, (long long)gy);
     dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
-    if (p.n_cols * p.xs < (1ll << 32)) spmm_group_kernel<RW, LPE, NV, VEC, EU, true, CTAS><<<grid, threads, 0, st>>>(p);
+    // a row's edges are bounded by the graph's, or by the schedule that cuts it
+    const bool small = p.n_cols * p.xs < (1ll << 32) &&
+                       (p.n_chunks > 0 ? p.chunk_edges < p.piece : p.nnz < p.piece);
+    if (small) spmm_group_kernel<RW, LPE, NV, VEC, EU, true, CTAS><<<grid, threads, 0, st>>>(p);
     else spmm_group_kernel<RW, LPE, NV, VEC, EU, false, CTAS><<<grid, threads, 0, st>>>(p);
     YITU_LAUNCH_CHECK();
     return reduce ? launch_hub_reduce(p, st) : YITU_OK;
@@ -752,7 +769,7 @@ extern "C" int yitu_spmm_csr_f32(const yitu_spmm_args_t *a, yitu_stream_t stream
         YITU_REQUIRE(g.nnz < (1ll << 31), YITU_ERR_LIMIT, "per-head edge values need nnz < 2^31");
 
     SpmmParams p{};
-    p.n_rows = g.n_rows; p.n_cols = g.n_cols; p.D = D; p.H = a->n_heads; p.F = a->n_feats;
+    p.n_rows = g.n_rows; p.n_cols = g.n_cols; p.nnz = g.nnz; p.D = D; p.H = a->n_heads; p.F = a->n_feats;
     p.indptr = g.indptr; p.indices = g.indices; p.is64 = g.indptr_is64; p.mask = g.index_mask;
     p.wmode = a->weight_mode; p.accumulate = a->accumulate;
     p.values = a->edge_values; p.perm = a->edge_perm;
@@ -760,6 +777,8 @@ extern "C" int yitu_spmm_csr_f32(const yitu_spmm_args_t *a, yitu_stream_t stream
     p.x = a->x; p.xs = a->x_stride; p.out = a->out; p.os = a->out_stride;
     p.bias = a->bias; p.act = a->activation; p.xshared = a->x_shared_heads ? 1 : 0;
     p.row_tasks = g.n_rows;
+    p.piece = static_cast<uint32_t>(env_int("YITU_SPMM_PIECE", 0));
+    if (p.piece == 0) p.piece = 1u << 31;
     if (a->plan && a->plan->n_chunks > 0) {
         YITU_REQUIRE(a->plan->chunk_edges >= 32, YITU_ERR_INVALID_ARG, "plan.chunk_edges must be >= 32");
         YITU_REQUIRE(a->plan->chunk_row && a->plan->chunk_begin, YITU_ERR_INVALID_ARG, "plan tables are NULL");
