@@ -624,3 +624,33 @@ def test_fused_gat_backward_of_unused_sources_is_zero(H, F, head_mean):
     for a, b in zip(got, want):
         assert torch.equal(a, b)
     assert float(got[1][0::3].abs().max()) == 0.0 and float(got[2][0::3].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("H,F", [(2, 8), (8, 32), (5, 40)])
+def test_backward_of_an_empty_graph_takes_null_inputs(H, F):
+    """The C interface lets x and key be NULL for a graph without edges; every gradient is zero."""
+    import ctypes as C
+    from yitu_b200 import ops
+    from yitu_b200._lib import GatBwdArgs, SpmmBwdArgs, check, lib
+    n_dst, n_src = 9, 70
+    ptr = lambda t: C.c_void_p(t.data_ptr())
+    indptr, t_indptr = torch.zeros(n_dst + 1, dtype=torch.int32, device="cuda"), torch.zeros(n_src + 1, dtype=torch.int32, device="cuda")
+    g = ops.PreparedGraph(indptr, torch.zeros(0, dtype=torch.int32, device="cuda"), n_src)
+    heads, rows = torch.ones(n_dst, H, device="cuda"), torch.ones(n_dst, H, F, device="cuda")
+    out = [torch.full(s, 7.0, device="cuda") for s in ((n_dst, H), (n_src, H), (n_src, H, F))]
+    b = GatBwdArgs()
+    b.fwd.graph, b.fwd.n_heads, b.fwd.n_feats, b.fwd.slope = g.csr, H, F, 0.2
+    b.fwd.query, b.fwd.out, b.fwd.row_max, b.fwd.row_sum = ptr(heads), ptr(rows), ptr(heads), ptr(heads)
+    b.grad_out, b.t_indptr = ptr(rows), ptr(t_indptr)
+    b.grad_query, b.grad_key, b.grad_x = (ptr(t) for t in out)
+    nbytes = lib().yitu_gat_bwd_scratch_bytes(n_dst, 0, 0, H, F)
+    scratch = torch.empty(nbytes // 4, device="cuda")
+    b.scratch, b.scratch_bytes = ptr(scratch), nbytes
+    check(lib().yitu_gat_bwd_f32(C.byref(b), ops._stream(indptr.device)))
+    assert all(float(t.abs().max()) == 0.0 for t in out)
+    if ops.spmm_bwd_supported(H, F):
+        a = SpmmBwdArgs()
+        a.graph, a.n_heads, a.n_feats = g.csr, H, F
+        a.t_indptr, a.grad_x = ptr(t_indptr), ptr(out[2].fill_(7.0))
+        check(lib().yitu_spmm_bwd_f32(C.byref(a), ops._stream(indptr.device)))
+        assert float(out[2].abs().max()) == 0.0

@@ -1511,6 +1511,14 @@ extern "C" int yitu_gat_bwd_f32(const yitu_gat_bwd_args_t *b, yitu_stream_t stre
     float *q_partial = rowpack + up256f(g.n_rows * H * 4);
     float *k_partial = q_partial + up256f(p.n_chunks * H);
     float *x_partial = k_partial + up256f(t_chunks * H);
+    if (g.nnz == 0) {  // x and key may be NULL then, which the kernels below read whether a source has edges or not
+        if (g.n_rows > 0) YITU_CUDA(cudaMemsetAsync(b->grad_query, 0, g.n_rows * H * sizeof(float), st));
+        if (g.n_cols > 0) {
+            YITU_CUDA(cudaMemsetAsync(b->grad_key, 0, g.n_cols * H * sizeof(float), st));
+            YITU_CUDA(cudaMemsetAsync(b->grad_x, 0, g.n_cols * D * sizeof(float), st));
+        }
+        return YITU_OK;
+    }
     const int64_t lph = F / 4;
     // lanes per head: a power of two, or any number when a row is one slice per lane
     const bool one_pass = lph <= 32 && ((lph & (lph - 1)) == 0 || D <= 128) && aligned16(a->x) && aligned16(out_heads);
@@ -1617,6 +1625,10 @@ extern "C" int yitu_spmm_bwd_f32(const yitu_spmm_bwd_args_t *a, yitu_stream_t st
     sp.g_scale = 1.0f; sp.grad_x = a->grad_x; sp.n_chunks = t_chunks; sp.x_partial = a->scratch;
     sp.values = a->edge_values; sp.grad_values = a->grad_values;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    if (g.nnz == 0) {  // x may be NULL then
+        YITU_CUDA(cudaMemsetAsync(a->grad_x, 0, g.n_cols * D * sizeof(float), st));
+        return YITU_OK;
+    }
     if (int rc = launch_src<true>(sp, st)) return rc;
     const HubRows h{a->t_indptr, g.indptr_is64, sp.chunk_edges, t_chunks, sp.chunk_row, sp.chunk_begin};
     return launch_chunk_sum(h, D, a->scratch, a->grad_x, st);
