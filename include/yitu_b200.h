@@ -327,7 +327,8 @@ typedef struct yitu_gat_bwd_args_t {
     float *grad_query;         /* [n_rows,H] */
     float *grad_key;           /* [n_cols,H] */
     float *grad_x;             /* [n_cols,H,F] */
-    float *edge_attn;          /* scratch [nnz,H]; needed only when F/4 is not a power of two <= 32 (may be NULL otherwise) */
+    float *edge_attn;          /* scratch [nnz,H]; may be NULL where the one-pass form applies: F <= 128, F/4 a power of two or
+                                  H*F <= 128, and fwd.out_heads (with head_mean) 16-byte aligned */
     float *edge_grad;          /* scratch [nnz,H]: the score gradient per edge, in CSR order */
     const yitu_hub_plan_t *t_plan; /* optional hub-row schedule of the transposed graph (fwd.plan is that of the graph) */
     float *scratch;            /* yitu_gat_bwd_scratch_bytes(n_rows, fwd.plan chunks or 0, t_plan chunks or 0, H, F) */

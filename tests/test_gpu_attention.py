@@ -654,3 +654,25 @@ def test_backward_of_an_empty_graph_takes_null_inputs(H, F):
         a.t_indptr, a.grad_x = ptr(t_indptr), ptr(out[2].fill_(7.0))
         check(lib().yitu_spmm_bwd_f32(C.byref(a), ops._stream(indptr.device)))
         assert float(out[2].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("H,F", [(2, 12), (2, 8), (8, 32), (3, 48)])
+def test_fused_gat_backward_takes_misaligned_head_results(H, F):
+    """out_heads is only read in the backward pass: a copy of it at any address will do."""
+    from yitu_b200 import ops
+    n = 60
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(H + F)
+    degs = torch.arange(n, device="cuda") % 7
+    indptr = torch.zeros(n + 1, dtype=torch.int32, device="cuda")
+    indptr[1:] = degs.cumsum(0).to(torch.int32)
+    indices = torch.randint(0, n, (int(degs.sum()),), device="cuda", generator=gen).to(torch.int32)
+    g = ops.PreparedGraph(indptr, indices, n)
+    q, k = (torch.randn(n, H, device="cuda", generator=gen) for _ in range(2))
+    x, grad = torch.randn(n, H, F, device="cuda", generator=gen), torch.randn(n, F, device="cuda", generator=gen)
+    out, row_max, row_sum, heads = ops.gat_fwd(g, q, k, x, head_mean=True)
+    want = ops.gat_bwd(g, q, k, x, out, row_max, row_sum, grad, head_mean=True, out_heads=heads)
+    moved = torch.empty(heads.numel() + 1, device="cuda")[1:].view_as(heads).copy_(heads)
+    got = ops.gat_bwd(g, q, k, x, out, row_max, row_sum, grad, head_mean=True, out_heads=moved)
+    for a, b in zip(got, want):
+        assert_close(a.cpu().numpy(), b.cpu().numpy(), rtol=3e-5, what="misaligned %dx%d" % (H, F))

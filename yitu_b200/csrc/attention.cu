@@ -806,6 +806,7 @@ struct GatBwdParams {
     const void *indptr;
     const int *indices;
     int is64, H, F, hshift;
+    int vec;  // out_heads is 16-byte aligned (the upstream gradient always is)
     float slope;
     const float *q, *k, *out_heads, *row_max, *row_sum;
     const float *g;  // upstream gradient: [n_rows,H,F], or [n_rows,F] shared by the heads (g_shared), times g_scale
@@ -851,7 +852,7 @@ __global__ void __launch_bounds__(256, 5) gat_bwd_score_kernel(const __grid_cons
     }
     // Dv[h] = <grad_out[row,h,:], out[row,h,:]>
     const int LPH = F >> 2;
-    if ((F & 3) == 0 && LPH <= 32 && (LPH & (LPH - 1)) == 0 && D <= 512) {
+    if (p.vec && (F & 3) == 0 && LPH <= 32 && (LPH & (LPH - 1)) == 0 && D <= 512) {
         // 128-bit slices, all requested before the first use; a head's lanes are adjacent: butterfly inside the head
         float d[4];
 #pragma unroll
@@ -1398,6 +1399,7 @@ extern "C" int yitu_gat_fwd_f32(const yitu_gat_args_t *a, yitu_stream_t stream) 
     if (a->graph.n_rows == 0) return YITU_OK;
     GatParams p{};
     fill_gat(p, a);
+    YITU_REQUIRE(aligned16(p.out_heads), YITU_ERR_INVALID_ARG, "out_heads must be 16-byte aligned");
     if (int rc = fill_plan(a->plan, &p.n_chunks, &p.chunk_edges, &p.chunk_row, &p.chunk_begin)) return rc;
     const int64_t D = a->n_heads * a->n_feats;
     if (p.n_chunks > 0) {
@@ -1563,7 +1565,7 @@ extern "C" int yitu_gat_bwd_f32(const yitu_gat_bwd_args_t *b, yitu_stream_t stre
         p.n_rows = g.n_rows; p.indptr = g.indptr; p.indices = g.indices; p.is64 = g.indptr_is64;
         p.H = static_cast<int>(H); p.F = static_cast<int>(F);
         p.hshift = (p.H & (p.H - 1)) == 0 ? 31 - __builtin_clz(p.H) : -1;
-        p.slope = a->slope; p.q = a->query; p.k = a->key; p.out_heads = out_heads;
+        p.slope = a->slope; p.q = a->query; p.k = a->key; p.out_heads = out_heads; p.vec = aligned16(out_heads);
         p.row_max = a->row_max; p.row_sum = a->row_sum;
         p.g = b->grad_out; p.g_shared = shared; p.g_scale = gscale;
         p.edge_attn = b->edge_attn; p.edge_grad = b->edge_grad; p.grad_q = b->grad_query;

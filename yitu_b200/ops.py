@@ -541,7 +541,8 @@ def gat_bwd(graph, query, key, x, out, row_max, row_sum, grad_out, slope=0.2, he
     grad_k = torch.empty_like(key)
     grad_x = torch.empty_like(x)
     lph = F // 4
-    one_pass = lph <= 32 and ((lph & (lph - 1)) == 0 or H * F <= 128)
+    one_pass = (lph <= 32 and ((lph & (lph - 1)) == 0 or H * F <= 128) and
+                (not head_mean or out_heads.data_ptr() % 16 == 0))  # yitu_gat_bwd_f32's own condition
     edge_attn = None if one_pass else torch.empty((graph.nnz, H), dtype=torch.float32, device=dev)
     edge_grad = torch.empty((graph.nnz, H), dtype=torch.float32, device=dev)
     b.grad_out = _ptr(grad_out)
