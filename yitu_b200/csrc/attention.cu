@@ -1443,15 +1443,20 @@ static int launch_src_as(const GatSrcParams &p, cudaStream_t st) {
     const int groups_per_cta = 128 / RW;
     const unsigned grid = static_cast<unsigned>((p.n_cols + p.n_chunks + groups_per_cta - 1) / groups_per_cta);
     // the butterfly over the lanes of a head is unrolled for the wide loads; the others (heads of four floats, misaligned
-    // tensors) branch over its steps
-    switch (VEC == 8 ? p.F / VEC : 0) {
-        case 1: gat_bwd_src_kernel<RW, LPE, NV, VEC, EU, GIVEN, 1, MINB><<<grid, 128, 0, st>>>(p); break;
-        case 2: if constexpr (VEC == 8 && LPE >= 2) gat_bwd_src_kernel<RW, LPE, NV, VEC, EU, GIVEN, 2, MINB><<<grid, 128, 0, st>>>(p); break;
-        case 4: if constexpr (VEC == 8 && LPE >= 4) gat_bwd_src_kernel<RW, LPE, NV, VEC, EU, GIVEN, 4, MINB><<<grid, 128, 0, st>>>(p); break;
-        case 8: if constexpr (VEC == 8 && LPE >= 8) gat_bwd_src_kernel<RW, LPE, NV, VEC, EU, GIVEN, 8, MINB><<<grid, 128, 0, st>>>(p); break;
-        case 16: if constexpr (VEC == 8 && LPE >= 16) gat_bwd_src_kernel<RW, LPE, NV, VEC, EU, GIVEN, 16, MINB><<<grid, 128, 0, st>>>(p); break;
-        case 32: if constexpr (VEC == 8 && LPE >= 32) gat_bwd_src_kernel<RW, LPE, NV, VEC, EU, GIVEN, 32, MINB><<<grid, 128, 0, st>>>(p); break;
-        default: gat_bwd_src_kernel<RW, LPE, NV, VEC, EU, GIVEN, 0, MINB><<<grid, 128, 0, st>>>(p); break;
+    // tensors) branch over its steps.  A head is at most 128 floats wide, and its lanes fit those of a row; a number of them
+    // that is no power of two comes with rows of 24 to 128 floats only, and not with GIVEN values.
+    const auto run = [&](auto lph) { gat_bwd_src_kernel<RW, LPE, NV, VEC, EU, GIVEN, decltype(lph)::value, MINB><<<grid, 128, 0, st>>>(p); };
+    if constexpr (VEC == 4) {
+        run(std::integral_constant<int, 0>{});
+    } else {
+        switch (p.F / VEC) {
+            case 1: run(std::integral_constant<int, 1>{}); break;
+            case 2: if constexpr (LPE >= 2) run(std::integral_constant<int, 2>{}); break;
+            case 4: if constexpr (LPE >= 4) run(std::integral_constant<int, 4>{}); break;
+            case 8: if constexpr (LPE >= 8) run(std::integral_constant<int, 8>{}); break;
+            case 16: if constexpr (LPE >= 16) run(std::integral_constant<int, 16>{}); break;
+            default: if constexpr (!GIVEN && LPE >= 4 && LPE < 32) run(std::integral_constant<int, 0>{}); break;
+        }
     }
     YITU_LAUNCH_CHECK();
     return YITU_OK;
