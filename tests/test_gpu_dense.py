@@ -195,3 +195,18 @@ def test_linear_is_seen_by_tracers_and_dispatch_modes():
     with FlopCounterMode(display=False) as counter:
         lin(x)
     assert counter.get_total_flops() == 2 * 50 * 24 * 12
+
+
+@pytest.mark.parametrize("M,N", [(4, 64), (8, 64), (16, 16), (64, 12), (40, 64)])
+def test_column_sums_are_rounded_once_per_split(M, N):
+    """Columns that cancel.  Rounded are the splits' sums and the result, each by 2^-24 * 0.58 of its size (rms), and the sizes
+    are those of random walks of n steps in all: 2^-24 * 0.58 * sqrt(2 n), where a chain over a split's 128 threads adds four
+    times that."""
+    from yitu_b200 import ops
+    n, err = 100003, []
+    for seed in range(8):
+        gen = torch.Generator(device="cuda")
+        gen.manual_seed(seed)
+        g, x = torch.randn(n, M, device="cuda", generator=gen), torch.randn(n, N, device="cuda", generator=gen)
+        err.append(ops.gram(g, x, sums=True)[1].double() - g.double().sum(0))
+    assert float(torch.stack(err).square().mean().sqrt()) <= 1.5 * 2.0 ** -24 * 0.58 * (2 * n) ** 0.5

@@ -335,9 +335,10 @@ __global__ void __launch_bounds__(256, 2) gram_kernel(const __grid_constant__ Gr
         __syncthreads();
         const int at = (p.sum_of == 2 ? b0 : a0) + tid, width = p.sum_of == 2 ? p.N : p.M;
         if (tid < sw && at < width) {
-            float v = 0.0f;
+            // up to 128 threads' sums: a plain chain over them would give away what the compensation has kept
+            double v = 0.0;
             for (int r = 0; r < sum_step; ++r) v += smem[r * sw + tid];
-            part[static_cast<int64_t>(p.M) * p.N + at] = v;
+            part[static_cast<int64_t>(p.M) * p.N + at] = static_cast<float>(v);
         }
         __syncthreads();
     }
@@ -371,14 +372,15 @@ __global__ void __launch_bounds__(256, 2) gram_kernel(const __grid_constant__ Gr
     }
 }
 
-// out = sum of the splits' partial results, in order: 32 results per CTA, eight threads share a result's splits
+// out = sum of the splits' partial results, in order and in 64 bits (up to 296 of them, which may nearly cancel: a bias
+// gradient): 32 results per CTA, eight threads share a result's splits
 __global__ void __launch_bounds__(256)
 gram_reduce_kernel(const float *partial, int64_t pstride, int splits, int M, int N, int sums, float *out, int64_t sa,
                    int64_t sb, float *colsum) {
-    __shared__ float s[8][33];
+    __shared__ double s[8][33];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t e = static_cast<int64_t>(blockIdx.x) * 32 + lane, total = static_cast<int64_t>(M) * N + sums;
-    float v = 0.0f;
+    double v = 0.0;
     if (e < total) {
 #pragma unroll 8
         for (int k = w; k < splits; k += 8) v += partial[k * pstride + e];
@@ -388,8 +390,8 @@ gram_reduce_kernel(const float *partial, int64_t pstride, int splits, int M, int
     if (w != 0 || e >= total) return;
 #pragma unroll
     for (int k = 1; k < 8; ++k) v += s[k][lane];
-    if (e < static_cast<int64_t>(M) * N) out[(e / N) * sa + (e % N) * sb] = v;
-    else colsum[e - static_cast<int64_t>(M) * N] = v;
+    if (e < static_cast<int64_t>(M) * N) out[(e / N) * sa + (e % N) * sb] = static_cast<float>(v);
+    else colsum[e - static_cast<int64_t>(M) * N] = static_cast<float>(v);
 }
 
 struct GramTile {
