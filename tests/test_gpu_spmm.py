@@ -96,7 +96,7 @@ STREAM_PATTERNS = {
 
 
 @pytest.mark.parametrize("pattern", sorted(STREAM_PATTERNS))
-@pytest.mark.parametrize("D", [96, 128, 136, 256])
+@pytest.mark.parametrize("D", [68, 96, 100, 128, 136, 256])
 def test_stream_kernel_row_patterns(oracle, monkeypatch, pattern, D):
     """The edge-stream SpMM (warp = batch of consecutive rows walked as one edge stream) on row patterns that put
     every bookkeeping branch to work: empty rows anywhere in a batch, rows ending on tile / group borders, hub rows
@@ -138,17 +138,25 @@ def test_stream_kernel_row_patterns(oracle, monkeypatch, pattern, D):
             out = _dev(base).clone()
             ops.spmm(g, _dev(x), out=out, accumulate=True, bias=_dev(bias), activation="relu", chunk_edges=chunk)
             assert_close(out.cpu().numpy(), ref_acc_epi, what=tag + " accumulate+epilogue")
-    # the default dispatch: hub chunks on the warp-per-row kernel, every other row on the edge-stream kernel
-    monkeypatch.setenv("YITU_SPMM_STREAM", "1")
+    # the split form of huge power-law graphs (hub chunks on the group kernel, every other row on the edge-stream kernel, one
+    # reduction) and, with 1, whatever the dispatch takes for so few rows
     monkeypatch.delenv("YITU_SPMM_STREAM_ROWS", raising=False)
     monkeypatch.delenv("YITU_SPMM_STREAM_EU", raising=False)
-    g = ops.PreparedGraph(_dev(indptr, torch.int64), _dev(indices), n_cols)
-    got = ops.spmm(g, _dev(x), mode=ops.W_NODE, norm_dst=_dev(nd), norm_src=_dev(ns), chunk_edges=chunk)
-    assert_close(got.cpu().numpy(), ref_node, what="split %s D=%d node" % (pattern, D))
-    out = _dev(base).clone()
-    ops.spmm(g, _dev(x), out=out, accumulate=True, bias=_dev(bias), activation="relu", chunk_edges=chunk)
-    assert_close(out.cpu().numpy(), ref_acc_epi, what="split %s D=%d accumulate+epilogue" % (pattern, D))
-    # the warp-per-row kernel on the same inputs gives the same sums up to the order of the additions
+    for form in ("3", "1"):
+        monkeypatch.setenv("YITU_SPMM_STREAM", form)
+        tag = "%s %s D=%d" % ("split" if form == "3" else "default", pattern, D)
+        g = ops.PreparedGraph(_dev(indptr, torch.int64), _dev(indices), n_cols)
+        got = ops.spmm(g, _dev(x), mode=ops.W_EDGE, edge_values=_dev(vals), chunk_edges=chunk)
+        assert_close(got.cpu().numpy(), ref_edge, what=tag + " edge")
+        got = ops.spmm(g, _dev(x), mode=ops.W_NODE, norm_dst=_dev(nd), norm_src=_dev(ns), chunk_edges=chunk)
+        assert_close(got.cpu().numpy(), ref_node, what=tag + " node")
+        out = _dev(base).clone()
+        ops.spmm(g, _dev(x), out=out, accumulate=True, alpha=0.5, chunk_edges=chunk)
+        assert_close(out.cpu().numpy(), ref_acc, what=tag + " accumulate")
+        out = _dev(base).clone()
+        ops.spmm(g, _dev(x), out=out, accumulate=True, bias=_dev(bias), activation="relu", chunk_edges=chunk)
+        assert_close(out.cpu().numpy(), ref_acc_epi, what=tag + " accumulate+epilogue")
+    # the group kernel on the same inputs gives the same sums up to the order of the additions
     monkeypatch.setenv("YITU_SPMM_STREAM", "0")
     g = ops.PreparedGraph(_dev(indptr, torch.int32), _dev(indices), n_cols)
     got = ops.spmm(g, _dev(x), mode=ops.W_EDGE, edge_values=_dev(vals), chunk_edges=chunk)

@@ -657,7 +657,8 @@ static int launch_stream(const SpmmParams &p, cudaStream_t st) {  // always foll
 
 // Development switches read from the environment at every call (measurement of one kernel form against another):
 // YITU_SPMM_STREAM=0 keeps the group kernel for every graph, =2 takes the edge-stream kernel for every graph
-// whose shape it covers (default 1: by the rule in yitu_spmm_csr_f32); YITU_SPMM_STREAM_ROWS=8|16|31 and
+// whose shape it covers, =3 the same with the hub rows' chunks on the group kernel (default 1: by the rule in
+// yitu_spmm_csr_f32); YITU_SPMM_STREAM_ROWS=8|16|31 and
 // YITU_SPMM_STREAM_EU pick an instantiation of the edge-stream kernel other than the default; YITU_SPMM_PIECE=<multiple of 32> is the
 // length of the pieces in which the group kernel walks a row (default 2^31).
 static int env_int(const char *name, int dflt) {
@@ -818,15 +819,16 @@ extern "C" int yitu_spmm_csr_f32(const yitu_spmm_args_t *a, yitu_stream_t stream
     // chunks go to the group kernel (a whole warp per chunk, two edges per load) and only the other rows are streamed: R-MAT
     // with 128 floats (ms, group alone / stream alone / both) 16.8 M rows x 31 edges 35.7 / 36.6 / 34.3, 8 M x 8 5.52 / - /
     // 5.23, 4 M x 15 3.93 / 4.16 / 3.87; below 2 M rows the group kernel alone.
-    // YITU_SPMM_STREAM (development switch): 0 never, 2 for everything the kernel covers, 1 (default) by this rule.
+    // YITU_SPMM_STREAM (development switch): 0 never, 2 for everything the kernel covers, chunks included, 3 for all rows that
+    // are not cut into chunks, 1 (default) by this rule.
     const int stream_mode = env_int("YITU_SPMM_STREAM", 1);
     const bool stream_shape = g.nnz < (1ll << 31) && D > 64 && (D <= 128 || (D <= 256 && vec8_ok));
-    const bool use_stream = stream_shape && (stream_mode == 2 || (stream_mode == 1 && (p.n_chunks > 0
+    const bool use_stream = stream_shape && (stream_mode >= 2 || (stream_mode == 1 && (p.n_chunks > 0
                             ? D <= 128 && g.n_rows >= (2 << 20) && g.nnz < 64 * g.n_rows
                             : g.n_rows >= 150000 && g.nnz < 24 * g.n_rows && !(vec8_ok && D <= 128 && g.nnz < 8 * g.n_rows))));
     if (use_stream) {
         SpmmParams r = p;
-        if (p.n_chunks > 0 && stream_mode == 1) {
+        if (p.n_chunks > 0 && stream_mode != 2) {
             SpmmParams c = p;
             c.row_tasks = 0;  // the chunks only; the reduction follows the second launch
             if (int rc = vec8_ok ? launch_group<32, 16, 1, 8, 8>(c, st, false) : dispatch_group4(c, st, false)) return rc;
