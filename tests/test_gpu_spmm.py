@@ -512,3 +512,20 @@ def test_long_rows_in_pieces(oracle, monkeypatch, D):
         monkeypatch.delenv("YITU_SPMM_PIECE")
         assert torch.equal(got, whole)
         assert_close(got.cpu().numpy(), oracle.spmm(indptr, indices, x, wmode=oracle.W_EDGE, values=vals), what="pieces D=%d" % D)
+
+
+def test_plan_of_no_argument():
+    """plan() is the schedule of chunks of 512 edges, and all that the operators need to be captured without a call before."""
+    from yitu_b200 import ops
+    n, deg = 300, 600
+    indptr = torch.arange(0, (n + 1) * deg, deg, dtype=torch.int32, device="cuda")
+    indices = torch.randint(0, n, (n * deg,), device="cuda").to(torch.int32)
+    x = torch.randn(n, 32, device="cuda")
+    want = ops.spmm(ops.PreparedGraph(indptr, indices, n), x)
+    g = ops.PreparedGraph(indptr, indices, n)
+    assert g.chunk_edges() < 512 and g.plan()[0].chunk_edges == 512 and g.plan()[0].n_chunks == 2 * n
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = ops.spmm(g, x)
+    graph.replay()
+    assert torch.equal(out, want)

@@ -133,10 +133,14 @@ class PreparedGraph:
         return min(max(1 << (share.bit_length() - 1), MIN_CHUNK_EDGES), DEFAULT_CHUNK_EDGES)
 
     # hub-row schedule ---------------------------------------------------------------------------
-    def plan(self, chunk_edges=OWN_CHUNKS):
-        """(HubPlan struct, its two tables, pointer to the struct), or None for a graph without hub rows."""
+    def plan(self, chunk_edges=DEFAULT_CHUNK_EDGES):
+        """(HubPlan struct, its two tables, pointer to the struct), or None for a graph without hub rows.  The default has the
+        fewest partial sums (the limit of yitu_spmm_csr_f32_static); the operators' own schedule is built with it, so that a
+        program that calls plan() ahead of a stream capture has both."""
         if chunk_edges == OWN_CHUNKS:
             chunk_edges = self.chunk_edges()
+        elif chunk_edges == DEFAULT_CHUNK_EDGES and self.chunk_edges() != DEFAULT_CHUNK_EDGES:
+            self.plan(self.chunk_edges())
         if chunk_edges in self._plans:
             return self._plans[chunk_edges]
         L = lib()
