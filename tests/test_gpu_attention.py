@@ -676,3 +676,22 @@ def test_fused_gat_backward_takes_misaligned_head_results(H, F):
     got = ops.gat_bwd(g, q, k, x, out, row_max, row_sum, grad, head_mean=True, out_heads=moved)
     for a, b in zip(got, want):
         assert_close(a.cpu().numpy(), b.cpu().numpy(), rtol=3e-5, what="misaligned %dx%d" % (H, F))
+
+
+@pytest.mark.parametrize("H", [1, 2, 4, 8, 16])
+def test_per_source_sums_are_rounded_in_pairs(H):
+    """yitu_edge_gather_sum_f32 over columns of 64 normal values.  The rounding error of a sum, rms in units of 2^-24 * 0.58, is the
+    root of its partial sums' variances added up: 46 for one chain of 64 additions, 22 for eight groups of eight added in
+    pairs, less where several lanes share a column.  The bound lies at 24."""
+    from yitu_b200 import ops
+    from yitu_b200._lib import check, lib
+    n, deg = 20000, 64
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(H)
+    vals = torch.randn(n * deg, H, device="cuda", generator=gen)
+    indptr = torch.arange(0, n * deg + 1, deg, dtype=torch.int32, device="cuda")
+    out = torch.empty(n, H, device="cuda")
+    check(lib().yitu_edge_gather_sum_f32(n, ops._ptr(indptr), 0, None, H, ops._ptr(vals), ops._ptr(out), None, ops._stream(vals.device)))
+    ref = vals.view(n, deg, H).double().sum(1)
+    rms = float((out.double() - ref).square().mean().sqrt())
+    assert rms <= 2.0 ** -24 * 0.58 * 24

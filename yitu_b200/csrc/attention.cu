@@ -352,8 +352,8 @@ __global__ void __launch_bounds__(128) edge_gather_sum_kernel(const __grid_const
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) v[u] = (at[u] >= 0 && h < H) ? __ldg(p.vals + at[u] * H + h) : 0.0f;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) a += v[u];
+            // in pairs: a column is no long chain of roundings (a bias gradient behind it may cancel to a thousandth)
+            a += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
         }
         for (int o = HB; o < RW; o <<= 1) a += __shfl_xor_sync(FULL, a, o, RW);
         if (dst && slot == 0 && h < H) dst[h] = a;
@@ -1093,9 +1093,15 @@ __global__ void __launch_bounds__(128, MINB) gat_bwd_src_kernel(const __grid_con
             const bool live = FULL || j + u * EPI + sub < n;
 #pragma unroll
             for (int i = 0; i < NV; ++i) {
-                float dp = 0.0f;
+                float part[VEC / 4];  // chains of four: fewer roundings (and waits) than one of eight
 #pragma unroll
-                for (int v = 0; v < VEC; ++v) dp = fmaf(gv[u][i][v], xr[i][v], dp);
+                for (int t = 0; t < VEC / 4; ++t) {
+                    part[t] = 0.0f;
+#pragma unroll
+                    for (int v = 4 * t; v < 4 * t + 4; ++v) part[t] = fmaf(gv[u][i][v], xr[i][v], part[t]);
+                }
+                float dp = part[0];
+                if constexpr (VEC == 8) dp += part[1];
                 if (LPH_T || pow2) {
 #pragma unroll
                     for (int o = LPE >> 1; o > 0; o >>= 1)
