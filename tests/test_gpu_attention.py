@@ -695,3 +695,44 @@ def test_per_source_sums_are_rounded_in_pairs(H):
     ref = vals.view(n, deg, H).double().sum(1)
     rms = float((out.double() - ref).square().mean().sqrt())
     assert rms <= 2.0 ** -24 * 0.58 * 24
+
+
+@pytest.mark.parametrize("chunk", [0, 32, 100, 512, 600])
+@pytest.mark.parametrize("B,H", [(1, 1), (1, 4), (1, 8), (1, 40), (2, 4), (3, 2), (4, 8), (5, 16), (9, 1)])
+def test_edge_softmax_row_lengths(B, H, chunk):
+    """Rows around every border of the stand-alone softmax: one, two and four edges per slot, held and walked rows, and rows
+    just below and above the length from which a CTA takes them, whatever the schedule's chunks."""
+    from yitu_b200 import ops
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(B * 100 + H)
+    n_src = 500
+    degs = torch.tensor([0, 1, 2, 3, 7, 8, 9, 15, 16, 17, 31, 32, 33, 63, 64, 65, 0, 127, 128, 129, 255, 256, 257, 5, 511, 512, 513, 300, 258,
+                         599, 600, 601, 1025, 0, 4], device="cuda")
+    n = degs.numel()
+    indptr = torch.zeros(n + 1, dtype=torch.int32, device="cuda")
+    indptr[1:] = degs.cumsum(0).to(torch.int32)
+    rows = torch.repeat_interleave(torch.arange(n, device="cuda"), degs)
+    cols = torch.randint(0, n_src, (rows.numel(),), device="cuda", generator=gen)
+    seg = (torch.arange(rows.numel(), device="cuda") - indptr[:-1].long()[rows]) * B // degs[rows]
+    stitched = cols | (seg << 24)
+    stitched = torch.where(stitched >= 2 ** 31, stitched - 2 ** 32, stitched).to(torch.int32)
+    g = ops.PreparedGraph(indptr, stitched, n_src, 0xFFFFFF if B > 1 else 0)
+    q, k = torch.randn(B, n, H, device="cuda", generator=gen), torch.randn(n_src, H, device="cuda", generator=gen)
+    score = q.double()[seg, rows] + k.double()[cols]
+    z = torch.nn.functional.leaky_relu(score, 0.2)
+    part = rows * B + seg
+    top = torch.full((n * B, H), -float("inf"), dtype=torch.float64, device="cuda").scatter_reduce(0, part[:, None].expand(-1, H), z, "amax")
+    e = torch.exp(z - top[part])
+    total = torch.zeros(n * B, H, dtype=torch.float64, device="cuda").index_add_(0, part, e)
+    want = e / total[part]
+    attn = ops.edge_softmax_fwd(g, q, k, chunk_edges=chunk)
+    assert_close(attn.cpu().numpy(), want.cpu().numpy(), what="edge-softmax B=%d H=%d chunk=%d" % (B, H, chunk))
+    a32, grad = want.float(), torch.randn(rows.numel(), H, device="cuda", generator=gen)
+    a, ga = a32.double(), grad.double()
+    t = torch.zeros(n * B, H, dtype=torch.float64, device="cuda").index_add_(0, part, a * ga)
+    ds = a * (ga - t[part]) * torch.where(score.float() < 0, 0.2, 1.0)
+    ref_q = torch.zeros(n * B, H, dtype=torch.float64, device="cuda").index_add_(0, part, ds).view(n, B, H).transpose(0, 1)
+    ref_k = torch.zeros(n_src, H, dtype=torch.float64, device="cuda").index_add_(0, cols, ds)
+    gq, gk = ops.edge_softmax_bwd(g, q, k, a32, grad, chunk_edges=chunk)
+    assert_close(gq.cpu().numpy(), ref_q.cpu().numpy(), rtol=2e-5, what="edge-softmax-grad-query B=%d H=%d" % (B, H))
+    assert_close(gk.cpu().numpy(), ref_k.cpu().numpy(), rtol=2e-5, what="edge-softmax-grad-key B=%d H=%d" % (B, H))

@@ -15,6 +15,7 @@
 // All of them are bound by gather bandwidth (HBM/L2); none uses float atomics.
 #include <math_constants.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -43,10 +44,15 @@ __device__ __forceinline__ float4 load_now(const float4 *p) {
 
 // ---------------------------------------------------------------------------------------------------------
 // Stand-alone edge softmax.  A lane is (edge slot, head): HB = pow2 >= min(H,32) lanes span the heads (coalesced key / attn
-// accesses).  A warp owns a row; a hub row gets a CTA of 512 threads.  A row of up to four edges per slot is held in
-// registers: ids, segments and scores are read once, all in flight together, whatever the number of segments.  Longer rows
-// are walked four edges per slot at a time, for four segments at once.  (One edge at a time, once per segment and pass, a row was a chain of gathers: the
-// hub rows of 2.4 M edges x 4 heads in 3 segments took 368 us forward and 416 us backward.)
+// accesses).  A warp owns a row; a row of more than HUB_EDGES edges gets a CTA of 512 threads.  A row of up to four edges per
+// slot is held in registers: ids, segments and scores are read once, all in flight together, whatever the number of segments.
+// Longer rows are walked four edges per slot at a time, for SEGS segments at once (1, 2 or 4, by their number: a plain graph
+// does not compute the sums of three segments it has not).  (One edge at a time, once per segment and pass, a row was a chain
+// of gathers: the hub rows of 2.4 M edges x 4 heads in 3 segments took 368 us forward and 416 us backward.)
+//   NARROW: a step is no wider than the edges left ask for.  On a plain graph of even rows the empty positions of four-wide steps
+// cost more than the gathers in flight gain (us, forward / backward, one edge at a time | always four | NARROW: 100 k rows x 33
+// edges x 4 heads 86 / 117 | 134 / 185 | 85 / 123, 300 k x 16 166 / 246 | 173 / 315 | 157 / 219, R-MAT 500 k x 32 1148 / 1713 |
+// 854 / 1374 | 604 / 977); with several segments the forward is better without (100 k x 100 in three: 371, NARROW 545).
 // ---------------------------------------------------------------------------------------------------------
 struct SoftmaxParams {
     int64_t n_rows;
@@ -56,25 +62,39 @@ struct SoftmaxParams {
     float slope;
     const float *q, *k, *attn_in, *grad_attn;
     float *attn_out, *grad_q, *edge_grad;
-    // optional hub schedule: rows longer than chunk_edges are left to the CTA-per-row variants below
+    // optional hub schedule: rows longer than hub_edges are left to the CTA-per-row variants below, one CTA per cta_chunks
+    // consecutive chunks
     int64_t n_chunks;
-    int chunk_edges;
+    int chunk_edges, hub_edges, cta_chunks;
     const int *chunk_row;
     const int64_t *chunk_begin;
 };
 
 constexpr int HUB_THREADS = 512;
-constexpr int SEGS = 4;  // segments whose sums a long row forms in one walk
+// Rows from which on a CTA is taken: 256 edges, and twice the average row, so that a graph whose rows are all long keeps a
+// warp for each.  (One B200, us, forward / backward with 4 heads, every row of the chunk schedule, 64 edges and more | 256 and
+// more: uniform 10 k rows x 70 edges 102 / 166 | 34 / 65, R-MAT 100 k x 24 133 / 249 | 131 / 242, with 1024 157 / 314; uniform
+// 4 k x 500 109 / 237 | 82 / 154, with 1024 78 / 127.)
+constexpr int HUB_EDGES = 256;
 
 // Row assignment shared by the stand-alone kernels.  CTA = false: one warp per row, hub rows skipped when a schedule
-// is given.  CTA = true: one CTA per hub row (launched with one CTA per chunk; the CTAs of a row's later
-// chunks leave at once), its edge slots advancing together.
+// is given.  CTA = true: one CTA per hub row, its edge slots advancing together; a CTA looks at cta_chunks consecutive chunks, and
+// at most one hub row begins there: it is longer than hub_edges >= cta_chunks * chunk_edges.
 template <bool CTA>
 __device__ __forceinline__ bool softmax_row(const SoftmaxParams &p, int64_t &row, int64_t &eb, int64_t &ee) {
     if constexpr (CTA) {
-        row = __ldg(p.chunk_row + blockIdx.x);
+        __shared__ int64_t s_chunk;
+        if (threadIdx.x == 0) s_chunk = -1;
+        __syncthreads();
+        const int64_t first = static_cast<int64_t>(blockIdx.x) * p.cta_chunks, last = min(first + p.cta_chunks, p.n_chunks);
+        for (int64_t c = first + threadIdx.x; c < last; c += blockDim.x) {
+            const int64_t r = __ldg(p.chunk_row + c), b = load_ptr(p.indptr, p.is64, r);
+            if (__ldg(p.chunk_begin + c) == b && load_ptr(p.indptr, p.is64, r + 1) - b > p.hub_edges) s_chunk = c;
+        }
+        __syncthreads();
+        if (s_chunk < 0) return false;
+        row = __ldg(p.chunk_row + s_chunk);
         eb = load_ptr(p.indptr, p.is64, row);
-        if (__ldg(p.chunk_begin + blockIdx.x) != eb) return false;
         ee = load_ptr(p.indptr, p.is64, row + 1);
         return true;
     } else {
@@ -82,7 +102,7 @@ __device__ __forceinline__ bool softmax_row(const SoftmaxParams &p, int64_t &row
         if (row >= p.n_rows) return false;
         eb = load_ptr(p.indptr, p.is64, row);
         ee = load_ptr(p.indptr, p.is64, row + 1);
-        return !(p.n_chunks > 0 && ee - eb > p.chunk_edges);
+        return !(p.n_chunks > 0 && ee - eb > p.hub_edges);
     }
 }
 
@@ -103,24 +123,54 @@ __device__ __forceinline__ float slot_reduce(float v, int HB, float *s_red) {
     return v;
 }
 
-// Four edges of a slot: position, segment (-1: none) and column.
-struct Edges4 {
-    int seg[4], col[4];
-    __device__ __forceinline__ void load(const SoftmaxParams &p, int64_t e0, int64_t ee, int ES) {
-        int raw[4];
+// U edges of a slot (`left` of them and of the other slots' up to there are edges of the row): segment (-1: none) and column.
+template <int U>
+struct Edges {
+    int seg[U], col[U];
+    __device__ __forceinline__ void load(const SoftmaxParams &p, int64_t at, int left, int ES) {
+        int raw[U];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) raw[u] = e0 + u * ES < ee ? __ldg(p.indices + e0 + u * ES) : 0;
+        for (int u = 0; u < U; ++u) raw[u] = u * ES < left ? __ldg(p.indices + at + u * ES) : 0;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            seg[u] = e0 + u * ES < ee ? (p.mask ? static_cast<int>(static_cast<unsigned>(raw[u]) >> 24) : 0) : -1;
+        for (int u = 0; u < U; ++u) {
+            seg[u] = u * ES < left ? (p.mask ? static_cast<int>(static_cast<unsigned>(raw[u]) >> 24) : 0) : -1;
             if (seg[u] >= p.B) seg[u] = -1;  // edges of segments without a query take no part
             col[u] = p.mask ? (raw[u] & p.mask) : raw[u];
         }
     }
 };
+template <int U>
+using Width = std::integral_constant<int, U>;
 
-template <bool CTA>
-__global__ void __launch_bounds__(CTA ? HUB_THREADS : 256) edge_softmax_fwd_kernel(const __grid_constant__ SoftmaxParams p) {
+// step(width, first edge of this slot, edges from there) over a row: four edges per slot at a time; NARROW: what is left of the
+// row in one step that is no wider than it has to be
+template <bool NARROW, typename Step>
+__device__ __forceinline__ void walk_row(int64_t eb, int64_t ee, int slot, int ES, Step step) {
+    if constexpr (NARROW) {
+        int64_t b = eb;
+        for (; ee - b >= 4 * ES; b += 4 * ES) step(Width<4>{}, b + slot, 4 * ES - slot);
+        const int left = static_cast<int>(ee - b);
+        if (left > 2 * ES) step(Width<4>{}, b + slot, left - slot);
+        else if (left > ES) step(Width<2>{}, b + slot, left - slot);
+        else if (left > 0) step(Width<1>{}, b + slot, left - slot);
+    } else {
+        for (int64_t b = eb; b < ee; b += 4 * ES) step(Width<4>{}, b + slot, static_cast<int>(min(ee - b, static_cast<int64_t>(4 * ES))) - slot);
+    }
+}
+// held(width): a row that fits the registers, NARROW: as narrow as it allows
+template <bool NARROW, typename Held>
+__device__ __forceinline__ void hold_row(int len, int ES, Held held) {
+    if (!NARROW || len > 2 * ES) {
+        held(Width<4>{});
+    } else if constexpr (NARROW) {
+        if (len > ES) held(Width<2>{});
+        else held(Width<1>{});
+    }
+}
+
+template <bool CTA, int SEGS>
+__global__ void __launch_bounds__(CTA ? HUB_THREADS : 256, CTA ? 2 : 5) edge_softmax_fwd_kernel(const __grid_constant__ SoftmaxParams p) {
+    constexpr bool NARROW = !CTA && SEGS == 1;
     __shared__ float s_red[CTA ? HUB_THREADS : 1];
     int64_t row, eb, ee;
     if (!softmax_row<CTA>(p, row, eb, ee)) return;
@@ -128,69 +178,74 @@ __global__ void __launch_bounds__(CTA ? HUB_THREADS : 256) edge_softmax_fwd_kern
     const int hs = lane & (p.HB - 1);
     const int slot = (CTA ? threadIdx.x : lane) >> pow2_shift(p.HB);
     const int ES = (CTA ? HUB_THREADS : 32) / p.HB;
-    const bool held = ee - eb <= 4 * ES;
     for (int hc = 0; hc < p.H; hc += p.HB) {
         const int h = hc + hs;
         const bool hv = h < p.H;
         const auto query = [&](int s) { return __ldg(p.q + (static_cast<int64_t>(s) * p.n_rows + row) * p.H + h); };
-        const auto scores = [&](const Edges4 &e, int first, int last, float (&z)[4]) {  // of the edges in segments [first, last)
+        const auto scores = [&](const auto &e, int first, int last, auto &z) {  // of the edges in segments [first, last)
+            constexpr int U = std::extent<std::remove_reference_t<decltype(z)>>::value;
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                z[u] = (hv && e.seg[u] >= first && e.seg[u] < last) ? __ldg(p.k + static_cast<int64_t>(e.col[u]) * p.H + h) : -CUDART_INF_F;
+            for (int u = 0; u < U; ++u)
+                z[u] = (hv && e.seg[u] >= first && e.seg[u] < last) ? __ldg(row_at(p.k + h, e.col[u], static_cast<uint32_t>(p.H) * 4u)) : -CUDART_INF_F;
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (int u = 0; u < U; ++u)
                 if (hv && e.seg[u] >= first && e.seg[u] < last) z[u] = leaky_relu(query(e.seg[u]) + z[u], p.slope);
         };
-        if (held) {
-            Edges4 e;
-            e.load(p, eb + slot, ee, ES);
-            float z[4];
-            scores(e, 0, p.B, z);
-            for (int s = 0; s < p.B; ++s) {
-                float m = -CUDART_INF_F, l = 0.0f;
+        if (ee - eb <= 4 * ES) {
+            hold_row<NARROW>(static_cast<int>(ee - eb), ES, [&](auto width) {
+                constexpr int U = decltype(width)::value;
+                Edges<U> e;
+                e.load(p, eb + slot, static_cast<int>(ee - eb) - slot, ES);
+                float z[U];
+                scores(e, 0, p.B, z);
+                for (int s = 0; s < p.B; ++s) {
+                    float m = -CUDART_INF_F, l = 0.0f;
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (e.seg[u] == s) m = fmaxf(m, z[u]);
-                m = slot_reduce<CTA, true>(m, p.HB, s_red);
-                float w[4];
+                    for (int u = 0; u < U; ++u)
+                        if (e.seg[u] == s) m = fmaxf(m, z[u]);
+                    m = slot_reduce<CTA, true>(m, p.HB, s_red);
+                    float w[U];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    w[u] = e.seg[u] == s ? expf(z[u] - m) : 0.0f;
-                    l += w[u];
+                    for (int u = 0; u < U; ++u) {
+                        w[u] = e.seg[u] == s ? expf(z[u] - m) : 0.0f;
+                        l += w[u];
+                    }
+                    l = slot_reduce<CTA, false>(l, p.HB, s_red);
+                    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        if (hv && e.seg[u] == s) p.attn_out[(eb + slot) * p.H + h + u * ES * p.H] = w[u] * inv;
                 }
-                l = slot_reduce<CTA, false>(l, p.HB, s_red);
-                const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (hv && e.seg[u] == s) p.attn_out[(eb + slot + u * ES) * p.H + h] = w[u] * inv;
-            }
+            });
             continue;
         }
         for (int s0 = 0; s0 < p.B; s0 += SEGS) {
-            float m[SEGS], l[SEGS], z[4];
+            float m[SEGS], l[SEGS];
 #pragma unroll
             for (int s = 0; s < SEGS; ++s) {
                 m[s] = -CUDART_INF_F;
                 l[s] = 0.0f;
             }
-            Edges4 e;
-            for (int64_t e0 = eb + slot; e0 < ee; e0 += 4 * ES) {
-                e.load(p, e0, ee, ES);
+            walk_row<NARROW>(eb, ee, slot, ES, [&](auto width, int64_t at, int left) {
+                constexpr int U = decltype(width)::value;
+                Edges<U> e;
+                e.load(p, at, left, ES);
+                float z[U];
                 scores(e, s0, s0 + SEGS, z);
 #pragma unroll
                 for (int s = 0; s < SEGS; ++s) {
                     float top = m[s];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
+                    for (int u = 0; u < U; ++u)
                         if (e.seg[u] == s0 + s) top = fmaxf(top, z[u]);
                     const float ref = top > -CUDART_INF_F ? top : 0.0f;
                     if (top > m[s]) l[s] *= expf(m[s] - ref);
                     m[s] = top;
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
+                    for (int u = 0; u < U; ++u)
                         if (e.seg[u] == s0 + s) l[s] += expf(z[u] - ref);
                 }
-            }
+            });
             float inv[SEGS];
 #pragma unroll
             for (int s = 0; s < SEGS; ++s) {
@@ -201,21 +256,25 @@ __global__ void __launch_bounds__(CTA ? HUB_THREADS : 256) edge_softmax_fwd_kern
                 m[s] = top;
                 inv[s] = l[s] > 0.0f ? 1.0f / l[s] : 0.0f;
             }
-            for (int64_t e0 = eb + slot; e0 < ee; e0 += 4 * ES) {
-                e.load(p, e0, ee, ES);
+            walk_row<NARROW>(eb, ee, slot, ES, [&](auto width, int64_t at, int left) {
+                constexpr int U = decltype(width)::value;
+                Edges<U> e;
+                e.load(p, at, left, ES);
+                float z[U];
                 scores(e, s0, s0 + SEGS, z);
 #pragma unroll
                 for (int s = 0; s < SEGS; ++s)
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (hv && e.seg[u] == s0 + s) p.attn_out[(e0 + u * ES) * p.H + h] = expf(z[u] - m[s]) * inv[s];
-            }
+                    for (int u = 0; u < U; ++u)
+                        if (hv && e.seg[u] == s0 + s) p.attn_out[at * p.H + h + u * ES * p.H] = expf(z[u] - m[s]) * inv[s];
+            });
         }
     }
 }
 
-template <bool CTA>
-__global__ void __launch_bounds__(CTA ? HUB_THREADS : 256, CTA ? 2 : 4) edge_softmax_bwd_kernel(const __grid_constant__ SoftmaxParams p) {
+template <bool CTA, int SEGS>
+__global__ void __launch_bounds__(CTA ? HUB_THREADS : 256, CTA ? 2 : SEGS == 1 ? 6 : 4) edge_softmax_bwd_kernel(const __grid_constant__ SoftmaxParams p) {
+    constexpr bool NARROW = !CTA;
     __shared__ float s_red[CTA ? HUB_THREADS : 1];
     int64_t row, eb, ee;
     if (!softmax_row<CTA>(p, row, eb, ee)) return;
@@ -223,81 +282,106 @@ __global__ void __launch_bounds__(CTA ? HUB_THREADS : 256, CTA ? 2 : 4) edge_sof
     const int hs = lane & (p.HB - 1);
     const int slot = (CTA ? threadIdx.x : lane) >> pow2_shift(p.HB);
     const int ES = (CTA ? HUB_THREADS : 32) / p.HB;
-    const bool held = ee - eb <= 4 * ES;
     for (int hc = 0; hc < p.H; hc += p.HB) {
         const int h = hc + hs;
         const bool hv = h < p.H;
         const auto query = [&](int s) { return __ldg(p.q + (static_cast<int64_t>(s) * p.n_rows + row) * p.H + h); };
-        // attention, its gradient and the sign of the score of four edges, those in segments [first, last)
-        const auto values = [&](const Edges4 &e, int64_t e0, int first, int last, float (&a)[4], float (&g)[4], bool (&neg)[4], bool score) {
-            float kv[4];
+        // attention and its gradient of the edges in segments [first, last)
+        const auto weights = [&](const auto &e, int64_t at, int first, int last, auto &a, auto &g) {
+            constexpr int U = std::extent<std::remove_reference_t<decltype(a)>>::value;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < U; ++u) {
                 const bool on = hv && e.seg[u] >= first && e.seg[u] < last;
-                a[u] = on ? __ldg(p.attn_in + (e0 + u * ES) * p.H + h) : 0.0f;
-                g[u] = on ? __ldg(p.grad_attn + (e0 + u * ES) * p.H + h) : 0.0f;
-                kv[u] = on && score ? __ldg(p.k + static_cast<int64_t>(e.col[u]) * p.H + h) : 0.0f;
+                a[u] = on ? __ldg(p.attn_in + at * p.H + h + u * ES * p.H) : 0.0f;
+                g[u] = on ? __ldg(p.grad_attn + at * p.H + h + u * ES * p.H) : 0.0f;
             }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                neg[u] = score && hv && e.seg[u] >= first && e.seg[u] < last && query(e.seg[u]) + kv[u] < 0.0f;
         };
-        float a[4], g[4];
-        bool neg[4];
-        Edges4 e;
-        if (held) {
-            e.load(p, eb + slot, ee, ES);
-            values(e, eb + slot, 0, p.B, a, g, neg, true);
-        }
-        for (int s0 = 0; s0 < p.B; s0 += SEGS) {
-            float t[SEGS], gq[SEGS];  // per segment: sum of attn * grad, sum of the score gradients
+        // whether their scores are negative
+        const auto signs = [&](const auto &e, int first, int last, auto &neg) {
+            constexpr int U = std::extent<std::remove_reference_t<decltype(neg)>>::value;
+            float kv[U];
 #pragma unroll
-            for (int s = 0; s < SEGS; ++s) t[s] = gq[s] = 0.0f;
-            const auto weigh = [&]() {
+            for (int u = 0; u < U; ++u)
+                kv[u] = hv && e.seg[u] >= first && e.seg[u] < last ? __ldg(row_at(p.k + h, e.col[u], static_cast<uint32_t>(p.H) * 4u)) : 0.0f;
 #pragma unroll
-                for (int s = 0; s < SEGS; ++s)
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (e.seg[u] == s0 + s) t[s] = fmaf(a[u], g[u], t[s]);
-            };
-            const auto finish = [&](int64_t e0) {
-#pragma unroll
-                for (int s = 0; s < SEGS; ++s)
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (hv && e.seg[u] == s0 + s) {
-                            const float gs = a[u] * (g[u] - t[s]), gv = gs * (neg[u] ? p.slope : 1.0f);
-                            p.edge_grad[(e0 + u * ES) * p.H + h] = gv;
-                            gq[s] += gv;
-                        }
-            };
-            if (held) {
-                weigh();
-            } else {
-                for (int64_t e0 = eb + slot; e0 < ee; e0 += 4 * ES) {
-                    e.load(p, e0, ee, ES);
-                    values(e, e0, s0, s0 + SEGS, a, g, neg, false);
-                    weigh();
-                }
-            }
+            for (int u = 0; u < U; ++u)
+                neg[u] = hv && e.seg[u] >= first && e.seg[u] < last && query(e.seg[u]) + kv[u] < 0.0f;
+        };
+        // per segment s0, s0 + 1, ...: t = sum of attn * grad, gq = sum of the score gradients
+        const auto weigh = [&](const auto &e, int s0, const auto &a, const auto &g, float (&t)[SEGS]) {
+            constexpr int U = std::extent<std::remove_reference_t<decltype(a)>>::value;
 #pragma unroll
             for (int s = 0; s < SEGS; ++s)
-                if (s0 + s < p.B) t[s] = slot_reduce<CTA, false>(t[s], p.HB, s_red);
-            if (held) {
-                finish(eb + slot);
-            } else {
-                for (int64_t e0 = eb + slot; e0 < ee; e0 += 4 * ES) {
-                    e.load(p, e0, ee, ES);
-                    values(e, e0, s0, s0 + SEGS, a, g, neg, true);
-                    finish(e0);
-                }
-            }
 #pragma unroll
-            for (int s = 0; s < SEGS; ++s) {
-                if (s0 + s >= p.B) break;
-                gq[s] = slot_reduce<CTA, false>(gq[s], p.HB, s_red);
-                if (slot == 0 && hv) p.grad_q[(static_cast<int64_t>(s0 + s) * p.n_rows + row) * p.H + h] = gq[s];
-            }
+                for (int u = 0; u < U; ++u)
+                    if (e.seg[u] == s0 + s) t[s] = fmaf(a[u], g[u], t[s]);
+        };
+        const auto finish = [&](const auto &e, int64_t at, int s0, const auto &a, const auto &g, const auto &neg, const float (&t)[SEGS],
+                                float (&gq)[SEGS]) {
+            constexpr int U = std::extent<std::remove_reference_t<decltype(a)>>::value;
+#pragma unroll
+            for (int s = 0; s < SEGS; ++s)
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (hv && e.seg[u] == s0 + s) {
+                        const float gs = a[u] * (g[u] - t[s]), gv = gs * (neg[u] ? p.slope : 1.0f);
+                        p.edge_grad[at * p.H + h + u * ES * p.H] = gv;
+                        gq[s] += gv;
+                    }
+        };
+        const auto total = [&](int s0, float (&v)[SEGS]) {
+#pragma unroll
+            for (int s = 0; s < SEGS; ++s)
+                if (s0 + s < p.B) v[s] = slot_reduce<CTA, false>(v[s], p.HB, s_red);
+        };
+        const auto store = [&](int s0, const float (&gq)[SEGS]) {
+#pragma unroll
+            for (int s = 0; s < SEGS; ++s)
+                if (s0 + s < p.B && slot == 0 && hv) p.grad_q[(static_cast<int64_t>(s0 + s) * p.n_rows + row) * p.H + h] = gq[s];
+        };
+        if (ee - eb <= 4 * ES) {
+            hold_row<NARROW>(static_cast<int>(ee - eb), ES, [&](auto width) {
+                constexpr int U = decltype(width)::value;
+                Edges<U> e;
+                e.load(p, eb + slot, static_cast<int>(ee - eb) - slot, ES);
+                float a[U], g[U];
+                bool neg[U];
+                weights(e, eb + slot, 0, p.B, a, g);
+                signs(e, 0, p.B, neg);
+                for (int s0 = 0; s0 < p.B; s0 += SEGS) {
+                    float t[SEGS] = {}, gq[SEGS] = {};
+                    weigh(e, s0, a, g, t);
+                    total(s0, t);
+                    finish(e, eb + slot, s0, a, g, neg, t, gq);
+                    total(s0, gq);
+                    store(s0, gq);
+                }
+            });
+            continue;
+        }
+        for (int s0 = 0; s0 < p.B; s0 += SEGS) {
+            float t[SEGS] = {}, gq[SEGS] = {};
+            walk_row<NARROW>(eb, ee, slot, ES, [&](auto width, int64_t at, int left) {
+                constexpr int U = decltype(width)::value;
+                Edges<U> e;
+                e.load(p, at, left, ES);
+                float a[U], g[U];
+                weights(e, at, s0, s0 + SEGS, a, g);
+                weigh(e, s0, a, g, t);
+            });
+            total(s0, t);
+            walk_row<NARROW>(eb, ee, slot, ES, [&](auto width, int64_t at, int left) {
+                constexpr int U = decltype(width)::value;
+                Edges<U> e;
+                e.load(p, at, left, ES);
+                float a[U], g[U];
+                bool neg[U];
+                weights(e, at, s0, s0 + SEGS, a, g);
+                signs(e, s0, s0 + SEGS, neg);
+                finish(e, at, s0, a, g, neg, t, gq);
+            });
+            total(s0, gq);
+            store(s0, gq);
         }
     }
 }
@@ -1218,6 +1302,30 @@ static int check_softmax_args(const yitu_csr_t *g, int32_t n_segments, int64_t H
     return YITU_OK;
 }
 
+template <bool BWD, int SEGS>
+static int launch_softmax_segs(const SoftmaxParams &p, cudaStream_t st) {
+    const unsigned grid = static_cast<unsigned>((p.n_rows + 7) / 8);
+    if constexpr (BWD) edge_softmax_bwd_kernel<false, SEGS><<<grid, 256, 0, st>>>(p);
+    else edge_softmax_fwd_kernel<false, SEGS><<<grid, 256, 0, st>>>(p);
+    YITU_LAUNCH_CHECK();
+    if (p.n_chunks == 0) return YITU_OK;
+    const unsigned hubs = static_cast<unsigned>((p.n_chunks + p.cta_chunks - 1) / p.cta_chunks);
+    if constexpr (BWD) edge_softmax_bwd_kernel<true, SEGS><<<hubs, HUB_THREADS, 0, st>>>(p);
+    else edge_softmax_fwd_kernel<true, SEGS><<<hubs, HUB_THREADS, 0, st>>>(p);
+    YITU_LAUNCH_CHECK();
+    return YITU_OK;
+}
+
+template <bool BWD>
+static int launch_softmax(SoftmaxParams &p, int64_t nnz, cudaStream_t st) {
+    const int64_t twice = 2 * (nnz / p.n_rows);
+    p.hub_edges = static_cast<int>(std::max<int64_t>({p.chunk_edges, HUB_EDGES, std::min<int64_t>(twice, INT32_MAX)}));
+    p.cta_chunks = p.n_chunks > 0 ? p.hub_edges / p.chunk_edges : 1;
+    if (p.B == 1) return launch_softmax_segs<BWD, 1>(p, st);
+    if (p.B == 2) return launch_softmax_segs<BWD, 2>(p, st);
+    return launch_softmax_segs<BWD, 4>(p, st);
+}
+
 extern "C" int yitu_edge_softmax_fwd_f32(const yitu_csr_t *g, int32_t n_segments, int64_t n_heads, float slope,
                                          const float *query, const float *key, float *attn,
                                          const yitu_hub_plan_t *plan, yitu_stream_t stream) {
@@ -1229,14 +1337,7 @@ extern "C" int yitu_edge_softmax_fwd_f32(const yitu_csr_t *g, int32_t n_segments
     p.mask = g->index_mask; p.B = n_segments; p.H = static_cast<int>(n_heads); p.HB = head_block(n_heads);
     p.slope = slope; p.q = query; p.k = key; p.attn_out = attn;
     if (int rc = fill_plan(plan, &p.n_chunks, &p.chunk_edges, &p.chunk_row, &p.chunk_begin)) return rc;
-    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    edge_softmax_fwd_kernel<false><<<static_cast<unsigned>((g->n_rows + 7) / 8), 256, 0, st>>>(p);
-    YITU_LAUNCH_CHECK();
-    if (p.n_chunks > 0) {  // hub rows: one CTA each
-        edge_softmax_fwd_kernel<true><<<static_cast<unsigned>(p.n_chunks), HUB_THREADS, 0, st>>>(p);
-        YITU_LAUNCH_CHECK();
-    }
-    return YITU_OK;
+    return launch_softmax<false>(p, g->nnz, reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" int yitu_edge_softmax_bwd_f32(const yitu_csr_t *g, int32_t n_segments, int64_t n_heads, float slope,
@@ -1253,14 +1354,7 @@ extern "C" int yitu_edge_softmax_bwd_f32(const yitu_csr_t *g, int32_t n_segments
     p.slope = slope; p.q = query; p.k = key; p.attn_in = attn; p.grad_attn = grad_attn;
     p.grad_q = grad_query; p.edge_grad = edge_grad;
     if (int rc = fill_plan(plan, &p.n_chunks, &p.chunk_edges, &p.chunk_row, &p.chunk_begin)) return rc;
-    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    edge_softmax_bwd_kernel<false><<<static_cast<unsigned>((g->n_rows + 7) / 8), 256, 0, st>>>(p);
-    YITU_LAUNCH_CHECK();
-    if (p.n_chunks > 0) {
-        edge_softmax_bwd_kernel<true><<<static_cast<unsigned>(p.n_chunks), HUB_THREADS, 0, st>>>(p);
-        YITU_LAUNCH_CHECK();
-    }
-    return YITU_OK;
+    return launch_softmax<true>(p, g->nnz, reinterpret_cast<cudaStream_t>(stream));
 }
 
 // partial: scratch of n_chunks * H floats for the hub columns' chunk sums, or NULL (a CTA per hub column)
@@ -1272,7 +1366,9 @@ static int gather_sum(int64_t n_cols, const void *t_indptr, int32_t indptr_is64,
     p.H = static_cast<int>(n_heads); p.HB = head_block(n_heads); p.vals = edge_vals; p.out = out;
     if (int rc = fill_plan(t_plan, &p.n_chunks, &p.chunk_edges, &p.chunk_row, &p.chunk_begin)) return rc;
     const int64_t n_parts = partial ? p.n_chunks : 0;
-    const int rw = p.HB < 8 ? 8 : p.HB;
+    // more lanes per column where the columns are too few to fill the chip (10 k columns x 70 edges, 8 heads, us: 16 with 8 lanes)
+    int rw = p.HB < 8 ? 8 : p.HB;
+    while (rw < 32 && n_cols * rw < 400000) rw *= 2;
     const unsigned grid = static_cast<unsigned>((n_cols + n_parts + 128 / rw - 1) / (128 / rw));
     if (rw == 8) edge_gather_sum_kernel<8><<<grid, 128, 0, st>>>(p, n_parts, partial);
     else if (rw == 16) edge_gather_sum_kernel<16><<<grid, 128, 0, st>>>(p, n_parts, partial);
