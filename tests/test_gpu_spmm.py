@@ -529,3 +529,16 @@ def test_plan_of_no_argument():
         out = ops.spmm(g, x)
     graph.replay()
     assert torch.equal(out, want)
+
+
+def test_an_explicit_chunk_length_builds_one_schedule():
+    """Only plan() builds the operators' own schedule along; a call that names its chunk length builds that one."""
+    from yitu_b200 import ops
+    n, deg = 300, 600
+    indptr = torch.arange(0, (n + 1) * deg, deg, dtype=torch.int32, device="cuda")
+    indices = torch.randint(0, n, (n * deg,), device="cuda").to(torch.int32)
+    x = torch.randn(n, 32, device="cuda")
+    for chunk in (64, 512):
+        g = ops.PreparedGraph(indptr, indices, n)
+        ops.spmm(g, x, chunk_edges=chunk)
+        assert list(g._plans) == [chunk]

@@ -137,12 +137,16 @@ class PreparedGraph:
         """(HubPlan struct, its two tables, pointer to the struct), or None for a graph without hub rows.  The default has the
         fewest partial sums (the limit of yitu_spmm_csr_f32_static); the operators' own schedule is built with it, so that a
         program that calls plan() ahead of a stream capture has both."""
-        if chunk_edges == OWN_CHUNKS:
-            chunk_edges = self.chunk_edges()
-        elif chunk_edges == DEFAULT_CHUNK_EDGES and self.chunk_edges() != DEFAULT_CHUNK_EDGES:
-            self.plan(self.chunk_edges())
+        if chunk_edges == DEFAULT_CHUNK_EDGES:
+            self._schedule(OWN_CHUNKS)
+        return self._schedule(chunk_edges)
+
+    def _schedule(self, chunk_edges):
         if chunk_edges in self._plans:
             return self._plans[chunk_edges]
+        if chunk_edges == OWN_CHUNKS:
+            self._plans[OWN_CHUNKS] = self._schedule(self.chunk_edges())
+            return self._plans[OWN_CHUNKS]
         L = lib()
         with torch.cuda.device(self.device):
             ws_bytes = L.yitu_hub_plan_workspace_bytes(self.n_rows)
@@ -266,7 +270,7 @@ def spmm(graph, x, *, n_heads=1, mode=W_NONE, edge_values=None, edge_perm=None, 
     plan = scratch = None
     scratch_floats = 0
     if chunk_edges:
-        pl = graph.plan(chunk_edges)
+        pl = graph._schedule(chunk_edges)
         if pl is not None:
             plan, scratch_floats = pl[3], pl[0].n_chunks * D
             scratch = x.new_empty(scratch_floats)
@@ -373,7 +377,7 @@ def _hub_plan(graph, chunk_edges):
     """(pointer to the HubPlan struct or None, number of chunks, objects to keep alive)."""
     if not chunk_edges:
         return None, 0, None
-    pl = graph.plan(chunk_edges)
+    pl = graph._schedule(chunk_edges)
     if pl is None:
         return None, 0, None
     return pl[3], pl[0].n_chunks, pl
