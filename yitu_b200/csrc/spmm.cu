@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(128, (VEC * EU <= 32) ? 6 : 4) spmm_stream_ker
                 const bool had = cur_end > cur_begin;
                 if (valid && (had || !p.accumulate || p.bias || p.act)) {
                     float s = p.alpha * (p.row_scale ? __ldg(p.row_scale + row) : 1.0f);
-                    if (p.wmode == YITU_W_NODE && had) s *= __ldg(p.norm_dst + row);
+                    if (p.wmode == YITU_W_NODE) s *= __ldg(p.norm_dst + row);
                     float *dst = p.out + row * p.os + off;
                     float r[VEC];
                     if (p.accumulate) {
