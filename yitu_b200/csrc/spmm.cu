@@ -30,7 +30,7 @@
 namespace yitu {
 
 struct SpmmParams {
-    int64_t n_rows, n_cols, nnz, D, H, F;
+    int64_t n_rows, n_cols, D, H, F;
     const void *indptr;
     const int *indices;
     int is64, mask, wmode, accumulate;
@@ -52,6 +52,7 @@ struct SpmmParams {
     const float *bias;
     int act, xshared;
     uint32_t piece;  // spmm_group_kernel without SMALL walks longer rows in pieces of this many edges
+    int64_t nnz;
 };
 
 // Last step of every output row: bias, then activation (both optional).
@@ -288,12 +289,14 @@ __global__ void __launch_bounds__(128, SMALL || CTAS < 16 ? CTAS : 12) spmm_grou
                 for (int u = 0; u < EU; ++u) {
                     const bool live = j + u * EPI + sub < n;
                     // one address per edge: the slices lie at constant distances from the lane's first
-                    const float *xr = SMALL ? p.x + (static_cast<uint32_t>(c[u]) * static_cast<uint32_t>(p.xs) + static_cast<uint32_t>(off[0]))
-                                            : p.x + static_cast<int64_t>(c[u]) * p.xs + off[0];
+                    const auto slice = [&](int i) {
+                        return (SMALL ? p.x + (static_cast<uint32_t>(c[u]) * static_cast<uint32_t>(p.xs) + static_cast<uint32_t>(off[0]))
+                                      : p.x + static_cast<int64_t>(c[u]) * p.xs + off[0]) + i * LPE * VEC;
+                    };
 #pragma unroll
                     for (int i = 0; i < NV; ++i) {
                         if (live && valid[i]) {
-                            load_vec<VEC>(v[u][i], xr + i * LPE * VEC);
+                            load_vec<VEC>(v[u][i], slice(i));
                         } else {
 #pragma unroll
                             for (int q = 0; q < VEC; ++q) v[u][i][q] = 0.0f;
