@@ -212,8 +212,8 @@ def test_group_kernel_dispatch_edges(oracle, monkeypatch, D, degrees):
 
 @pytest.mark.parametrize("D", [1, 4, 7, 8, 16, 20, 24, 32, 40, 41, 64, 100, 128, 200, 256, 260, 320])
 def test_rows_are_summed_in_the_order_they_are_stored(D):
-    """The order of a row's additions is fixed by its width alone (edge after edge; 33..64 floats in whole 32-byte slices: four
-    interleaved sums), so that the sign of a sum near zero does not depend on the graph around the row."""
+    """A row that is not cut into chunks is summed edge after edge, rows of 33..64 floats in whole 32-byte slices in four
+    interleaved sums.  (A schedule cuts longer rows by the graph's size, and sums their chunks apart.)"""
     from yitu_b200 import ops
     gen = torch.Generator(device="cuda")
     gen.manual_seed(D)
@@ -542,3 +542,25 @@ def test_an_explicit_chunk_length_builds_one_schedule():
         g = ops.PreparedGraph(indptr, indices, n)
         ops.spmm(g, x, chunk_edges=chunk)
         assert list(g._plans) == [chunk]
+
+
+@pytest.mark.parametrize("D", [1, 4, 8, 16, 20, 32, 41, 48, 50, 64, 72, 100, 101, 128, 200, 256])
+def test_few_long_rows(oracle, D):
+    """The deeper forms that graphs of few, evenly long rows take (64 edges per row on average), with and without chunks."""
+    from yitu_b200 import ops
+    rng = np.random.default_rng(D)
+    n_cols = 300
+    indptr, indices = _csr_from_degrees(rng, [64, 65, 95, 96, 97, 70, 0, 1, 128, 130, 200, 31, 33, 66], n_cols)
+    assert indices.size >= 64 * (indptr.size - 1)
+    x, vals = rng.standard_normal((n_cols, D)).astype(np.float32), rng.standard_normal(indices.shape[0]).astype(np.float32)
+    bias, base = rng.standard_normal(D).astype(np.float32), rng.standard_normal((indptr.size - 1, D)).astype(np.float32)
+    ref = oracle.spmm(indptr, indices, x, wmode=oracle.W_EDGE, values=vals)
+    ref_acc = np.maximum(oracle.spmm(indptr, indices, x, alpha=0.5, out=base) + bias, 0)
+    for dtype in (torch.int32, torch.int64):
+        g = ops.PreparedGraph(_dev(indptr, dtype), _dev(indices), n_cols)
+        for chunk in (0, 64, ops.OWN_CHUNKS):
+            got = ops.spmm(g, _dev(x), mode=ops.W_EDGE, edge_values=_dev(vals), chunk_edges=chunk)
+            assert_close(got.cpu().numpy(), ref, what="few-long-rows D=%d chunk=%s" % (D, chunk))
+            out = _dev(base).clone()
+            ops.spmm(g, _dev(x), out=out, accumulate=True, alpha=0.5, bias=_dev(bias), activation="relu", chunk_edges=chunk)
+            assert_close(out.cpu().numpy(), ref_acc, what="few-long-rows D=%d chunk=%s accumulate" % (D, chunk))

@@ -711,34 +711,45 @@ static int launch_group(const SpmmParams &p, cudaStream_t st, bool reduce = true
 // Rows of 33..64 floats are the exception to the narrow group: a warp per row, four edges per load, is as fast on uniform
 // graphs (660 us against 671) and faster on power-law ones, where the longest of a warp's rows holds up the others (R-MAT
 // 1 M x 15: 511 against 624).
-// Every row's edges are summed in the order the CSR stores them, rows of 33..64 floats in four interleaved sums: the order
-// does not depend on the graph's size, so a ReLU behind the sum sees the same signs whatever form is taken here.
+// Rows of up to 16 floats run unbounded up to half a million rows (100 k rows x 16 edges 16.5 us at 16 CTAs, 15.1 without; R-MAT
+// 16 k x 14 23 and 16; 1 M x 16 162 and 168).  Where all rows are long and too few to fill the chip twelve CTAs deep, a chain of one
+// or two gathers is what counts, and the deeper forms win (128 floats, us: 1 k rows x 100 edges in chunks of 64 18.1 and 10.3,
+// 10 k x 70 43.2 and 36.6, whole rows of 30 k x 400 406 and 341; but 100 k x 100 284 and 293.  64 floats, whole rows: 30 k x 400
+// 199 and 180; in chunks the shallow form is as good: 3 k x 100 13.1 and 14.6).
+// The edges of a row that is not cut into chunks are summed in the order the CSR stores them; 33..64 floats by 256-bit loads in
+// four interleaved sums.
+static bool few_long_rows(const SpmmParams &p) { return p.n_rows <= 65536 && p.nnz >= 64 * p.n_rows; }
 static int dispatch_group4(const SpmmParams &p, cudaStream_t st, bool reduce = true) {
-    if (p.D <= 16) return launch_group<4, 4, 1, 4, 4, 16>(p, st, reduce);
+    if (p.D <= 16) return p.n_rows <= 524288 ? launch_group<4, 4, 1, 4, 4>(p, st, reduce) : launch_group<4, 4, 1, 4, 4, 16>(p, st, reduce);
     if (p.D <= 32) return launch_group<8, 8, 1, 4, 4, 12>(p, st, reduce);
     if (p.D <= 64) return launch_group<16, 16, 1, 4, 8>(p, st, reduce);
+    if (p.D <= 128 && few_long_rows(p)) return launch_group<32, 32, 1, 4, 8>(p, st, reduce);
     if (p.D <= 128) return launch_group<32, 32, 1, 4, 2, 12>(p, st, reduce);
     if (p.D <= 256) return launch_group<32, 32, 2, 4, 8>(p, st, reduce);
     return launch_group<32, 32, 4, 4, 4>(p, st, reduce);
 }
 static int dispatch_group8(const SpmmParams &p, cudaStream_t st, bool reduce = true) {
-    if (p.D <= 32) return dispatch_group4(p, st, reduce);
+    if (p.D <= 32 || (p.D > 64 && p.D <= 128 && few_long_rows(p))) return dispatch_group4(p, st, reduce);
+    if (p.D <= 64 && p.n_chunks == 0 && few_long_rows(p)) return launch_group<32, 8, 1, 8, 2>(p, st, reduce);
     if (p.D <= 64) return launch_group<32, 8, 1, 8, 1, 16>(p, st, reduce);
     if (p.D <= 128) return launch_group<16, 16, 1, 8, 2, 12>(p, st, reduce);
     if (p.D <= 256) return launch_group<32, 32, 1, 8, 2>(p, st, reduce);
     return launch_group<32, 32, 2, 8, 4>(p, st, reduce);
 }
 // Widths that are no multiple of four, or rows that are not 16-byte aligned: scalar loads, NV of them per lane and edge
-// (41 floats, 170 k rows x 13 edges: 200 us with one warp and four masked slices per row, 120 us with 16 lanes x 3).
+// (41 floats, 170 k rows x 13 edges: 200 us with one warp and four masked slices per row, 120 us with 16 lanes x 3).  From 49
+// floats on four edges per step without a bound (us, two edges at 12 CTAs | four: 50 floats, 30 k x 100 79 | 66, 1 M x 16 733 |
+// 662; 101 floats 114 | 98 and 1323 | 1294); 33..48 up to half a million rows (41 floats, 100 k x 100 185 | 170, 1 M x 16 507 |
+// 555).  With an address per load instead of one per edge, 101 floats took 202 (30 k x 100).
 static int dispatch_group1(const SpmmParams &p, cudaStream_t st) {
     if (p.D <= 4) return launch_group<4, 4, 1, 1, 4, 16>(p, st);
     if (p.D <= 8) return launch_group<8, 8, 1, 1, 8, 16>(p, st);
     if (p.D <= 16) return launch_group<16, 16, 1, 1, 8, 12>(p, st);
     if (p.D <= 32) return launch_group<16, 16, 2, 1, 4, 12>(p, st);
-    if (p.D <= 48) return launch_group<16, 16, 3, 1, 2, 16>(p, st);
-    if (p.D <= 64) return launch_group<16, 16, 4, 1, 2, 12>(p, st);
-    if (p.D <= 96) return launch_group<32, 32, 3, 1, 2, 12>(p, st);
-    return launch_group<32, 32, 4, 1, 2, 12>(p, st);
+    if (p.D <= 48) return p.n_rows <= 524288 ? launch_group<16, 16, 3, 1, 4>(p, st) : launch_group<16, 16, 3, 1, 2, 16>(p, st);
+    if (p.D <= 64) return launch_group<16, 16, 4, 1, 4>(p, st);
+    if (p.D <= 96) return launch_group<32, 32, 3, 1, 4>(p, st);
+    return launch_group<32, 32, 4, 1, 4>(p, st);
 }
 
 }  // namespace yitu
