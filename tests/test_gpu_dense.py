@@ -229,3 +229,24 @@ def test_gram_counts_every_row_once(n, M, N, layout):
     for x, y in ((a, b), (b, a)):
         c, s = ops.gram(x, y, sums=True)
         assert torch.equal(c.double(), x.double().t() @ y.double()) and torch.equal(s.double(), x.double().sum(0))
+
+
+@pytest.mark.parametrize("n", [100, 511, 512, 1499, 1500, 2048, 4096, 4097])
+@pytest.mark.parametrize("K,N", [(32, 64), (33, 64), (64, 17), (65, 64), (128, 64), (128, 128), (129, 16), (129, 17), (256, 128), (256, 129),
+                                 (257, 16), (512, 16), (513, 8), (1024, 16), (1025, 8), (1433, 41), (64, 65), (8, 4096)])
+def test_products_at_the_borders_of_the_dispatch(n, K, N):
+    """Own kernel or library, with and without a bias: the same product within the rounding of a sum of its length."""
+    from yitu_b200 import ops
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n + K + N)
+    a, w, bias = (torch.randn(*s, device="cuda", generator=gen) for s in ((n, K), (N, K), (N,)))
+    exact, size = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+    for got, add in ((ops.matmul(a, w, b_transposed=True, bias=bias), bias), (ops.matmul(a, w, b_transposed=True), None),
+                     (ops.matmul(a, w.t().contiguous()), None)):
+        ref, scale = (exact, size) if add is None else (exact + add.double(), size + add.double().abs())
+        assert bool(((got.double() - ref).abs() <= _bound(K, scale)).all())
+    g = torch.randn(n, N, device="cuda", generator=gen)
+    for sums in (False, True):
+        c, s = ops.gram(g, a, sums=sums)
+        assert bool(((c.double() - g.double().t() @ a.double()).abs() <= _bound(n, g.double().abs().t() @ a.double().abs())).all())
+        assert s is None if not sums else bool(((s.double() - g.double().sum(0)).abs() <= _bound(n, g.double().abs().sum(0))).all())

@@ -128,7 +128,9 @@ class PreparedGraph:
         """Edges per chunk of this graph's hub rows.  A chunk is one serial task, so it has to be a small part of the
         whole pass: about nnz / 16000 edges, between 64 (below that the partial sums cost more than the tail) and 512
         (1024 is no faster on graphs of 60 to 520 M edges).  Measured against 512 for every graph: R-MAT 16 k nodes x
-        14 edges, 16 features 124 -> 26 us; 50 k x 18, 128 features 98 -> 69; 1 M x 8, 64 features 468 -> 409."""
+        14 edges, 16 features 124 -> 26 us; 50 k x 18, 128 features 98 -> 69; 1 M x 8, 64 features 468 -> 409.  Short
+        chunks are also the more exact sums: 1.7e-7 against 2.6e-7 with 512 for the gradients of a layer whose sources have 250
+        edges each.  (What they cost is a graph of evenly long rows: 10 k x 70, 128 features 26 us whole, 37 in two chunks.)"""
         share = max(self.nnz // 16000, 1)
         return min(max(1 << (share.bit_length() - 1), MIN_CHUNK_EDGES), DEFAULT_CHUNK_EDGES)
 
@@ -318,14 +320,33 @@ def _recorded(*tensors):
     return any(t is not None and t.requires_grad for t in tensors)
 
 
+def _linear_pays(n, K, N):
+    """Whether yitu_linear_f32 is the faster one for x W^T + b (figures: its time by the library's on one B200, launches of a CUDA
+    graph; the results are the same bits where the library does not split the sum).  The library adds the bias in a second
+    pass, which counts most for short sums: K <= 128 0.2 to 0.97 at 100 to 1 M rows.  Behind that its deeper tiles win back
+    what the pass costs, except for narrow results (N <= 16: 0.4 to 0.97 up to K = 512) and where the rows fill the chip (256
+    x 64: 0.88 at 50 k rows, 1.17 at 16 k, 0.88 at 4 k; 500 x 64: 0.95 at 170 k, 1.45 at 16 k); 1433 x 16 is 1.29 at 170 k
+    rows and 2.0 at 700."""
+    if K * N > 65536:
+        return False
+    if K <= 128:
+        return True
+    if K <= 256:
+        return N <= 16 or n >= 49152 or (n <= 4096 and N <= 128)
+    if N > 16:
+        return K <= 512 and n >= 131072
+    if K <= 1024:
+        return K <= 512 or n >= 4096
+    return N <= 8 and 2048 <= n < 131072
+
+
 def matmul(a, b, b_transposed=False, bias=None, out=None):
     """a b (+ bias), or a b^T (+ bias) with b_transposed, for a matrix a of many rows: yitu_linear_f32, or the library
     GEMM for other types and where it is the faster one.  Without a bias that is where both widths are large (60 k x
-    128 x 128: 59 us against 55; 20 k x 500 x 500: 256 against 205; 1 M x 64 x 64: 175 against 251); with one the
-    library adds it in a second pass (1 M x 64 x 64: 190 us against 540, 170 k x 128 x 256: 257 against 447, 20 k x 500
-    x 500: 274 against 267).  out: a matrix with contiguous rows that receives the result."""
+    128 x 128: 59 us against 55; 20 k x 500 x 500: 256 against 205; 1 M x 64 x 64: 175 against 251).  out: a matrix with
+    contiguous rows that receives the result."""
     K, N = a.size(-1), b.size(0 if b_transposed else -1)
-    own = min(K, N) <= 64 and max(K, N) <= 256 if bias is None else K * N <= 65536
+    own = min(K, N) <= 64 and max(K, N) <= 256 if bias is None else _linear_pays(a.size(0), K, N)
     if (not own or a.dim() != 2 or b.dim() != 2 or b.size(1 if b_transposed else 0) != K or not _dense_kernels_apply(a, b) or
             _recorded(a, b, bias) or
             (bias is not None and not (bias.dtype == torch.float32 and bias.device == a.device and bias.dim() == 1 and
@@ -346,7 +367,9 @@ def matmul(a, b, b_transposed=False, bias=None, out=None):
 def gram(a, b, sums=False):
     """(a^T b, column sums of a or None) for matrices of many rows: yitu_gram_f32 in one pass over a and b; the library's
     GEMM and reduction for other types and for results of more than 65536 values (20 k x 500 x 500: 341 us against 278;
-    1 M x 64 x 64 with sums: 206 us against 768; 170 k x 128 x 256: 247 against 350)."""
+    1 M x 64 x 64 with sums: 206 us against 768; 170 k x 128 x 256: 247 against 350).  Below 1500 rows (6 us against 4) and for
+    1433 x 41 over 16 k and more (1.15 to 1.44 times the library's time) the library is faster, but two to seven times as far
+    from the 64-bit product."""
     if (a.dim() != 2 or b.dim() != 2 or a.size(0) != b.size(0) or a.size(1) * b.size(1) > 65536 or
             not _dense_kernels_apply(a, b) or _recorded(a, b)):
         return torch.mm(a.t(), b), a.sum(0) if sums else None
