@@ -264,8 +264,9 @@ int yitu_spmm_bwd_f32(const yitu_spmm_bwd_args_t *args, yitu_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------------- GAT */
 /* The `plan` argument of the functions below is the optional hub-row schedule of the graph they walk (the transposed
- * graph's for yitu_edge_gather_sum_f32): with it, rows longer than plan->chunk_edges are processed by a whole CTA, or
- * chunk by chunk, instead of by one warp.  NULL keeps one warp per row. */
+ * graph's for yitu_edge_gather_sum_f32): with it, rows longer than plan->chunk_edges are processed chunk by chunk, or by a
+ * whole CTA (the edge softmax: those of more than 256 edges and twice the average row), instead of by one warp.  NULL keeps
+ * one warp per row. */
 /* attn[e,h] = softmax over {edges of the same row and segment} of LeakyReLU_slope(query[seg,row,h] + key[col,h]).
  * Replaces sddmm_forward (YiTu_GNN/YiTu_H/src/sddmm_cuda.cu:5-33,69-89).  Unlike the reference the row maximum
  * is subtracted before exponentiation (same value, no overflow).  n_segments = query.size(0) (<= 16). */
