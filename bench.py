@@ -80,7 +80,8 @@ def spmm_form(nnz, n_rows, d, has_hub_plan):
 
 
 def spmm_kernel_name(nnz, n_rows, d, has_hub_plan=True):
-    """The instantiation(s) behind spmm_form, for 32-byte aligned rows of 33 to 256 floats."""
+    """The instantiation(s) behind spmm_form, for 32-byte aligned rows of 33 to 256 floats; graphs of few long rows (at most
+    65536, 64 edges and more on average) take others."""
     form = spmm_form(nnz, n_rows, d, has_hub_plan)
     if form == "group":
         return "spmm_group_kernel<32,8,1,8,1,true,16>" if d <= 64 else \
