@@ -289,14 +289,12 @@ __global__ void __launch_bounds__(128, SMALL || CTAS < 16 ? CTAS : 12) spmm_grou
                 for (int u = 0; u < EU; ++u) {
                     const bool live = j + u * EPI + sub < n;
                     // one address per edge: the slices lie at constant distances from the lane's first
-                    const auto slice = [&](int i) {
-                        return (SMALL ? p.x + (static_cast<uint32_t>(c[u]) * static_cast<uint32_t>(p.xs) + static_cast<uint32_t>(off[0]))
-                                      : p.x + static_cast<int64_t>(c[u]) * p.xs + off[0]) + i * LPE * VEC;
-                    };
+                    const float *xr = SMALL ? p.x + (static_cast<uint32_t>(c[u]) * static_cast<uint32_t>(p.xs) + static_cast<uint32_t>(off[0]))
+                                            : p.x + static_cast<int64_t>(c[u]) * p.xs + off[0];
 #pragma unroll
                     for (int i = 0; i < NV; ++i) {
                         if (live && valid[i]) {
-                            load_vec<VEC>(v[u][i], slice(i));
+                            load_vec<VEC>(v[u][i], xr + i * LPE * VEC);
                         } else {
 #pragma unroll
                             for (int q = 0; q < VEC; ++q) v[u][i][q] = 0.0f;
